@@ -1,312 +1,310 @@
-// level_sweep.cu -- BILU(0) application (kernel/applyBILU0.m:10-48) as ONE launch per apply.
+// level_sweep.cu -- BILU(0) application (kernel/applyBILU0.m:10-48) as ONE data-driven launch.
 //
 // A sequential elimination order such as the minimum-discarded-fill order of
 // kernel/computeMDFordering.m has long dependency chains: on the 2D NS p = 3 mesh of 49,408
-// faces the level schedule has 1,100 levels of 45 rows on average.  One launch per level and
-// sweep costs ~13 us of launch gap and dependent index loads per level.  Here a single thread-
-// block cluster (CS CTAs, co-scheduled by the hardware) walks all levels of the forward and
-// the backward sweep; the levels are separated by the hardware cluster barrier, so no flag is
-// polled and no wait can hang.  Every row's dependencies are pre-flattened on the host into one
-// fixed-width record (row, diagonal block, (block, column) pairs of the earlier and of the later
-// neighbours), so a thread reaches its data with one load instead of a chain of index loads,
-// and the record and matrix values of the next level (which do not depend on this level's
-// results) are loaded between the barrier's arrive and its wait.
+// faces the level schedule has 1,100 levels of 45 rows on average, and the apply is bound by
+// the latency of a level, not by the 0.5 GB of factors it reads.  Here a warp owns a row, and a
+// row starts when the values it needs have arrived, not when a whole level is done.
 //
-// Work split inside a level: rows s = 0..nr-1 of the level go to CTA s % CS; inside a CTA a
-// pass covers NT / BS rows with one thread per row component r.  The forward sweep computes
-//   y_i[r] = x_i[r] - sum_j L_ij[r, :] y_j        (rows j eliminated before i)
-// and the backward sweep
-//   t_i[r] = y_i[r] - sum_j U_ij[r, :] v_j        (rows j eliminated after i)
-//   v_i[r] = sum_c inv(U_ii)[r, c] t_i[c]         (diagonal blocks are stored inverted)
-// in the operation order of the per-level kernels.  Values written in one level are read in a
-// later one by other CTAs: the writes are followed by a GPU-scope fence before the barrier's
-// arrive, the wait has acquire semantics, and those reads go through L2 (ld.global.cg).
-#include <cooperative_groups.h>
+// Work split: slot q of the plan (rows in level order) belongs to warp q % W of a grid of W warps
+// that are resident together (one cluster, or a cooperative launch).  A warp walks its slots in
+// ascending order in the forward sweep and in descending order in the backward sweep:
+//   y_i = x_i - sum_j L_ij y_j                   (rows j eliminated before i)
+//   v_i = inv(U_ii) (y_i - sum_j U_ij v_j)       (rows j eliminated after i; inverses are stored)
+// The row with the lowest unfinished slot never waits, so the sweep always advances.
+//
+// A value is its own ready flag: y and v are filled with kPending (all bits set, a NaN no kernel
+// here produces: a result with these bits is stored as the default NaN) before the launch, and a
+// reader polls the value itself at L2 until it differs.  One store and one load carry a row to its
+// readers; there is no fence, no barrier and no separate flag.  Waits are bounded (kPollLimit
+// polls, then NaN is used and passed on, so that a plan that is not a schedule ends in NaN, never
+// in a hang).
+//
+// What bounds a level is then the store-to-load time through L2 (0.47 us measured between two SMs)
+// and the arithmetic after it, so both are kept short: the row's factor blocks are staged in
+// shared memory before its inputs arrive, lane r of part p (PARTS = 32 / BS parts) adds up only
+// the neighbours p, p + PARTS, .. in two chains each (a dependent FP64 multiply-add takes 17.6
+// cycles), and the parts are added with shuffles.
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "hdgx_common.cuh"
-
-namespace cg = cooperative_groups;
+#include "trace_internal.cuh"
 
 namespace hdgx {
 
-__device__ __forceinline__ void cluster_arrive_relaxed() {
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait_acquire() {
-    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-// the 16-byte aligned interior of [p, p + bytes) into L2 (a bulk prefetch needs aligned ends)
+constexpr unsigned long long kPending = ~0ull;
+constexpr int kPollLimit = 1 << 21;
+
 __device__ __forceinline__ void bulk_prefetch_l2(const void *p, unsigned bytes) {
+    // the 16-byte aligned interior of [p, p + bytes) (a bulk prefetch needs aligned ends)
     const unsigned long long a0 = ((unsigned long long)p + 15) & ~15ull;
     const unsigned long long a1 = ((unsigned long long)p + bytes) & ~15ull;
     if (a1 > a0) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a0), "r"((unsigned)(a1 - a0)) : "memory");
 }
+__device__ __forceinline__ unsigned long long load_value(const double *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_value(double *p, double v) {
+    unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    if (b == kPending) b = 0x7ff8000000000000ull;
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
+}
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
 
-// One row component's record and (PL) matrix values, loadable ahead of the level that uses them.
-// MT is the storage type of the factors (double, or float for the mixed-precision preconditioner:
-// the values are widened on use and every sum runs in FP64).
-template <int BS, int MAXD, bool PL, bool DIAG, class MT>
-struct RowPrefetch {
-    int i, k0;
-    int k[MAXD], j[MAXD];
-    MT lv[PL ? MAXD * BS : 1];
-    MT dv[(PL && DIAG) ? BS : 1];
-
-    // slot record R (NULL: inactive); OFF = 0 for the earlier neighbours, 2 * MAXD for the later
-    template <int OFF>
-    __device__ __forceinline__ void load(const int *R, const MT *__restrict__ Mg, int r) {
-        if (!R) { i = -1; return; }
-        i = __ldg(R);
-        k0 = __ldg(R + 1);
-#pragma unroll
-        for (int d = 0; d < MAXD; d++) { k[d] = __ldg(R + 2 + OFF + 2 * d); j[d] = __ldg(R + 3 + OFF + 2 * d); }
-        if constexpr (PL) {
-#pragma unroll
-            for (int d = 0; d < MAXD; d++) {
-                if (k[d] >= 0) {
-                    const MT *B = Mg + (size_t)BS * BS * k[d] + r;
-#pragma unroll
-                    for (int c = 0; c < BS; c++) lv[d * BS + c] = __ldg(B + BS * c);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < BS; c++) lv[d * BS + c] = MT(0);     // padded slot: contributes 0
-                }
-            }
-            if constexpr (DIAG) {
-                const MT *D = Mg + (size_t)BS * BS * k0 + r;
-#pragma unroll
-                for (int c = 0; c < BS; c++) dv[c] = __ldg(D + BS * c);
-            }
-        }
-    }
-
-    // acc - sum_d B_d[r, :] in_{j_d}
-    __device__ __forceinline__ double reduce(double acc, const MT *__restrict__ Mg, const double *in, int r) const {
-        if constexpr (PL) {
-            // every neighbour's values are loaded before the first multiply-add, so their L2
-            // round trips overlap; padded slots (k < 0) contribute exact zeros
-            double ov[MAXD][BS];
-#pragma unroll
-            for (int d = 0; d < MAXD; d++) {
-                const bool live = k[d] >= 0;
-                const double *oj = in + (size_t)BS * (live ? j[d] : 0);
-#pragma unroll
-                for (int c = 0; c < BS; c++) ov[d][c] = live ? __ldcg(oj + c) : 0.0;
-            }
-#pragma unroll
-            for (int d = 0; d < MAXD; d++)
-#pragma unroll
-                for (int c = 0; c < BS; c++) acc -= (double)lv[d * BS + c] * ov[d][c];
-            return acc;
-        } else {
-#pragma unroll
-            for (int d = 0; d < MAXD; d++) {
-                if (k[d] < 0) break;
-                const double *oj = in + (size_t)BS * j[d];
-                double ov[BS];
-#pragma unroll
-                for (int c = 0; c < BS; c++) ov[c] = __ldcg(oj + c);
-                const MT *B = Mg + (size_t)BS * BS * k[d] + r;
-                double bv[BS];
-#pragma unroll
-                for (int c = 0; c < BS; c++) bv[c] = (double)__ldg(B + BS * c);
-#pragma unroll
-                for (int c = 0; c < BS; c++) acc -= bv[c] * ov[c];
-            }
-            return acc;
-        }
-    }
-
-    // sum_c inv(U_ii)[r, c] t[c]
-    __device__ __forceinline__ double diag(const MT *__restrict__ Mg, const double *t, int r) const {
-        double o = 0.0;
-        if constexpr (PL && DIAG) {
-#pragma unroll
-            for (int c = 0; c < BS; c++) o += (double)dv[c] * t[c];
-        } else {
-            const MT *D = Mg + (size_t)BS * BS * k0 + r;
-#pragma unroll
-            for (int c = 0; c < BS; c++) o += (double)__ldg(D + BS * c) * t[c];
-        }
-        return o;
-    }
+// Shared memory of one warp: MAXD neighbour blocks and the diagonal block of its row, the
+// neighbours' values and the row's intermediate t; as many warps per CTA as fit (at most 16).
+template <int BS, int MAXD, class MT>
+struct SweepShape {
+    static constexpr int PARTS = 32 / BS, DP = (MAXD + PARTS - 1) / PARTS;
+    static constexpr int RW = 2 + 4 * MAXD;                                  // record width (ints)
+    static constexpr int BLK = BS * BS;
+    static constexpr size_t stage = (sizeof(MT) * BLK * (MAXD + 1) + 15) / 16 * 16;
+    static constexpr int BSP = (BS + 1) / 2 * 2;                             // 16-byte aligned value rows
+    static constexpr size_t warp_bytes = stage + sizeof(double) * BSP * (MAXD + 1);
+    static constexpr int fit = (int)(216 * 1024 / warp_bytes);
+    static constexpr int WPC = fit > 16 ? 16 : fit;
+    static constexpr size_t smem = warp_bytes * WPC;
+    static_assert(BS <= 32 && RW <= 32 && WPC >= 1, "one lane per row component and per record entry");
 };
 
-template <int BS, int MAXD, int CS, int NT, class MT>
-__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(NT)
-    bilu0_level_sweep_kernel(int nlev, const int *__restrict__ plan, const MT *__restrict__ Mg,
-                             const double *__restrict__ x, double *y, double *v) {
-    constexpr int RPP = NT / BS;                        // rows per pass per CTA
-    constexpr int RW = 2 + 4 * MAXD;                    // record width (ints)
-    constexpr bool PLF = MAXD * BS <= 64;               // forward: L values prefetched
-    constexpr bool PLB = (MAXD + 1) * BS <= 80;         // backward: U and inv(D) values prefetched
-    extern __shared__ int lp[];                         // level offsets [nlev + 1]
-    __shared__ double tsh[RPP * BS];
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank();
-    const int *rec = plan + nlev + 1;
-    const int m = threadIdx.x / BS, r = threadIdx.x - (threadIdx.x / BS) * BS;
-    for (int t = threadIdx.x; t <= nlev; t += NT) lp[t] = __ldg(plan + t);
-    __syncthreads();
-    auto slot_rec = [&](int lev) -> const int * {      // this thread's first-pass record, or NULL
-        const int q0 = lp[lev], nr = lp[lev + 1] - q0, s = rank + CS * m;
-        return (m < RPP && s < nr) ? rec + (size_t)(q0 + s) * RW : nullptr;
-    };
-    // L2 pipeline for the first pass of later levels (the factors are read once per apply and
-    // do not stay in L2 between applies): the records of level lev + DR are prefetched to L2;
-    // one block index per thread (component r < NK of the row: a neighbour block, in the
-    // backward sweep r = 0 the diagonal block) is loaded DK levels ahead and its block
-    // prefetched to L2 one level later, so the register prefetch of the next level hits L2.
-    constexpr int DR = 7, DK = 4;
-    auto prefetch_rec = [&](int lev) {
-        if (r == 0 && lev >= 0 && lev < nlev) {
-            const int *R = slot_rec(lev);
-            if (R) { prefetch_l2(R); prefetch_l2(R + RW - 1); }
+template <int BS, int MAXD, class MT>
+__global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
+    bilu0_sweep_kernel(int nf, const int *__restrict__ rec, const MT *__restrict__ Mg, const double *__restrict__ x,
+                       double *y, double *v, int phases) {
+    using S = SweepShape<BS, MAXD, MT>;
+    constexpr int PARTS = S::PARTS, DP = S::DP, RW = S::RW, BLK = S::BLK, BSP = S::BSP;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char *mine = smem_raw + S::warp_bytes * warp;
+    MT *blk = reinterpret_cast<MT *>(mine);                          // [MAXD + 1][BS, BS]
+    double *val = reinterpret_cast<double *>(mine + S::stage);       // [MAXD][BSP], then t [BSP]
+    double *tsh = val + MAXD * BSP;
+    const int part = lane / BS, r = lane - part * BS;
+    const bool on = part < PARTS;
+    const int W = gridDim.x * S::WPC, w = warp * gridDim.x + blockIdx.x;   // neighbouring slots on different SMs
+    const bool wide = sizeof(MT) * BLK % 16 == 0 && ((size_t)Mg & 15) == 0;
+    int limit = kPollLimit;
+
+    // slot record, one entry per lane: (row, diagonal block, MAXD (block, column) of the earlier
+    // neighbours, MAXD of the later ones)
+    auto record = [&](int q) { return (q >= 0 && q < nf && lane < RW) ? __ldg(rec + (size_t)q * RW + lane) : -1; };
+    auto stage_block = [&](int slot, int k) {
+        const MT *src = Mg + (size_t)BLK * k;
+        MT *dst = blk + slot * BLK;
+        if (wide) {
+            constexpr int PER = 16 / sizeof(MT);
+            for (int t = lane * PER; t < BLK; t += 32 * PER) cp_async<16>(dst + t, src + t);
+        } else {
+            for (int t = lane; t < BLK; t += 32) cp_async<sizeof(MT)>(dst + t, src + t);
         }
     };
-    // the block index component r prefetches at level lev (-1: none); BWD: backward-sweep blocks
-    auto block_of = [&](int lev, bool bwd) -> int {
-        if (lev < 0 || lev >= nlev) return -1;
-        const int *R = slot_rec(lev);
-        if (!R) return -1;
-        if (!bwd) return r < MAXD ? __ldcg(R + 2 + 2 * r) : -1;
-        return r == 0 ? __ldcg(R + 1) : (r <= MAXD ? __ldcg(R + 2 + 2 * MAXD + 2 * (r - 1)) : -1);
+    // this lane's row of block B times the values u, in two chains
+    auto dot_row = [&](const MT *B, const double *u, double &s0, double &s1) {
+#pragma unroll
+        for (int c = 0; c < BS; c += 2) {
+            s0 = fma((double)B[r + BS * c], u[c], s0);
+            if (c + 1 < BS) s1 = fma((double)B[r + BS * (c + 1)], u[c + 1], s1);
+        }
     };
-    auto prefetch_block = [&](int k) {
-        if (k >= 0) bulk_prefetch_l2(Mg + (size_t)BS * BS * k, (unsigned)(sizeof(MT) * BS * BS));
+    auto add_parts = [&](double s) {
+        double t = s;
+#pragma unroll
+        for (int p = 1; p < PARTS; p++) t += __shfl_down_sync(0xffffffffu, s, p * BS);
+        return t;                                                        // valid in part 0
     };
 
-    // forward sweep: y_i = x_i - sum_{j before i} L_ij y_j, levels in elimination order
-    {
-        for (int l = 0; l < DR; l++) prefetch_rec(l);
-        int pk = block_of(DK - 1, false);
-        RowPrefetch<BS, MAXD, PLF, false, MT> pf;
-        pf.template load<0>(slot_rec(0), Mg, r);
-        double xv = pf.i >= 0 ? __ldg(x + (size_t)BS * pf.i + r) : 0.0;
-        for (int lev = 0; lev < nlev; lev++) {
-            const int q0 = lp[lev], nr = lp[lev + 1] - q0;
-            if (pf.i >= 0) y[(size_t)BS * pf.i + r] = pf.reduce(xv, Mg, y, r);
-            for (int base = CS * RPP; base < nr; base += CS * RPP) {
-                const int s = base + rank + CS * m;
-                if (m < RPP && s < nr) {
-                    RowPrefetch<BS, MAXD, false, false, MT> row;
-                    row.template load<0>(rec + (size_t)(q0 + s) * RW, Mg, r);
-                    y[(size_t)BS * row.i + r] = row.reduce(__ldg(x + (size_t)BS * row.i + r), Mg, y, r);
+    auto sweep = [&](auto dir) {
+        constexpr bool BWD = decltype(dir)::value;
+        constexpr int OFF = BWD ? 2 + 2 * MAXD : 2;
+        const double *in = BWD ? v : y;
+        double *out = BWD ? v : y;
+        const int step = BWD ? -W : W;
+        int q = BWD ? nf - 1 - w : w;
+        int cur = record(q), nxt = record(q + step), nxt2 = record(q + 2 * step);
+        auto begin_row = [&](int R) {                                    // stage the row's blocks
+            const int i = __shfl_sync(0xffffffffu, R, 0);
+            if (i < 0) return;
+#pragma unroll
+            for (int d = 0; d < MAXD; d++) {
+                const int k = __shfl_sync(0xffffffffu, R, OFF + 2 * d);
+                if (k >= 0) stage_block(d, k);
+            }
+            if (BWD) stage_block(MAXD, __shfl_sync(0xffffffffu, R, 1));
+        };
+        auto prefetch_row = [&](int R) {                                 // the blocks of a later row into L2
+            const int at = lane < MAXD ? OFF + 2 * lane : 1;
+            const int k = __shfl_sync(0xffffffffu, R, at);
+            if ((lane < MAXD || (BWD && lane == MAXD)) && k >= 0) bulk_prefetch_l2(Mg + (size_t)BLK * k, sizeof(MT) * BLK);
+        };
+        begin_row(cur);
+        prefetch_row(nxt);
+        auto load_x = [&](int R) {
+            const int i = __shfl_sync(0xffffffffu, R, 0);
+            return (!BWD && i >= 0 && on) ? __ldg(x + (size_t)BS * i + r) : 0.0;
+        };
+        double xv = load_x(cur);
+        while (q >= 0 && q < nf) {
+            const int i = __shfl_sync(0xffffffffu, cur, 0);
+            int k[DP], j[DP];
+#pragma unroll
+            for (int s = 0; s < DP; s++) {
+                const int d = part + s * PARTS;
+                const int at = OFF + 2 * (d < MAXD ? d : 0);
+                k[s] = __shfl_sync(0xffffffffu, cur, at);
+                j[s] = __shfl_sync(0xffffffffu, cur, at + 1);
+                if (!on || d >= MAXD) k[s] = -1;
+            }
+            prefetch_row(nxt2);
+            const int nxt3 = record(q + 3 * step);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            // wait for the neighbours' values (and, backward, for the row's own y)
+            unsigned long long got[DP], own = 0;
+            bool ready;
+            int n = 0;
+            do {
+                ready = true;
+#pragma unroll
+                for (int s = 0; s < DP; s++) {
+                    got[s] = k[s] >= 0 ? load_value(in + (size_t)BS * j[s] + r) : 0ull;
+                    ready &= got[s] != kPending;
                 }
+                if (BWD) {
+                    own = part == 0 ? load_value(y + (size_t)BS * i + r) : 0ull;
+                    ready &= own != kPending;
+                }
+            } while (!__all_sync(0xffffffffu, ready) && ++n < limit);
+            if (n >= limit) limit = 1;                                   // NaN (kPending is one) from here on
+#pragma unroll
+            for (int s = 0; s < DP; s++)
+                if (k[s] >= 0) val[(part + s * PARTS) * BSP + r] = __longlong_as_double((long long)got[s]);
+            __syncwarp();
+            double acc[2 * DP];
+#pragma unroll
+            for (int s = 0; s < 2 * DP; s++) acc[s] = 0.0;
+#pragma unroll
+            for (int s = 0; s < DP; s++) {
+                const int d = part + s * PARTS;
+                if (k[s] >= 0) dot_row(blk + d * BLK, val + d * BSP, acc[2 * s], acc[2 * s + 1]);
             }
-            __threadfence();
-            cluster_arrive_relaxed();
-            if (lev + 1 < nlev) {
-                pf.template load<0>(slot_rec(lev + 1), Mg, r);
-                xv = pf.i >= 0 ? __ldg(x + (size_t)BS * pf.i + r) : 0.0;
+            double sum = acc[0] + acc[1];
+#pragma unroll
+            for (int s = 1; s < DP; s++) sum += acc[2 * s] + acc[2 * s + 1];
+            sum = add_parts(sum);
+            if (!BWD) {
+                if (part == 0) store_value(out + (size_t)BS * i + r, xv - sum);
+            } else {
+                if (part == 0) tsh[r] = __longlong_as_double((long long)own) - sum;
+                __syncwarp();
+                double s0 = 0.0, s1 = 0.0;
+                if (on) {
+                    constexpr int CP = (BS + PARTS - 1) / PARTS;         // columns of a part
+                    const MT *D = blk + MAXD * BLK + r;
+#pragma unroll
+                    for (int c = 0; c < CP; c += 2) {
+                        const int c0 = part * CP + c;
+                        if (BS % PARTS == 0 || c0 < BS) s0 = fma((double)D[BS * c0], tsh[c0], s0);
+                        if (c + 1 < CP && (BS % PARTS == 0 || c0 + 1 < BS)) s1 = fma((double)D[BS * (c0 + 1)], tsh[c0 + 1], s1);
+                    }
+                }
+                const double o = add_parts(s0 + s1);
+                if (part == 0) store_value(out + (size_t)BS * i + r, o);
             }
-            prefetch_block(pk);                         // level lev + DK - 1
-            pk = block_of(lev + DK, false);
-            prefetch_rec(lev + DR);
-            cluster_wait_acquire();
+            __syncwarp();                                                // the staged blocks and values are free
+            cur = nxt;
+            nxt = nxt2;
+            nxt2 = nxt3;
+            q += step;
+            begin_row(cur);
+            xv = load_x(cur);
         }
-    }
-    // backward sweep: v_i = inv(U_ii) (y_i - sum_{j after i} U_ij v_j), levels in reverse order
-    {
-        for (int l = 0; l < DR; l++) prefetch_rec(nlev - 1 - l);
-        int pk = block_of(nlev - DK, true);
-        RowPrefetch<BS, MAXD, PLB, true, MT> pf;
-        pf.template load<2 * MAXD>(slot_rec(nlev - 1), Mg, r);
-        for (int lev = nlev - 1; lev >= 0; lev--) {
-            const int q0 = lp[lev], nr = lp[lev + 1] - q0;
-            // pass 0 (prefetched); y_i[r] was written by this same thread in the forward sweep
-            if (pf.i >= 0) tsh[m * BS + r] = pf.reduce(__ldcg(y + (size_t)BS * pf.i + r), Mg, v, r);
-            __syncthreads();
-            if (pf.i >= 0) v[(size_t)BS * pf.i + r] = pf.diag(Mg, tsh + m * BS, r);
-            if (nr > CS * RPP) __syncthreads();      // tsh is rewritten by the next pass (else the
-                                                     // cluster barrier below orders its reuse)
-            for (int base = CS * RPP; base < nr; base += CS * RPP) {    // trip count is uniform in the CTA
-                const int s = base + rank + CS * m;
-                const bool act = m < RPP && s < nr;
-                RowPrefetch<BS, MAXD, false, true, MT> row;
-                row.template load<2 * MAXD>(act ? rec + (size_t)(q0 + s) * RW : nullptr, Mg, r);
-                if (act) tsh[m * BS + r] = row.reduce(__ldcg(y + (size_t)BS * row.i + r), Mg, v, r);
-                __syncthreads();
-                if (act) v[(size_t)BS * row.i + r] = row.diag(Mg, tsh + m * BS, r);
-                __syncthreads();
-            }
-            __threadfence();
-            cluster_arrive_relaxed();
-            if (lev > 0) pf.template load<2 * MAXD>(slot_rec(lev - 1), Mg, r);
-            prefetch_block(pk);                         // level lev - DK + 1
-            pk = block_of(lev - DK, true);
-            prefetch_rec(lev - DR);
-            cluster_wait_acquire();
-        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+    };
+    if (phases & 1) sweep(std::false_type{});
+    if (phases & 2) sweep(std::true_type{});
+}
+
+__global__ void fill_pending_kernel(size_t n, unsigned long long *a, unsigned long long *b) {
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+        if (a) a[t] = kPending;
+        if (b) b[t] = kPending;
     }
 }
 
-constexpr int kSweepCS = 8;     // CTAs in the cluster (portable maximum)
-constexpr int kSweepNT = 256;
-
-// 0 launched, 1 not possible (caller falls back), 2 the device cannot place such a cluster
-template <int BS, int MAXD, int CS, int NT, class MT>
-static int launch_cluster(int nlev, const int *plan, const MT *Mg, const double *x, double *y, double *v,
-                          size_t smem, cudaStream_t st) {
-    auto kern = bilu0_level_sweep_kernel<BS, MAXD, CS, NT, MT>;
-    if (smem > 40 * 1024 && allow_dynamic_smem((const void *)kern, smem) != cudaSuccess) return 1;
-    if (CS > 8) {
-        if (cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+// The grid must be resident at once.  Up to 8 CTAs are one cluster, which the hardware places
+// together or not at all, so that the sweeps of many concurrent solves share the GPU; larger grids
+// are a cooperative launch.
+template <int BS, int MAXD, class MT>
+static int launch_sweep(const hdgx_bsr *A, const MT *Mg, const double *x, double *y, double *v, cudaStream_t st) {
+    using S = SweepShape<BS, MAXD, MT>;
+    auto kern = bilu0_sweep_kernel<BS, MAXD, MT>;
+    if (allow_dynamic_smem((const void *)kern, S::smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    const int nf = A->nf;
+    const size_t n = (size_t)BS * nf;
+    // two warps per row of an average level: one works while the other's blocks are staged
+    const long long want = (2ll * nf / A->ncolors + S::WPC - 1) / S::WPC;
+    const int nsm = sm_count_of(current_device());
+    int G = want < 1 ? 1 : (want > nsm ? nsm : (int)want);
+    if (G <= 8) G = G > 4 ? 8 : (G > 2 ? 4 : G);
+    const int *rec = A->sweep_plan + A->ncolors + 1;
+    const unsigned fg = (unsigned)((n + 255) / 256 < (size_t)nsm * 8 ? (n + 255) / 256 : (size_t)nsm * 8);
+    auto launch = [&](int phases) -> bool {
+        if (G > 8) {
+            int nf_ = nf, ph = phases;
+            void *args[] = {&nf_, &rec, &Mg, &x, &y, &v, &ph};
+            if (cudaLaunchCooperativeKernel((const void *)kern, dim3(G), dim3(S::WPC * 32), args, S::smem, st) == cudaSuccess)
+                return true;
             cudaGetLastError();
-            return 2;
+            G = 8;
         }
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(CS);
-        cfg.blockDim = dim3(NT);
-        cfg.dynamicSmemBytes = smem;
+        cfg.gridDim = dim3(G);
+        cfg.blockDim = dim3(S::WPC * 32);
+        cfg.dynamicSmemBytes = S::smem;
         cfg.stream = st;
-        int ncl = 0;
-        if (cudaOccupancyMaxActiveClusters(&ncl, (const void *)kern, &cfg) != cudaSuccess || ncl < 1) {
-            cudaGetLastError();
-            return 2;
-        }
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = G;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, kern, nf, rec, Mg, x, y, v, phases) == cudaSuccess;
+    };
+    unsigned long long *yb = reinterpret_cast<unsigned long long *>(y), *vb = reinterpret_cast<unsigned long long *>(v);
+    if (v == x) {                                       // x is read before v is marked
+        fill_pending_kernel<<<fg, 256, 0, st>>>(n, yb, nullptr);
+        if (!launch(1)) return 1;
+        fill_pending_kernel<<<fg, 256, 0, st>>>(n, vb, nullptr);
+        return launch(2) ? 0 : 1;
     }
-    kern<<<CS, NT, smem, st>>>(nlev, plan, Mg, x, y, v);
-    return 0;
+    fill_pending_kernel<<<fg, 256, 0, st>>>(n, yb, vb);
+    return launch(3) ? 0 : 1;
 }
 
-// Large blocks (bs >= 20: 3D, or 2D p = 4) run CTAs of 512 threads (fewer passes per level).
-// When a level moves more matrix than 8 SMs stream in the time of a level (kWideLevelBytes of
-// factors per level on average) the cluster has 16 CTAs (a non-portable size) when the device
-// can place one, else 8.  (3D Euler p = 2, 399,360 faces, 12 MB per level: 69.5 ms per apply
-// with 8 CTAs of 256, 57.9 ms with 8 of 512, 37.2 ms with 16 of 512.)  Small systems stay on 8:
-// a 16-CTA cluster needs 16 free SMs of one GPC, which concurrent solves rarely leave (64 queued
-// serving requests: 32 solves/s with 16-CTA clusters for their bs = 20 systems, 74 with 8).
-constexpr size_t kWideLevelBytes = 4u << 20;
-template <int BS, int MAXD, class MT>
-static int launch_level_sweep(int nlev, long long nnzb, const int *plan, const MT *Mg, const double *x, double *y,
-                              double *v, cudaStream_t st) {
-    const size_t smem = sizeof(int) * ((size_t)nlev + 1);
-    if (smem > 160 * 1024) return 1;                    // very long schedules: per-level launches
-    if constexpr (BS >= 20) {
-        const size_t level_bytes = sizeof(MT) * BS * BS * (size_t)nnzb / (size_t)nlev;
-        if (level_bytes >= kWideLevelBytes) {
-            const int rc = launch_cluster<BS, MAXD, 16, 512, MT>(nlev, plan, Mg, x, y, v, smem, st);
-            if (rc != 2) return rc;
-        }
-        return launch_cluster<BS, MAXD, 8, 512, MT>(nlev, plan, Mg, x, y, v, smem, st) == 0 ? 0 : 1;
-    } else {
-        return launch_cluster<BS, MAXD, kSweepCS, kSweepNT, MT>(nlev, plan, Mg, x, y, v, smem, st) == 0 ? 0 : 1;
-    }
-}
-
-// 0 when launched, 1 when there is no plan or no specialisation for it (the caller falls back)
+// 0 when launched, 1 when there is no plan, no specialisation for it, or the vectors overlap in a
+// way the marked values do not allow (the caller falls back to one launch per level)
 template <class MT>
 static int level_sweep_apply_t(const hdgx_bsr *A, const MT *Mg, const double *x, double *y, double *v, cudaStream_t st) {
-    if (!A->sweep_plan || A->ncolors < 1) return 1;
+    if (!A->sweep_plan || A->ncolors < 1 || A->nf < 1) return 1;
     const int md = A->sweep_maxd;
     if (md != 4 && md != 6) return 1;
+    const size_t n = (size_t)A->bs * A->nf;
+    auto overlap = [n](const double *a, const double *b) { return a < b + n && b < a + n; };
+    if (overlap(x, y) || overlap(y, v) || (overlap(x, v) && x != v)) return 1;
     switch (A->bs) {
-#define HDGX_LS(B)                                                                                \
-    case B:                                                                                       \
-        return md == 4 ? launch_level_sweep<B, 4, MT>(A->ncolors, A->nnzb, A->sweep_plan, Mg, x, y, v, st)    \
-                       : launch_level_sweep<B, 6, MT>(A->ncolors, A->nnzb, A->sweep_plan, Mg, x, y, v, st);
+#define HDGX_LS(B)                                                                            \
+    case B:                                                                                   \
+        return md == 4 ? launch_sweep<B, 4, MT>(A, Mg, x, y, v, st) : launch_sweep<B, 6, MT>(A, Mg, x, y, v, st);
         HDGX_LS(8) HDGX_LS(12) HDGX_LS(15) HDGX_LS(16) HDGX_LS(20) HDGX_LS(30)
 #undef HDGX_LS
         default: return 1;
