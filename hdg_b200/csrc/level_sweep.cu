@@ -23,8 +23,8 @@
 // What bounds a level is then the store-to-load time through L2 (0.47 us measured between two SMs)
 // and the arithmetic after it, so both are kept short: the row's factor blocks are staged in
 // shared memory before its inputs arrive, lane r of part p (PARTS = 32 / BS parts) adds up only
-// the neighbours p, p + PARTS, .. in two chains each (a dependent FP64 multiply-add takes 17.6
-// cycles), and the parts are added with shuffles.
+// the neighbours p, p + PARTS, .. in CH independent chains (a dependent FP64 multiply-add takes
+// 17.6 cycles), and the parts are added with shuffles.
 #include <cuda_runtime.h>
 #include <type_traits>
 #include "hdgx_common.cuh"
@@ -65,6 +65,7 @@ struct SweepShape {
     static constexpr int PARTS = 32 / BS, DP = (MAXD + PARTS - 1) / PARTS;
     static constexpr int RW = 2 + 4 * MAXD;                                  // record width (ints)
     static constexpr int BLK = BS * BS;
+    static constexpr int CH = BS == 30 ? 6 : (BS == 15 ? 5 : 4);             // chains of a row sum
     static constexpr size_t stage = (sizeof(MT) * BLK * (MAXD + 1) + 15) / 16 * 16;
     static constexpr int BSP = (BS + 1) / 2 * 2;                             // 16-byte aligned value rows
     static constexpr size_t warp_bytes = stage + sizeof(double) * BSP * (MAXD + 1);
@@ -74,12 +75,27 @@ struct SweepShape {
     static_assert(BS <= 32 && RW <= 32 && WPC >= 1, "one lane per row component and per record entry");
 };
 
+// columns [c0, c0 + N) of a row of the block at B (its first column) times the values u, added to CH chains
+template <int BS, int N, int CH, class MT>
+__device__ __forceinline__ void dot_cols(const MT *B, const double *u, int c0, double (&acc)[CH]) {
+#pragma unroll
+    for (int c = 0; c < N; c++)
+        if (BS % N == 0 || c0 + c < BS) acc[c % CH] = fma((double)B[BS * (c0 + c)], u[c0 + c], acc[c % CH]);
+}
+template <int CH>
+__device__ __forceinline__ double chain_sum(const double (&acc)[CH]) {
+    double t = acc[0] + acc[1];
+#pragma unroll
+    for (int c = 2; c < CH; c += 2) t += c + 1 < CH ? acc[c] + acc[(c + 1) % CH] : acc[c];
+    return t;
+}
+
 template <int BS, int MAXD, class MT>
 __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
     bilu0_sweep_kernel(int nf, const int *__restrict__ rec, const MT *__restrict__ Mg, const double *__restrict__ x,
                        double *y, double *v, int phases) {
     using S = SweepShape<BS, MAXD, MT>;
-    constexpr int PARTS = S::PARTS, DP = S::DP, RW = S::RW, BLK = S::BLK, BSP = S::BSP;
+    constexpr int PARTS = S::PARTS, DP = S::DP, RW = S::RW, BLK = S::BLK, BSP = S::BSP, CH = S::CH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char *mine = smem_raw + S::warp_bytes * warp;
@@ -103,14 +119,6 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
             for (int t = lane * PER; t < BLK; t += 32 * PER) cp_async<16>(dst + t, src + t);
         } else {
             for (int t = lane; t < BLK; t += 32) cp_async<sizeof(MT)>(dst + t, src + t);
-        }
-    };
-    // this lane's row of block B times the values u, in two chains
-    auto dot_row = [&](const MT *B, const double *u, double &s0, double &s1) {
-#pragma unroll
-        for (int c = 0; c < BS; c += 2) {
-            s0 = fma((double)B[r + BS * c], u[c], s0);
-            if (c + 1 < BS) s1 = fma((double)B[r + BS * (c + 1)], u[c + 1], s1);
         }
     };
     auto add_parts = [&](double s) {
@@ -185,35 +193,22 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
             for (int s = 0; s < DP; s++)
                 if (k[s] >= 0) val[(part + s * PARTS) * BSP + r] = __longlong_as_double((long long)got[s]);
             __syncwarp();
-            double acc[2 * DP];
-#pragma unroll
-            for (int s = 0; s < 2 * DP; s++) acc[s] = 0.0;
+            double acc[CH] = {};
 #pragma unroll
             for (int s = 0; s < DP; s++) {
                 const int d = part + s * PARTS;
-                if (k[s] >= 0) dot_row(blk + d * BLK, val + d * BSP, acc[2 * s], acc[2 * s + 1]);
+                if (k[s] >= 0) dot_cols<BS, BS, CH>(blk + d * BLK + r, val + d * BSP, 0, acc);
             }
-            double sum = acc[0] + acc[1];
-#pragma unroll
-            for (int s = 1; s < DP; s++) sum += acc[2 * s] + acc[2 * s + 1];
-            sum = add_parts(sum);
+            const double sum = add_parts(chain_sum(acc));
             if (!BWD) {
                 if (part == 0) store_value(out + (size_t)BS * i + r, xv - sum);
             } else {
                 if (part == 0) tsh[r] = __longlong_as_double((long long)own) - sum;
                 __syncwarp();
-                double s0 = 0.0, s1 = 0.0;
-                if (on) {
-                    constexpr int CP = (BS + PARTS - 1) / PARTS;         // columns of a part
-                    const MT *D = blk + MAXD * BLK + r;
-#pragma unroll
-                    for (int c = 0; c < CP; c += 2) {
-                        const int c0 = part * CP + c;
-                        if (BS % PARTS == 0 || c0 < BS) s0 = fma((double)D[BS * c0], tsh[c0], s0);
-                        if (c + 1 < CP && (BS % PARTS == 0 || c0 + 1 < BS)) s1 = fma((double)D[BS * (c0 + 1)], tsh[c0 + 1], s1);
-                    }
-                }
-                const double o = add_parts(s0 + s1);
+                double ad[CH] = {};
+                constexpr int CP = (BS + PARTS - 1) / PARTS;             // columns of a part
+                if (on) dot_cols<BS, CP, CH>(blk + MAXD * BLK + r, tsh, part * CP, ad);
+                const double o = add_parts(chain_sum(ad));
                 if (part == 0) store_value(out + (size_t)BS * i + r, o);
             }
             __syncwarp();                                                // the staged blocks and values are free
@@ -251,8 +246,10 @@ static int launch_sweep(const hdgx_bsr *A, const MT *Mg, const double *x, double
     }
     const int nf = A->nf;
     const size_t n = (size_t)BS * nf;
-    // two warps per row of an average level: one works while the other's blocks are staged
-    const long long want = (2ll * nf / A->ncolors + S::WPC - 1) / S::WPC;
+    // four warps per row of an average level, so that a row's warp is there, its blocks staged, when
+    // the values arrive (2D p = 3, 12,416 faces in 440 levels: 1,322, 769, 611 and 641 us per apply
+    // with 1, 2, 4 and 8; 3D p = 2, 6,528 faces in 282 levels: 1,153, 900, 720 and 680)
+    const long long want = (4ll * nf / A->ncolors + S::WPC - 1) / S::WPC;
     const int nsm = sm_count_of(current_device());
     int G = want < 1 ? 1 : (want > nsm ? nsm : (int)want);
     if (G <= 8) G = G > 4 ? 8 : (G > 2 ? 4 : G);
