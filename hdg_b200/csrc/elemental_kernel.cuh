@@ -24,6 +24,7 @@
 #include <type_traits>
 #include <math.h>
 #include "hdgx_common.cuh"
+#include "dmma.cuh"
 #include "tcgen05.cuh"
 
 namespace hdgx {
@@ -84,6 +85,7 @@ struct Dims {
 // is dead during the solve).  The geometry tables shapmv / shapmf are read from global
 // memory (L1) instead: they are used once per element.  Less shared memory per element means
 // more elements resident per SM (the kernel is latency-bound).
+constexpr int ev(int x) { return (x + 1) / 2 * 2; }        // rounded up to 16 bytes
 constexpr int al16(int x) { return (x + 15) / 16 * 16; }   // a double offset rounded up to 128 bytes
 
 // Placement of the tensor-core operands of the mixed form in the free scratch ranges
@@ -160,7 +162,15 @@ struct Plan {
     static constexpr int p_dudg = p_Rh + D::NH;
     static constexpr int p_jv = p_dudg + D::NQ;                   // [NGV] volume jac (time-dependent mass term)
     static constexpr int p_SDsep = p_jv + D::NGV;                 // SD when it does not fit the scratch
-    static constexpr int p_end = p_SDsep + (SD_ALIAS ? 0 : D::NU * D::NU);
+    // column blocks published by the FP64 elimination of SD (block_gj): in the scratch next to SD
+    // (dead once SD is built) where they fit, else behind everything else
+    static constexpr int PUB = MIXED ? 0 : BlockGJ<D::NU, 1, 32>::pub_doubles;
+    static constexpr int pub_in = ev(x_start + (SD_ALIAS ? D::NU * D::NU : 0));
+    static constexpr bool PUB_ALIAS = pub_in + PUB <= x_end;
+    static constexpr int p_pubsep = ev(p_SDsep + (SD_ALIAS ? 0 : D::NU * D::NU));
+    static constexpr int p_pub = PUB_ALIAS ? pub_in : p_pubsep;
+    static constexpr int p_end = p_pubsep + (PUB_ALIAS ? 0 : PUB);
+    static_assert(ev(x_wrl) + BlockGJ<D::NPV, 1, 32>::pub_doubles <= x_end, "inv(M)'s column blocks fit the scratch");
     static constexpr int p_SD = SD_ALIAS ? x_start : p_SDsep;
     // column tiles of DUDG_DUH (reuse the scratch)
     static constexpr int NCG = VISC ? D::NC : D::NCU;
@@ -233,6 +243,8 @@ struct Plan {
                                                ? lu_off + D::NU * D::NU + (D::NU + 1) * LU_CH
                                                : ws_dead + x_dead_end - x_start;
     static constexpr size_t smem_bytes = WS ? sizeof(double) * ws_smem_doubles : bytes;   // of it in shared memory
+    static constexpr int ws_pubM = ev(ws_dead + x_dead_end - x_start);      // inv(M)'s column blocks
+    static_assert(!WS || ws_pubM + BlockGJ<D::NPV, 1, 32>::pub_doubles <= ws_smem_doubles, "they fit behind the first group");
     static_assert(!WS || LU_CHMAX >= 1, "the LU factors and one column fit shared memory");
     static_assert(!WS || smem_bytes <= 227 * 1024, "the shared-memory part of the plan fits");
 };
@@ -516,7 +528,8 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
 
         // ============================ Mi = inv(M): MiC, MiE, MiRq (schur_primal.m:86-91)
         // M is SPD (exact quadrature of phi phi jac): eliminate without pivoting
-        gj_regs_nopiv<NPV, NPV * ND + NDF * ND + NCU * ND, NT, 8>(s_M, s_MiC, s_pcol, s_bad);
+        block_gj<NPV, NPV * ND + NDF * ND + NCU * ND, NT, false, NaturalOrder>(
+            s_M, s_MiC, L::WS ? smd + L::ws_pubM : wk + ev(L::x_wrl), s_bad);
         if (tid == 0 && *s_bad) *s_bad = 1;
         __syncthreads();
         if (Q.QDG) {
@@ -947,7 +960,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                     __syncthreads();
                 }
             } else {
-                gj_regs_nopiv<NU, 1 + NH, NT, 8, NPV>(s_SD, s_R, s_pcol, s_bad);
+                block_gj<NU, 1 + NH, NT, true, PairedOrder<NPV, NCU>>(s_SD, s_R, wk + L::p_pub, s_bad);
             }
             {
                 double rmax = 0.0, amax = 0.0, xmax = 0.0, bmax = 0.0;
@@ -991,16 +1004,11 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
             }
             tc_go = s_gslot[0] == 0;
             if (s_gslot[0]) {
-                // fall back to partial pivoting on the original system
-                if (L::SD_ALIAS || L::INV_ALIAS) {
-                    force_piv = true;            // the right-hand sides' inputs are overwritten (by SD,
-                    __syncthreads();             // or by the FP32 inverse): evaluate the element again
-                    goto elem_start;
-                } else {
-                    build_rhs();
-                    __syncthreads();
-                    gj_regs<NU, 1 + NH, NT, 8, true>(s_SD, s_R, s_pcol, s_diag, s_rowvar, s_gslot, s_bad);
-                }
+                // fall back to partial pivoting: the right-hand sides' inputs are overwritten (by SD, the
+                // published column blocks or the FP32 inverse), so the element is evaluated again
+                force_piv = true;
+                __syncthreads();
+                goto elem_start;
             }
             }
             if (tid == 0 && *s_bad && !bad_before) *s_bad = 2;
