@@ -79,23 +79,15 @@ __device__ __forceinline__ bool inv8(double (&z)[2]) {
 
 // Elimination orders: position i of the order -> row of the system.
 struct NaturalOrder {
-    __device__ __forceinline__ static int at(int i) { return i; }
+    __device__ __forceinline__ int operator()(int i) const { return i; }
 };
-// Local system of NCU components of NPV nodes (row = node + NPV component): the first two momentum
-// components node by node, so that the 2 x 2 pivots of inv8 are a node's, the other components, the
-// density last (an interior node has no density pivot before that: the continuity flux does not
-// depend on the density).  Without pivoting, largest error of the Jacobian columns over the local
-// systems of 2D and 3D Euler and NS states, p = 1 .. 4, against extended precision: 6e-14 (with the
-// refined inverses of block_gj); 2e-12 in the order by components with the density last.
-template <int NPV, int NCU>
-struct PairedOrder {
-    __device__ __forceinline__ static int at(int i) {
-        return i < 2 * NPV ? NPV * (1 + (i & 1)) + (i >> 1) : (i + NPV < NPV * NCU ? i + NPV : i + NPV - NPV * NCU);
-    }
+struct TableOrder {
+    const int *at;
+    __device__ __forceinline__ int operator()(int i) const { return at[i]; }
 };
 
-// Block Gauss-Jordan elimination of [A | B] (A: N x N, B: N x NR, column-major, leading dimension N)
-// without pivoting, in the order Order, B overwritten by the solution, A left as it is; by all NT
+// Block Gauss-Jordan elimination of [A | B] (A: N x N, B: N x NR, column-major, leading dimensions N
+// and LDB) without pivoting, in the order Order, B overwritten by the solution, A left as it is; by all NT
 // threads.
 //
 // The transposed system lives in C fragments: warp w holds the columns 8 c .. 8 c + 7 of [A | B] for
@@ -106,13 +98,12 @@ struct PairedOrder {
 // right factors are the 8 columns of block k, which their owner has left in shared memory (inv(D)^T
 // and -L(i)^T; rows of ten doubles, so that the fragment reads are free of bank conflicts).  While
 // the others update, the owner of block k + 1 brings its tile up to date first and inverts the next
-// diagonal tile, so one barrier per 8 unknowns remains.  REFINE: the inverse Y of a diagonal tile Q
-// gets one Newton step, Y + (I - Y Q) Y.
+// diagonal tile, so one barrier per 8 unknowns remains.
 // What bounds it: the chain of N / 8 inversions (about 1,300 cycles each), with the tensor work of
 // other resident elements beside it.  Measured in a loop, cycles per system against an elimination
 // of one unknown at a time in registers with a barrier each: N = 40, 49 right-hand sides, three
 // CTAs of 192 threads per SM: 31,500 -> 14,200; N = 60, 61, one CTA of 256: 50,200 -> 19,700; N = 50,
-// 121, one of 256: 45,700 -> 21,100; N = 24, 37, four of 128: 14,700 -> 6,500 (without REFINE).
+// 121, one of 256: 45,700 -> 21,100; N = 24, 37, four of 128: 14,700 -> 6,500.
 // pub: pub_doubles doubles of shared memory, 16-byte aligned, that overlap neither A nor B.
 // *bad = 8 k + 1 when block k is singular.
 template <int N, int NR, int NT>
@@ -121,90 +112,80 @@ struct BlockGJ {
     static constexpr int TS = 80, pub_doubles = 2 * MT * TS;
 };
 
-template <int N, int NR, int NT, bool REFINE, class Order>
-__device__ __forceinline__ void block_gj(const double *__restrict__ A, double *B, double *pub, int *bad) {
+// The owner of column block k: the inverse of its diagonal tile and its other tiles, negated, into the
+// MT tiles at `to`.
+template <int k, int MT>
+__device__ __forceinline__ void publish_tiles(double (&z)[MT][2], double *to, int *bad) {
+    constexpr int TS = 80;
+    const int lane = threadIdx.x & 31, m = lane >> 2, n0 = 2 * (lane & 3);
+    to += 10 * m + n0;
+    const bool ok = inv8(z[k]);
+    if (!ok && lane == 0 && *bad == 0) *bad = 8 * k + 1;
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+        *reinterpret_cast<double2 *>(to + i * TS) =
+            i == k ? make_double2(z[i][0], z[i][1]) : make_double2(-z[i][0], -z[i][1]);
+}
+
+// Block step k on one column block, with the tiles published at `from`
+template <int k, int MT>
+__device__ __forceinline__ void apply_step(double (&z)[MT][2], const double *from) {
+    constexpr int TS = 80;
+    const int lane = threadIdx.x & 31;
+    from += 20 * (lane & 3) + (lane >> 2);                      // element (row 2 (l % 4) + t, column l / 4)
+    double p[2] = {0.0, 0.0};
+    dmma(p, z[k][0], from[k * TS]);
+    dmma(p, z[k][1], from[k * TS + 10]);
+    z[k][0] = p[0];
+    z[k][1] = p[1];
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+        if (i != k) {
+            dmma(z[i], p[0], from[i * TS]);
+            dmma(z[i], p[1], from[i * TS + 10]);
+        }
+}
+
+template <int N, int NR, int LDB, int NT, class Order>
+__device__ __forceinline__ void block_gj(const double *__restrict__ A, double *B, double *pub, int *bad, Order order) {
     using G = BlockGJ<N, NR, NT>;
     constexpr int MT = G::MT, CT = G::CT, NW = G::NW, CPT = G::CPT, TS = G::TS;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = lane >> 2, n0 = 2 * (lane & 3);
     double z[CPT][MT][2];
+    int at[MT][2];                                              // this lane's rows
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int t = 0; t < 2; t++) at[i][t] = 8 * i + n0 + t < N ? order(8 * i + n0 + t) : 0;
 #pragma unroll
     for (int s = 0; s < CPT; s++) {
         const int c = w + s * NW, col = 8 * c + m;
-        const double *src = c < MT ? A + N * Order::at(col < N ? col : 0) : B + N * (col - 8 * MT < NR ? col - 8 * MT : 0);
+        const double *src = c < MT ? A + N * order(col < N ? col : 0) : B + LDB * (col - 8 * MT < NR ? col - 8 * MT : 0);
         const bool in = c < MT ? col < N : (c < CT && col - 8 * MT < NR);
 #pragma unroll
         for (int i = 0; i < MT; i++)
 #pragma unroll
             for (int t = 0; t < 2; t++) {
                 const int row = 8 * i + n0 + t;
-                z[s][i][t] = (in && row < N) ? src[Order::at(row)] : (c < MT && col == row ? 1.0 : 0.0);
+                z[s][i][t] = (in && row < N) ? src[at[i][t]] : (c < MT && col == row ? 1.0 : 0.0);
             }
     }
-    // the owner of column block k: inverse of its diagonal tile and its other tiles, negated
-    auto publish = [&](auto kc) {
-        constexpr int k = decltype(kc)::value, s = k / NW;
-        double *to = pub + (k & 1) * MT * TS + 10 * m + n0;
-        const double *from = pub + (k & 1) * MT * TS + 10 * n0 + m + k * TS;
-        double q0 = 0.0, q1 = 0.0;
-        if constexpr (REFINE) {                                 // the tile as a right factor
-            *reinterpret_cast<double2 *>(to + k * TS) = make_double2(z[s][k][0], z[s][k][1]);
-            __syncwarp();
-            q0 = from[0];
-            q1 = from[10];
-        }
-        const bool ok = inv8(z[s][k]);
-        if (!ok && lane == 0 && *bad == 0) *bad = 8 * k + 1;
-        if constexpr (REFINE) {
-            double e[2] = {m == n0 ? 1.0 : 0.0, m == n0 + 1 ? 1.0 : 0.0};
-            __syncwarp();
-            *reinterpret_cast<double2 *>(to + k * TS) = make_double2(z[s][k][0], z[s][k][1]);
-            dmma(e, -z[s][k][0], q0);
-            dmma(e, -z[s][k][1], q1);
-            __syncwarp();
-            q0 = from[0];
-            q1 = from[10];
-            dmma(z[s][k], e[0], q0);
-            dmma(z[s][k], e[1], q1);
-            __syncwarp();
-        }
-#pragma unroll
-        for (int i = 0; i < MT; i++)
-            *reinterpret_cast<double2 *>(to + i * TS) =
-                i == k ? make_double2(z[s][i][0], z[s][i][1]) : make_double2(-z[s][i][0], -z[s][i][1]);
-    };
     auto step = [&](auto kc) {
-        constexpr int k = decltype(kc)::value;
-        // right factors: element (row 2 (l % 4) + t, column l / 4) of tile i
-        const double *from = pub + (k & 1) * MT * TS + 10 * n0 + m;
-        auto update = [&](int s) {
-            double p[2] = {0.0, 0.0};
-            dmma(p, z[s][k][0], from[k * TS]);
-            dmma(p, z[s][k][1], from[k * TS + 10]);
-            z[s][k][0] = p[0];
-            z[s][k][1] = p[1];
-#pragma unroll
-            for (int i = 0; i < MT; i++)
-                if (i != k) {
-                    dmma(z[s][i], p[0], from[i * TS]);
-                    dmma(z[s][i], p[1], from[i * TS + 10]);
-                }
-        };
-        constexpr int sn = (k + 1) / NW;                        // the next block's slot in its owner
-        const bool next = k + 1 < MT && w == (k + 1) % NW;
-        if constexpr (k + 1 < MT) {
-            if (next) {
-                update(sn);
-                publish(std::integral_constant<int, (k + 1 < MT ? k + 1 : 0)>{});
-            }
+        constexpr int k = decltype(kc)::value, kn = k + 1 < MT ? k + 1 : k, sn = kn / NW;   // the next block, its slot
+        const double *from = pub + (k & 1) * MT * TS;
+        const bool next = k + 1 < MT && w == kn % NW;
+        if (next) {
+            apply_step<k, MT>(z[sn], from);
+            publish_tiles<kn, MT>(z[sn], pub + (kn & 1) * MT * TS, bad);
         }
 #pragma unroll
         for (int s = 0; s < CPT; s++) {
             const int c = w + s * NW;
-            if (c < CT && c > k && !(next && s == sn)) update(s);
+            if (c < CT && c > k && !(next && s == sn)) apply_step<k, MT>(z[s], from);
         }
         __syncthreads();
     };
-    if (w == 0) publish(std::integral_constant<int, 0>{});
+    if (w == 0) publish_tiles<0, MT>(z[0], pub, bad);
     __syncthreads();
     unroll_for<MT>(step);
 #pragma unroll
@@ -216,9 +197,70 @@ __device__ __forceinline__ void block_gj(const double *__restrict__ A, double *B
 #pragma unroll
                 for (int t = 0; t < 2; t++) {
                     const int row = 8 * i + n0 + t;
-                    if (row < N) B[Order::at(row) + N * col] = z[s][i][t];
+                    if (row < N) B[at[i][t] + LDB * col] = z[s][i][t];
                 }
         }
+    }
+    __syncthreads();
+}
+
+// The same elimination in two phases, for systems whose fragments do not fit the registers at once
+// (3D p = 3: 100 unknowns, 201 right-hand sides).  block_gj_factor runs the steps on A alone and keeps
+// what every step published (MT * MT tiles in `steps`, outside A); block_gj_apply then takes the right-hand
+// sides through them, each warp its own 8 columns at a time, without a barrier.
+template <int N, int NT, class Order>
+__device__ __forceinline__ void block_gj_factor(const double *A, double *steps, int *bad, Order order) {
+    constexpr int MT = (N + 7) / 8, NW = NT / 32, TS = 80;
+    static_assert(MT <= NW, "one column block per warp");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = lane >> 2, n0 = 2 * (lane & 3);
+    double z[MT][2];
+    const int col = 8 * w + m;
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            const int row = 8 * i + n0 + t;
+            z[i][t] = (w < MT && col < N && row < N) ? A[order(row) + N * order(col)] : (col == row ? 1.0 : 0.0);
+        }
+    unroll_for<MT>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        double *step = steps + k * MT * TS;
+        if (w == k) publish_tiles<k, MT>(z, step, bad);
+        __syncthreads();
+        if (w > k && w < MT) apply_step<k, MT>(z, step);
+    });
+}
+
+template <int N, int NR, int LDB, int NT, class Order>
+__device__ __forceinline__ void block_gj_apply(double *B, const double *steps, Order order) {
+    constexpr int MT = (N + 7) / 8, NW = NT / 32, TS = 80;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = lane >> 2, n0 = 2 * (lane & 3);
+    int at[MT][2];                                              // this lane's rows
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int t = 0; t < 2; t++) at[i][t] = 8 * i + n0 + t < N ? order(8 * i + n0 + t) : 0;
+    for (int c = w; c < (NR + 7) / 8; c += NW) {
+        const int col = 8 * c + m;
+        double z[MT][2];
+#pragma unroll
+        for (int i = 0; i < MT; i++)
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                const int row = 8 * i + n0 + t;
+                z[i][t] = (col < NR && row < N) ? B[at[i][t] + LDB * col] : 0.0;
+            }
+        unroll_for<MT>([&](auto kc) {
+            constexpr int k = decltype(kc)::value;
+            apply_step<k, MT>(z, steps + k * MT * TS);
+        });
+#pragma unroll
+        for (int i = 0; i < MT; i++)
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                const int row = 8 * i + n0 + t;
+                if (col < NR && row < N) B[at[i][t] + LDB * col] = z[i][t];
+            }
     }
     __syncthreads();
 }

@@ -25,6 +25,7 @@
 #include <math.h>
 #include "hdgx_common.cuh"
 #include "dmma.cuh"
+#include "element_mma.cuh"
 #include "tcgen05.cuh"
 
 namespace hdgx {
@@ -77,7 +78,7 @@ struct Dims {
     static constexpr int NGT = NGF * NFE;
 };
 
-// Shared-memory plan (in doubles).  "P" = persistent through the element, "X" = the
+// Shared-memory plan of the mixed form (in doubles).  "P" = persistent through the element, "X" = the
 // assembly-phase scratch, reused by the DUDG_DUH / AE column tiles at the end.  The scratch
 // is ordered so that everything the SD build does not read comes first (dead once the
 // right-hand sides and Rh are built); when it is large enough SD is built on top of it
@@ -112,8 +113,12 @@ constexpr TcPlace tc_place(bool mixed, int x_start, int inv_lo, int inv_hi, int 
     return {0, 16, 1, 0, 0};
 }
 
-template <class D, bool VISC, bool MIXED = false, bool TAB = true>
+template <class D, bool VISC, bool TAB = true>
 struct Plan {
+    static constexpr bool MIXED = true, WS = false;
+    // strides: flux Jacobians by component (volume, face), values at the quadrature points, right-hand sides
+    static constexpr int CW = D::NGV * D::ND * D::NCU, CF = D::NGT * D::NCU, ZV = D::NGV, ZF = D::NGT, LDR = D::NU;
+    static constexpr int SG = 0, ws_stride = 0, i_ord = 0;
     // master tables (loaded once per CTA; shapvt / shapvg stay in global memory when !TAB)
     static constexpr bool TABLES = TAB;
     static constexpr int t_vt = 0;
@@ -162,15 +167,7 @@ struct Plan {
     static constexpr int p_dudg = p_Rh + D::NH;
     static constexpr int p_jv = p_dudg + D::NQ;                   // [NGV] volume jac (time-dependent mass term)
     static constexpr int p_SDsep = p_jv + D::NGV;                 // SD when it does not fit the scratch
-    // column blocks published by the FP64 elimination of SD (block_gj): in the scratch next to SD
-    // (dead once SD is built) where they fit, else behind everything else
-    static constexpr int PUB = MIXED ? 0 : BlockGJ<D::NU, 1, 32>::pub_doubles;
-    static constexpr int pub_in = ev(x_start + (SD_ALIAS ? D::NU * D::NU : 0));
-    static constexpr bool PUB_ALIAS = pub_in + PUB <= x_end;
-    static constexpr int p_pubsep = ev(p_SDsep + (SD_ALIAS ? 0 : D::NU * D::NU));
-    static constexpr int p_pub = PUB_ALIAS ? pub_in : p_pubsep;
-    static constexpr int p_end = p_pubsep + (PUB_ALIAS ? 0 : PUB);
-    static_assert(ev(x_wrl) + BlockGJ<D::NPV, 1, 32>::pub_doubles <= x_end, "inv(M)'s column blocks fit the scratch");
+    static constexpr int p_end = p_SDsep + (SD_ALIAS ? 0 : D::NU * D::NU);
     static constexpr int p_SD = SD_ALIAS ? x_start : p_SDsep;
     // column tiles of DUDG_DUH (reuse the scratch)
     static constexpr int NCG = VISC ? D::NC : D::NCU;
@@ -217,36 +214,117 @@ struct Plan {
     static constexpr int i_bad = i_bf + D::NFE;
     static constexpr int i_tmem = i_bad + 1;              // TMEM address of the tensor-core accumulator
     static constexpr int n_ints = i_tmem + 1;
-    // Plans beyond a CTA's shared memory (3D p = 3: 520 KB for 100 unknowns and 201 right-hand
-    // sides) keep every double array in a per-CTA slice of a global workspace, read and written
-    // through L1 and L2 (one CTA per SM), with the integers in shared memory; the local system is
-    // then LU-factored and solved in shared memory (below).
-    static constexpr bool WS = sizeof(double) * n_doubles_core + sizeof(int) * n_ints > 227 * 1024;
     static constexpr int n_doubles = n_doubles_core;
-    static constexpr int ws_stride = al16(n_doubles);                       // doubles per CTA slice
-    static constexpr bool TC = !WS && TC_PL != 0 && tc_a * 8 + 16 * TC_KC * 128 <= (int)(sizeof(double) * n_doubles) &&
+    static constexpr bool TC = TC_PL != 0 && tc_a * 8 + 16 * TC_KC * 128 <= (int)(sizeof(double) * n_doubles) &&
                                TC_NP <= 256 && D::NU <= 64;
+    static constexpr size_t bytes = sizeof(double) * n_doubles + sizeof(int) * n_ints, smem_bytes = bytes;
+};
+
+// Shared-memory plan of the FP64 form (in doubles).  The products of an element run on tensor-core
+// fragments (element_mma.cuh), whose four columns or rows at a time must sit on different banks: the
+// strides below are 4 modulo 8.  The scratch has two groups: what only the right-hand sides and Rh
+// read (SD is built on top of it), and what the SD build and, after the solve, the trace Jacobian
+// read.  x_G, the trace Jacobian's factor G' = GK_u + GK_q Mi C (face unknowns by local unknowns; for
+// inviscid fluxes by the unknowns on the face alone), is formed after the solve on top of both except
+// the face values ZFc and ZFe.
+// The inviscid flux does not depend on q: its Jacobians keep the u columns only, which doubles the
+// resident elements of the inviscid shapes.
+template <class D, bool VISC>
+struct PlanMma {
+    static constexpr bool MIXED = false, TABLES = true;
+    static constexpr int NCG = VISC ? D::NC : D::NCU;
+    static constexpr int CW = pad4(D::NGV * D::ND * D::NCU), CF = pad4(D::NGT * D::NCU), ZV = pad4(D::NGV), ZF = pad4(D::NGT);
+    static constexpr int LDR = pad4(D::NU);
+    static constexpr int KQ = D::NPF * D::NCU, SG = VISC ? pad4(D::NH) : pad4(KQ);
+    static constexpr int mx(int a, int b) { return a > b ? a : b; }
+    // master tables (loaded once per CTA): values only; shapvg is read from global memory (L1)
+    static constexpr int t_vt = 0;                                // [NGV, NPV]
+    static constexpr int t_ft = t_vt + D::NGV * D::NPV;
+    static constexpr int t_fg = t_ft + D::NGF * D::NPF;
+    // scratch, first group: not read by the SD build
+    static constexpr int x_start = ev(t_fg + D::NPF * D::NGF);
+    static constexpr int x_Xx = x_start;                          // [NGV, ND, ND]
+    static constexpr int x_jac = x_Xx + D::NGV * D::ND * D::ND;
+    static constexpr int x_nl = x_jac + D::NGV;                   // [NGT, ND]
+    static constexpr int x_jf = x_nl + D::NGT * D::ND;
+    static constexpr int x_ug = x_jf + D::NGT;                    // [NGV, NC]
+    static constexpr int x_fu = x_ug + D::NGV * D::NC;            // [NGT, NC]
+    static constexpr int x_fuh = x_fu + D::NGT * D::NC;           // [NGT, NCU]
+    static constexpr int x_wrk = x_fuh + D::NGT * D::NCU;         // [NGV, ND, NCU]
+    static constexpr int x_FH = x_wrk + D::NGV * D::ND * D::NCU;  // [NGT, NCU] jac*fhat
+    static constexpr int x_BH = x_FH + D::NGT * D::NCU;           // [NGT, NCU] jac*(fbou or fhat)
+    static constexpr int x_FHh = x_BH + D::NGT * D::NCU;          // [NGT, NCU, NCU] jac*dfhat/duh
+    static constexpr int x_Ze = x_FHh + D::NGT * D::NCU * D::NCU; // [ZV, NDF, ND]
+    static constexpr int x_Zr = x_Ze + (VISC ? ZV * D::NDF * D::ND : 0);       // [NGV, NCU, ND]
+    static constexpr int x_ZFr = x_Zr + (VISC ? D::NGV * D::NCU * D::ND : 0);  // [NGT, NCU, ND]
+    static constexpr int p_M = x_ZFr + (VISC ? D::NGT * D::NCU * D::ND : 0);   // mass matrix (dead after inv(M))
+    static constexpr int p_dg = p_M + D::NPV * D::NPV, p_uh = p_dg + D::NPV * D::ND;    // the element's nodes and trace
+    static constexpr int x_dead_end = ev(mx(p_uh + D::NCU * D::NDF, x_start + D::NU * D::NU));
+    // second group
+    static constexpr int x_wrl = x_dead_end;                      // [NGV, ND, NCU | CW, NCG]
+    static constexpr int x_FHu = x_wrl + CW * NCG;                // [NGT, NCU | CF, NCG] jac*dfhat/dudg
+    static constexpr int x_Zc = x_FHu + CF * NCG;                 // [ZV, NPV, ND]
+    static constexpr int PUB = BlockGJ<D::NU, 1, 32>::pub_doubles, PUBM = BlockGJ<D::NPV, 1, 32>::pub_doubles;
+    static constexpr int GS = VISC ? D::NU * SG : D::NFE * KQ * SG;
+    // before the flux Jacobians: inv(M)'s column blocks, then SH_q / fc_q - q; after them: SD's column
+    // blocks, or what the pivoted elimination works with
+    static constexpr int p_pub = x_wrl, p_rqs = x_wrl + PUBM;
+    static constexpr int d_slots = x_wrl, d_pcol = d_slots + 4, d_diag = d_pcol + 2 * D::NU, d_fall = d_diag + D::NU;
+    static constexpr int x_ZFc = ev(mx(mx(x_Zc + (VISC ? ZV * D::NPV * D::ND : 0), mx(d_fall, x_wrl + mx(PUB, PUBM + D::NPV * D::NCU * D::ND))),
+                                       x_start + GS));
+    static constexpr int x_ZFe = x_ZFc + (VISC ? ZF * D::NPV * D::ND : 0);     // [ZF, NPV, ND], [ZF, NDF, ND]
+    static constexpr int x_w0 = x_ZFe + (VISC ? ZF * D::NDF * D::ND : 0);      // [NGV ND + NGT, NCU] of the residual column
+    static constexpr int x_end = x_w0 + (D::NGV * D::ND + D::NGT) * D::NCU;
+    static constexpr int x_G = x_start;
+    static constexpr bool SD_ALIAS = true, INV_ALIAS = false;
+    // persistent per element
+    static constexpr int p_udg = x_end, p_dudg = p_udg;           // [NPV, NC]: the state, later its update
+    static constexpr int p_R = ev(p_udg + D::NQ);                 // [NU | LDR, 1+NH]
+    static constexpr int p_MiC = p_R + LDR * (1 + D::NH);         // [NPV, NPV*ND] | MiE | MiRq contiguous
+    static constexpr int p_MiE = p_MiC + D::NPV * D::NPV * D::ND;
+    static constexpr int p_MiRq = p_MiE + D::NPV * D::NDF * D::ND;
+    static constexpr int p_Gp = p_MiRq + D::NPV * D::NCU * D::ND; // [NGT, NCU | CF, NCG] jac * dRh-flux/dudg
+    static constexpr int p_Hp = p_Gp + CF * NCG;                  // [NGT, NCU, NCU] jac * dRh-flux/duh
+    static constexpr int p_Rh = p_Hp + D::NGT * D::NCU * D::NCU;
+    static constexpr int p_jv = p_Rh + D::NH;                     // [NGV] volume jac (time-dependent mass term)
+    static constexpr int p_SD = x_start;
+    static constexpr int y_Xg = x_start;                          // [NGT, NCG] of FE
+    static constexpr int d_b0 = p_jv + D::NGV;                    // [NU] first right-hand side
+    static constexpr int d_red = d_b0 + D::NU;                    // [4, warps] of the backward-error check
+    static constexpr int d_mbar = d_red + 64, d_inv = d_mbar;
+    static constexpr int n_doubles = d_mbar;
+    static constexpr bool TC = false;
+    static constexpr int TC_KP = 8, TC_KC = 2, TC_G = 1, TC_NP = 16, TC_NB = 16, TC_NBUF = 1, TC_BSTRIDE = 0, tc_a = 0, tc_b = 0;
+    // integers (after the doubles in shared memory)
+    static constexpr int i_perm = 0;                      // [NPF, NFE] 0-based
+    static constexpr int i_invp = D::NPF * D::NFE;        // [NPV, NFE] face-local index or -1
+    static constexpr int i_piv = i_invp + D::NPV * D::NFE;
+    static constexpr int i_pivM = i_piv + D::NU;
+    static constexpr int i_rowused = i_pivM + D::NPV;
+    static constexpr int i_rowvar = i_rowused + D::NU;
+    static constexpr int i_gslot = i_rowvar + D::NU;
+    static constexpr int i_bf = i_gslot + 2;
+    static constexpr int i_bad = i_bf + D::NFE;
+    static constexpr int i_tmem = i_bad + 1;
+    static constexpr int i_ord = i_tmem + 1;              // [NU] elimination order of the local system
+    static constexpr int n_ints = i_ord + D::NU;
     static constexpr size_t bytes = sizeof(double) * n_doubles + sizeof(int) * n_ints;   // the whole plan
-    // WS shared memory, in doubles after the integers: the face tables t_ft / t_fg (ws_tabs), SD
-    // (built there and LU-factored in place, at lu_off) followed by the right-hand sides solved in
-    // LU_NCH chunks of LU_CH columns (leading dimension NU + 1 against bank conflicts); before the
-    // SD build the same space holds the first scratch group [x_start, x_dead_end) (ws_dead: on
-    // top of SD when SD is built over that group, else after it)
+    // Plans beyond a CTA's shared memory (3D p = 3) keep the double arrays in a per-CTA slice of a
+    // global workspace, read and written through L1 and L2, one CTA of 512 threads per SM.  In shared
+    // memory, after the integers: the tables, the first group with SD on top of it (ws_dead), and the
+    // tiles that the elimination of SD publishes, all steps of them (block_gj_factor), or those of
+    // inv(M), or the right-hand sides of the pivoted fallback in chunks of LU_CH columns (leading
+    // dimension NU + 1 against bank conflicts).
+    static constexpr bool WS = bytes > 227 * 1024;
+    static constexpr int ws_stride = al16(n_doubles);                       // doubles per CTA slice
     static constexpr int ws_tabs = al16((n_ints * (int)sizeof(int) + 7) / 8);
-    static constexpr int lu_off = al16(ws_tabs + 2 * D::NGF * D::NPF);
-    static constexpr int ws_dead = SD_ALIAS ? lu_off : lu_off + D::NU * D::NU;
-    static constexpr int LU_CHMAX = (227 * 1024 / 8 - lu_off - D::NU * D::NU) / (D::NU + 1);
-    static constexpr int LU_NCH = (1 + D::NH + LU_CHMAX - 1) / (LU_CHMAX > 0 ? LU_CHMAX : 1);
-    static constexpr int LU_CH = (1 + D::NH + LU_NCH - 1) / LU_NCH;
-    static constexpr int ws_smem_doubles = (lu_off + D::NU * D::NU + (D::NU + 1) * LU_CH) >
-                                                   (ws_dead + x_dead_end - x_start)
-                                               ? lu_off + D::NU * D::NU + (D::NU + 1) * LU_CH
-                                               : ws_dead + x_dead_end - x_start;
-    static constexpr size_t smem_bytes = WS ? sizeof(double) * ws_smem_doubles : bytes;   // of it in shared memory
-    static constexpr int ws_pubM = ev(ws_dead + x_dead_end - x_start);      // inv(M)'s column blocks
-    static_assert(!WS || ws_pubM + BlockGJ<D::NPV, 1, 32>::pub_doubles <= ws_smem_doubles, "they fit behind the first group");
-    static_assert(!WS || LU_CHMAX >= 1, "the LU factors and one column fit shared memory");
-    static_assert(!WS || smem_bytes <= 227 * 1024, "the shared-memory part of the plan fits");
+    static constexpr int ws_dead = al16(ws_tabs + x_start);
+    static constexpr int ws_pub = ev(ws_dead + x_dead_end - x_start);
+    static constexpr int MT = (D::NU + 7) / 8, ws_pub_doubles = mx(MT * MT * 80, PUBM);
+    static constexpr int LU_CHMAX = ws_pub_doubles / (D::NU + 1);
+    static constexpr int LU_NCH = (1 + D::NH + LU_CHMAX - 1) / LU_CHMAX, LU_CH = (1 + D::NH + LU_NCH - 1) / LU_NCH;
+    static constexpr size_t smem_bytes = WS ? sizeof(double) * (ws_pub + ws_pub_doubles) : bytes;   // of it in shared memory
+    static_assert(smem_bytes <= 227 * 1024, "the shared-memory part of the plan fits");
 };
 
 // Resident elements per SM: the kernel is latency-bound (barrier-separated phases, a 40-step
@@ -257,12 +335,11 @@ struct Plan {
 // The volume tables shapvt / shapvg move from shared to global memory (read through L1) only
 // when that raises the number of resident CTAs (2D p = 4: 119 -> 108 KB, one -> two per SM).
 constexpr int blocks_for(size_t bytes) {
-    return bytes <= 45 * 1024 ? 4 : (bytes <= 74 * 1024 ? 3 : (bytes <= 110 * 1024 ? 2 : 1));
+    return bytes <= 45 * 1024 ? 4 : (bytes <= 74 * 1024 ? 3 : (bytes <= 113 * 1024 ? 2 : 1));
 }
 template <class D, bool VISC, bool MIXED>
-using PlanSel = Plan<D, VISC, MIXED,
-                     (!Plan<D, VISC, MIXED, false>::WS &&
-                      blocks_for(Plan<D, VISC, MIXED, false>::bytes) <= blocks_for(Plan<D, VISC, MIXED, true>::bytes))>;
+using PlanSel = std::conditional_t<MIXED, Plan<D, VISC, blocks_for(Plan<D, VISC, false>::bytes) <= blocks_for(Plan<D, VISC, true>::bytes)>,
+                                   PlanMma<D, VISC>>;
 template <class D, bool VISC, bool MIXED>
 constexpr int min_blocks() { return blocks_for(PlanSel<D, VISC, MIXED>::bytes); }
 template <class D, bool VISC, bool MIXED>
@@ -293,20 +370,26 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
     extern __shared__ __align__(16) double sm[];
     // the doubles of the plan: shared memory, or this CTA's slice of the global workspace
     double *wk = L::WS ? P.ws + (size_t)blockIdx.x * L::ws_stride : sm;
-    int *si = L::WS ? reinterpret_cast<int *>(sm) : reinterpret_cast<int *>(sm + L::n_doubles);
+    int *si = reinterpret_cast<int *>(L::WS ? sm : sm + L::n_doubles);
     const int tid = threadIdx.x;
 
-    const double *t_vt = L::TABLES ? wk + L::t_vt : P.shapvt, *t_vg = L::TABLES ? wk + L::t_vg : P.shapvg;
-    // WS: the face tables, SD and the first scratch group in shared memory (see Plan)
-    double *smd = reinterpret_cast<double *>(sm);
-    double *t_ft = L::WS ? smd + L::ws_tabs : wk + L::t_ft, *t_fg = L::WS ? t_ft + NGF * NPF : wk + L::t_fg;
-    double *xd = L::WS ? smd + L::ws_dead - L::x_start : wk;     // base of the first scratch group
+    // WS: the tables, SD and the first scratch group in shared memory (see PlanMma)
+    double *smd = reinterpret_cast<double *>(sm), *tabs = wk, *xd = wk;   // base of the tables, of the first scratch group
+    if constexpr (L::WS) {
+        tabs = smd + L::ws_tabs;
+        xd = smd + L::ws_dead - L::x_start;
+    }
+    const double *t_vt = L::TABLES ? tabs + L::t_vt : P.shapvt, *t_vg = P.shapvg;
+    if constexpr (MIXED && L::TABLES) t_vg = wk + L::t_vg;
+    double *t_ft = tabs + L::t_ft, *t_fg = tabs + L::t_fg;
     const double *__restrict__ t_mv = P.shapmv;   // geometry tables: read once per element from L1
     const double *__restrict__ t_mf = P.shapmf;
     int *perm = si + L::i_perm, *invp = si + L::i_invp;
 
     // ---- master tables, once per CTA
-    if constexpr (L::TABLES) {
+    if constexpr (!MIXED) {
+        for (int i = tid; i < NGV * NPV; i += NT) tabs[L::t_vt + i] = P.shapvt[i];
+    } else if constexpr (L::TABLES) {
         for (int i = tid; i < NGV * NPV * (ND + 1); i += NT) {
             wk[L::t_vt + i] = P.shapvt[i];
             wk[L::t_vg + i] = P.shapvg[i];
@@ -320,6 +403,37 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
     for (int i = tid; i < NPV * NFE; i += NT) invp[i] = -1;
     __syncthreads();
     for (int i = tid; i < NPF * NFE; i += NT) invp[perm[i] + NPV * (i / NPF)] = i % NPF;
+    if constexpr (!MIXED) {
+        // Elimination order of the local system: the unknowns of the face nodes, then those of the
+        // interior nodes, each as the first two momentum components node by node (so that the 2 x 2
+        // pivots of inv8 are a node's), the other momentum and the energy, the density.  Where the
+        // interior nodes come last and the density after what it is transported by, no pivot is
+        // structurally zero (an interior node has no face term, and the continuity flux does not
+        // depend on the density).  Over 601 local systems (2D and 3D, p = 1 .. 4, Euler and NS, smooth and
+        // noisy states) the unpivoted block elimination in this order is off extended precision by at most
+        // 4.8e-15 of the largest entry, LAPACK's pivoted LU by 1.1e-14, the elimination by components with
+        // the density last by 9.5e-12, and, with a 2D p = 4 Euler state, 1e-7 when it pairs the momenta.
+        __syncthreads();
+        auto on_face = [&](int r) {
+            bool f = false;
+            for (int j = 0; j < NFE; j++) f |= invp[r + NPV * j] >= 0;
+            return f;
+        };
+        for (int r = tid; r < NPV; r += NT) {
+            int nface = 0, before = 0;                   // face nodes; nodes of r's kind before r
+            const bool f = on_face(r);
+            for (int s = 0; s < NPV; s++) {
+                nface += on_face(s);
+                before += s < r && on_face(s) == f;
+            }
+            int *ord = si + L::i_ord + (f ? 0 : NCU * nface);
+            const int n = f ? nface : NPV - nface;
+            ord[2 * before] = r + NPV;
+            ord[2 * before + 1] = r + 2 * NPV;
+            for (int c = 3; c < NCU; c++) ord[(c - 1) * n + before] = r + NPV * c;
+            ord[(NCU - 1) * n + before] = r;
+        }
+    }
     // mixed form: the tensor-memory accumulator of the Schur product and its mbarrier, once per CTA
     constexpr uint32_t TC_COLS = L::TC_NP <= 32 ? 32 : (L::TC_NP <= 64 ? 64 : (L::TC_NP <= 128 ? 128 : 256));
     // Kernels that hold tensor memory run one CTA per SM (the runtime limits a TMEM-allocating
@@ -344,8 +458,8 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
         tmem = *reinterpret_cast<const uint32_t *>(si + L::i_tmem);
     }
 
-    double *s_dg = wk + L::p_dg, *s_udg = wk + L::p_udg, *s_uh = wk + L::p_uh;
-    double *s_SD = L::WS ? smd + L::lu_off : wk + L::p_SD, *s_R = wk + L::p_R;
+    double *s_dg = xd + L::p_dg, *s_udg = wk + L::p_udg, *s_uh = xd + L::p_uh;
+    double *s_SD = xd + L::p_SD, *s_R = wk + L::p_R;
     double *s_MiC = wk + L::p_MiC, *s_MiE = wk + L::p_MiE, *s_MiRq = wk + L::p_MiRq;
     double *s_Gp = wk + L::p_Gp, *s_Hp = wk + L::p_Hp, *s_Rh = wk + L::p_Rh, *s_M = xd + L::p_M;
     double *s_dudg = wk + L::p_dudg, *s_jv = wk + L::p_jv;
@@ -354,7 +468,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
     double *x_wrk = xd + L::x_wrk, *x_wrl = wk + L::x_wrl, *x_FH = xd + L::x_FH, *x_BH = xd + L::x_BH;
     double *x_FHu = wk + L::x_FHu, *x_FHh = xd + L::x_FHh;
     double *x_Zc = wk + L::x_Zc, *x_Ze = xd + L::x_Ze, *x_Zr = xd + L::x_Zr;
-    double *x_ZFc = wk + L::x_ZFc, *x_ZFe = xd + L::x_ZFe, *x_ZFr = xd + L::x_ZFr;
+    double *x_ZFc = wk + L::x_ZFc, *x_ZFe = wk + L::x_ZFe, *x_ZFr = xd + L::x_ZFr;
     int *s_piv = si + L::i_piv, *s_pivM = si + L::i_pivM, *s_bf = si + L::i_bf, *s_bad = si + L::i_bad;
     int *s_rowused = si + L::i_rowused, *s_rowvar = si + L::i_rowvar, *s_gslot = si + L::i_gslot;
     unsigned long long *s_slot = reinterpret_cast<unsigned long long *>(wk + L::d_slots);
@@ -384,6 +498,12 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
             for (int i = tid; i < NCU * NDF; i += NT) s_uh[i] = g_uh[i];
             if (tid < NFE) s_bf[tid] = Q.bf[(size_t)e * NFE + tid];
             if (tid == 0) *s_bad = 0;
+            if constexpr (!MIXED) {
+                const double *__restrict__ g_sh = Q.SH + (size_t)e * NPV * NC;
+                const bool no_q = Q.QDG || Q.RU;                     // getq: q does not enter
+                for (int i = NPV * NCU + tid; i < NPV * NC; i += NT)
+                    wk[L::p_rqs + i - NPV * NCU] = (Q.SH ? g_sh[i] / Q.fc_q : 0.0) - (no_q ? 0.0 : g_udg[i]);
+            }
         }
         __syncthreads();
 
@@ -516,9 +636,13 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
             const int cq = NCU + a + NCU * d;
             double t = 0.0;
 #pragma unroll
-            for (int s = 0; s < NPV; s++)
-                t += s_M[r + NPV * s] * ((Q.SH ? g_shq[s + NPV * (a + NCU * d)] / Q.fc_q : 0.0) -
-                                         ((Q.QDG || Q.RU) ? 0.0 : s_udg[s + NPV * cq]));   // getq: q does not enter
+            for (int s = 0; s < NPV; s++) {
+                double v;
+                if constexpr (!MIXED) v = wk[L::p_rqs + s + NPV * (a + NCU * d)];
+                else v = (Q.SH ? g_shq[s + NPV * (a + NCU * d)] / Q.fc_q : 0.0) -
+                         ((Q.QDG || Q.RU) ? 0.0 : s_udg[s + NPV * cq]);   // getq: q does not enter
+                t += s_M[r + NPV * s] * v;
+            }
 #pragma unroll
             for (int s = 0; s < NPV; s++) t += s_MiC[r + NPV * (s + NPV * d)] * s_udg[s + NPV * a];
             for (int f = 0; f < NDF; f++) t -= s_MiE[r + NPV * (f + NDF * d)] * s_uh[a + NCU * f];
@@ -528,8 +652,10 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
 
         // ============================ Mi = inv(M): MiC, MiE, MiRq (schur_primal.m:86-91)
         // M is SPD (exact quadrature of phi phi jac): eliminate without pivoting
-        block_gj<NPV, NPV * ND + NDF * ND + NCU * ND, NT, false, NaturalOrder>(
-            s_M, s_MiC, L::WS ? smd + L::ws_pubM : wk + ev(L::x_wrl), s_bad);
+        double *pub = wk;                                 // column blocks of the eliminations
+        if constexpr (L::WS) pub = smd + L::ws_pub;
+        else pub = wk + ev(L::x_wrl);
+        block_gj<NPV, NPV * ND + NDF * ND + NCU * ND, NPV, NT>(s_M, s_MiC, pub, s_bad, NaturalOrder{});
         if (tid == 0 && *s_bad) *s_bad = 1;
         __syncthreads();
         if (Q.QDG) {
@@ -568,7 +694,8 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
 
         // ================================ flux / fhat / fbou at the Gauss points
         // volume: thread (g, seed); volint.m:81, 241-254
-        for (int i = tid; i < NGV * NSEED; i += NT) {
+        const int nseed = !MIXED && Q.RU ? 1 : NSEED;      // the residual alone needs no derivatives
+        for (int i = tid; i < NGV * nseed; i += NT) {
             const int g = i % NGV, sd = i / NGV;
             D1 u[NCU], q[NCU * ND], f[NCU * ND];
 #pragma unroll
@@ -588,14 +715,14 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                         dw += f[a + NCU * jd].d * xx;
                     }
                     if (sd == 0) x_wrk[g + NGV * (id + ND * a)] = w;
-                    x_wrl[g + NGV * (id + ND * (a + NCU * sd))] = -dw;
+                    x_wrl[g + NGV * (id + ND * a) + L::CW * sd] = -dw;
                 }
         }
-        if constexpr (!VISC) {
+        if constexpr (!VISC && MIXED) {
             for (int i = tid; i < NGV * ND * NCU * (NC - NCU); i += NT) x_wrl[NGV * ND * NCU * NCU + i] = 0.0;
         }
         // faces: thread (gg, seed); fhat.m:49-67 = f(uh,q).n + tau (u - uh)
-        for (int i = tid; i < NGT * NSEED; i += NT) {
+        for (int i = tid; i < NGT * nseed; i += NT) {
             const int gg = i % NGT, sd = i / NGT;
             D1 u[NCU], q[NCU * ND], f[NCU * ND];
 #pragma unroll
@@ -631,14 +758,14 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                     const double fhh = dfn - (a == sd ? Q.pc.tau : 0.0);
                     const double fhu = (a == sd ? Q.pc.tau : 0.0);
                     x_FHh[gg + NGT * (a + NCU * sd)] = jc * fhh;
-                    x_FHu[gg + NGT * (a + NCU * sd)] = jc * fhu;
+                    x_FHu[gg + NGT * a + L::CF * sd] = jc * fhu;
                     if (!gen) {
                         s_Hp[gg + NGT * (a + NCU * sd)] = jc * (dir ? (a == sd ? 1.0 : 0.0) : fhh);
-                        s_Gp[gg + NGT * (a + NCU * sd)] = jc * (dir ? 0.0 : fhu);
+                        s_Gp[gg + NGT * a + L::CF * sd] = jc * (dir ? 0.0 : fhu);
                     }
                 } else {
-                    x_FHu[gg + NGT * (a + NCU * sd)] = jc * dfn;
-                    if (!gen) s_Gp[gg + NGT * (a + NCU * sd)] = jc * (dir ? 0.0 : dfn);
+                    x_FHu[gg + NGT * a + L::CF * sd] = jc * dfn;
+                    if (!gen) s_Gp[gg + NGT * a + L::CF * sd] = jc * (dir ? 0.0 : dfn);
                 }
             }
             if (gen) {
@@ -662,7 +789,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                 for (int a = 0; a < NCU; a++) {
                     if (sd == 0) x_BH[gg + NGT * a] = jc * fb[a].v;
                     if (sd < NCU) s_Hp[gg + NGT * (a + NCU * sd)] = jc * fb[a].d;
-                    else s_Gp[gg + NGT * (a + NCU * sd)] = jc * fb[a].d;
+                    else s_Gp[gg + NGT * a + L::CF * sd] = jc * fb[a].d;
                 }
                 if (sd < NCU) {
 #pragma unroll
@@ -672,31 +799,31 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                     }
                     fbou_point<ND>(Q.fb, Q.pc, btype, ub, nlp, uu, qq, hh, fb);
 #pragma unroll
-                    for (int a = 0; a < NCU; a++) s_Gp[gg + NGT * (a + NCU * sd)] = jc * fb[a].d;
+                    for (int a = 0; a < NCU; a++) s_Gp[gg + NGT * a + L::CF * sd] = jc * fb[a].d;
                 }
             }
         }
-        if constexpr (!VISC) {
+        if constexpr (!VISC && MIXED) {
             for (int i = tid; i < NGT * NCU * (NC - NCU); i += NT) {
                 x_FHu[NGT * NCU * NCU + i] = 0.0;
                 s_Gp[NGT * NCU * NCU + i] = 0.0;
             }
         }
         // Mi C, Mi E, Mi Rq at the volume and face Gauss points (only B couples through them)
-        if constexpr (VISC) {
+        if (VISC && (MIXED || !Q.RU)) {
             for (int i = tid; i < NGV * NPV * ND; i += NT) {
                 const int g = i % NGV, kd = i / NGV;
                 double t = 0.0;
 #pragma unroll
                 for (int s = 0; s < NPV; s++) t += t_vt[g + NGV * s] * s_MiC[s + NPV * kd];
-                x_Zc[i] = t;
+                x_Zc[g + L::ZV * kd] = t;
             }
             for (int i = tid; i < NGV * NDF * ND; i += NT) {
                 const int g = i % NGV, fd = i / NGV;
                 double t = 0.0;
 #pragma unroll
                 for (int s = 0; s < NPV; s++) t += t_vt[g + NGV * s] * s_MiE[s + NPV * fd];
-                x_Ze[i] = t;
+                x_Ze[g + L::ZV * fd] = t;
             }
             for (int i = tid; i < NGV * NCU * ND; i += NT) {
                 const int g = i % NGV, bd = i / NGV;
@@ -710,14 +837,14 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                 double t = 0.0;
 #pragma unroll
                 for (int n = 0; n < NPF; n++) t += t_ft[g + NGF * n] * s_MiC[perm[n + NPF * j] + NPV * kd];
-                x_ZFc[i] = t;
+                x_ZFc[gg + L::ZF * kd] = t;
             }
             for (int i = tid; i < NGT * NDF * ND; i += NT) {
                 const int gg = i % NGT, fd = i / NGT, g = gg % NGF, j = gg / NGF;
                 double t = 0.0;
 #pragma unroll
                 for (int n = 0; n < NPF; n++) t += t_ft[g + NGF * n] * s_MiE[perm[n + NPF * j] + NPV * fd];
-                x_ZFe[i] = t;
+                x_ZFe[gg + L::ZF * fd] = t;
             }
             for (int i = tid; i < NGT * NCU * ND; i += NT) {
                 const int gg = i % NGT, bd = i / NGT, g = gg % NGF, j = gg / NGF;
@@ -738,6 +865,146 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
         // W is formed on the fly, once per register tile.
         constexpr int KV = NGV * ND, KK = KV + NFE * NGF;
         constexpr int TMS = NPV <= 6 ? NPV : (NPV + 1) / 2;
+        // The FP64 form: the same sums on tensor-core fragments, columns (k, b) of SD and (b, f) of the
+        // right-hand sides as their rows (column_product).
+        // the left factors at a volume (g, id) or face (gg) point for column unknown (k, b) and flux Jacobian J
+        auto left_node = [&](const double *J, double shape, const double *Zk, int zs, int ys, int cs, double (&w)[NCU]) {
+            double z[1 + ND];
+            z[0] = shape;
+#pragma unroll
+            for (int d = 0; d < ND; d++) z[1 + d] = VISC ? Zk[zs * d] : 0.0;
+#pragma unroll
+            for (int a = 0; a < NCU; a++) {
+                w[a] = J[ys * a] * z[0];
+                if constexpr (VISC) {
+#pragma unroll
+                    for (int d = 0; d < ND; d++) w[a] += J[ys * a + cs * NCU * (1 + d)] * z[1 + d];
+                }
+            }
+        };
+        auto right_v = [&](int r, int kk) { return t_vg[r + NPV * (kk + NGV)]; };   // shapvg(r, g, id + 1), kk = g + NGV id
+        auto right_f = [&](int r, int kf) {
+            const int m = invp[r + NPV * (kf / NGF)];
+            return m >= 0 ? t_fg[m + NPF * (kf % NGF)] : 0.0;
+        };
+        // the face point's factor for local unknown (k, b), J = FHu (SD) or Gp (trace Jacobian)
+        auto left_face = [&](const double *J, int k, int b, int kf, double (&w)[NCU]) {
+            const int nk = invp[k + NPV * (kf / NGF)];
+            left_node(J + kf + L::CF * b, nk >= 0 ? t_ft[kf % NGF + NGF * nk] : 0.0, x_ZFc + kf + L::ZF * k, L::ZF * NPV, NGT,
+                      L::CF, w);
+        };
+        double *x_w0 = wk + L::p_dudg;
+        if constexpr (!MIXED) x_w0 = wk + L::x_w0;
+        auto mma_residual = [&]() {
+            // the residual column Ru - B Mi Rq: four lanes a row
+            for (int i = tid; i < (4 * NU + 31) / 32 * 32; i += NT) {
+                const int row = i >> 2, r = row % NPV, a = row / NPV;
+                double v = 0.0;
+                if (row < NU) {
+                    for (int kk = i & 3; kk < KV; kk += 4) v += right_v(r, kk) * x_w0[kk + (KV + NGT) * a];
+                    for (int kf = i & 3; kf < NGT; kf += 4) v += right_f(r, kf) * x_w0[KV + kf + (KV + NGT) * a];
+                    if (Q.tdep) {
+                        // s = SH_u - fc_u u at the volume Gauss points, Ru += shapvg(:,:,1) (s jac)
+                        // (volint.m:180-221 with dtcoef = 1 and no axisymmetry; volint.m:241,258)
+                        const double *__restrict__ g_sh = Q.SH ? Q.SH + (size_t)e * NPV * NC + NPV * a : nullptr;
+                        for (int g = i & 3; g < NGV; g += 4) {
+                            double st = 0.0, ug = 0.0;
+#pragma unroll
+                            for (int s = 0; s < NPV; s++) {
+                                st += t_vt[g + NGV * s] * (g_sh ? g_sh[s] : 0.0);
+                                ug += t_vt[g + NGV * s] * s_udg[s + NPV * a];
+                            }
+                            v += t_vg[r + NPV * g] * ((st - ug * Q.fc_u) * s_jv[g]);
+                        }
+                    }
+                }
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if (row < NU && (i & 3) == 0) s_R[row] = v;
+            }
+        };
+        auto mma_sd = [&]() {
+            column_product<NCU, NPV, KV, NGT, NU, NT>(
+                [&](int c, int kk, double (&w)[NCU]) {
+                    const int k = c % NPV, b = c / NPV, g = kk % NGV;
+                    left_node(x_wrl + kk + L::CW * b, t_vt[g + NGV * k], x_Zc + g + L::ZV * k, L::ZV * NPV, NGV * ND, L::CW, w);
+                },
+                right_v, [&](int c, int kf, double (&w)[NCU]) { left_face(x_FHu, c % NPV, c / NPV, kf, w); }, right_f,
+                [&](int c, int a, int r, double v) {
+                    const int k = c % NPV, b = c / NPV;
+                    if (Q.tdep && a == b) {
+                        // time-dependent problems: the source Jacobian -fc_u on the u components
+                        // (volint.m:215-216) enters BD, hence D, as fc_u * sum_g phi_r phi_k w_g jac_g
+                        double mu = 0.0;
+#pragma unroll
+                        for (int g = 0; g < NGV; g++) mu += t_vg[r + NPV * g] * t_vt[g + NGV * k] * s_jv[g];
+                        v += Q.fc_u * mu;
+                    }
+                    s_SD[(r + NPV * a) + NU * c] = v;
+                });
+            mma_residual();
+        };
+        auto mma_rhs = [&]() {
+            // the residual column at the quadrature points (volint.m:258, faceint.m:306-331; schur_primal.m:95,111)
+            for (int i = tid; i < (KV + NGT) * NCU; i += NT) {
+                const int kk = i % (KV + NGT), a = i / (KV + NGT), kf = kk - KV;
+                double w = kk < KV ? x_wrk[kk + KV * a] : -x_FH[kf + NGT * a];
+                if (VISC && !Q.RU) {
+                    const double *J = kk < KV ? x_wrl + kk + NGV * ND * a + L::CW * NCU : x_FHu + kf + NGT * a + L::CF * NCU;
+                    const double *Zr = kk < KV ? x_Zr + kk % NGV : x_ZFr + kf;
+                    const int js = kk < KV ? L::CW : L::CF, zs = kk < KV ? NGV : NGT;
+                    double s[2] = {};
+#pragma unroll 4
+                    for (int bd = 0; bd < NCU * ND; bd++) s[bd & 1] += J[js * bd] * Zr[zs * bd];
+                    w -= s[0] + s[1];
+                }
+                x_w0[i] = w;
+            }
+            if (Q.RU) return;
+            // RHS((r,a), (b,f)) = B Mi E - F   (schur_primal.m:98,118; faceint.m:319-333)
+            if constexpr (VISC) {
+                column_product<NCU, NPV, KV, NGT, NH, NT>(
+                    [&](int c, int kk, double (&w)[NCU]) {
+                        const int b = c % NCU, f = c / NCU;
+                        const double *J = x_wrl + kk + L::CW * (NCU + b), *Z = x_Ze + kk % NGV + L::ZV * f;
+#pragma unroll
+                        for (int d = 0; d < ND; d++) {
+                            const double z = Z[L::ZV * NDF * d];
+#pragma unroll
+                            for (int a = 0; a < NCU; a++) w[a] += J[NGV * ND * a + L::CW * NCU * d] * z;
+                        }
+                    },
+                    right_v,
+                    [&](int c, int kf, double (&w)[NCU]) {
+                        const int b = c % NCU, f = c / NCU;
+                        if (f / NPF == kf / NGF) {
+                            const double z = t_ft[kf % NGF + NGF * (f % NPF)];
+#pragma unroll
+                            for (int a = 0; a < NCU; a++) w[a] = -x_FHh[kf + NGT * (a + NCU * b)] * z;
+                        }
+                        const double *J = x_FHu + kf + L::CF * (NCU + b), *Z = x_ZFe + kf + L::ZF * f;
+#pragma unroll
+                        for (int d = 0; d < ND; d++) {
+                            const double z = Z[L::ZF * NDF * d];
+#pragma unroll
+                            for (int a = 0; a < NCU; a++) w[a] += J[NGT * a + L::CF * NCU * d] * z;
+                        }
+                    },
+                    right_f, [&](int c, int a, int r, double v) { s_R[L::LDR * (1 + c) + r + NPV * a] = v; });
+            } else {
+                for (int i = tid; i < NU * NH; i += NT) {
+                    const int row = i % NU, c = i / NU, r = row % NPV, a = row / NPV, b = c % NCU, f = c / NCU;
+                    const int nf = f % NPF, jf = f / NPF, mf = invp[r + NPV * jf];
+                    double t = 0.0;
+                    if (mf >= 0) {
+#pragma unroll
+                        for (int g = 0; g < NGF; g++)
+                            t -= t_fg[mf + NPF * g] * t_ft[g + NGF * nf] * x_FHh[(g + NGF * jf) + NGT * (a + NCU * b)];
+                    }
+                    s_R[L::LDR * (1 + c) + row] = t;
+                }
+            }
+        };
         auto phi = [&](int, int r, int kk) -> double {
             if (kk < KV) return t_vg[r + NPV * (kk + NGV)];      // shapvg(r, g, id + 1), kk = g + NGV id
             const int kf = kk - KV, j = kf / NGF, g = kf % NGF, m = invp[r + NPV * j];
@@ -856,10 +1123,15 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                 s_R[NU + (r + NPV * a) + NU * (b + NCU * f)] = v;
             });
         };
-        build_rhs();
+        if constexpr (MIXED) build_rhs();
+        else mma_rhs();
         if (Q.RU) {
             // cuda_residual.m: the element u residual Ru (volume and face terms, time source)
             __syncthreads();
+            if constexpr (!MIXED) {
+                mma_residual();
+                __syncthreads();
+            }
             for (int i = tid; i < NU; i += NT) Q.RU[(size_t)e * NU + i] = s_R[i];
             if (tid == 0 && Q.status) Q.status[e] = *s_bad;
             __syncthreads();
@@ -873,7 +1145,8 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
             s_Rh[i] = -t;
         }
         if constexpr (L::SD_ALIAS) __syncthreads();     // SD overwrites what the RHS and Rh read
-        build_sd();
+        if constexpr (MIXED) build_sd();
+        else mma_sd();
         __syncthreads();
 
         // ================================ LU of SD and the 1 + NH solves (schur_primal.m:111,118)
@@ -881,12 +1154,13 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
             int bad_before = *s_bad;
             bool tc_go = false;          // the unpivoted mixed solve passed its check: Schur product next
             __syncthreads();
-            if constexpr (L::WS) {
+            if (force_piv) {
+                if constexpr (L::WS) {
                 // LU with partial pivoting of SD in shared memory (dgesv's factorisation), then the
                 // 1 + NH right-hand sides in chunks: gathered in the pivot order, forward and back
                 // substitution in shared memory, the solution written straight to s_R
                 constexpr int NU1 = NU + 1, CH = L::LU_CH;
-                double *l_LU = s_SD, *l_B = l_LU + NU * NU;   // SD is built in shared memory: factored in place
+                double *l_LU = s_SD, *l_B = smd + L::ws_pub;  // SD is built in shared memory: factored in place
                 int *ip = s_rowvar;                      // row of SD that ends up at position i
                 block_lu<NT>(l_LU, NU, NU, s_piv, s_bad);
                 if (tid == 0) {
@@ -902,7 +1176,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                     const int nc = (1 + NH - c0) < CH ? (1 + NH - c0) : CH;
                     for (int t = tid; t < NU * nc; t += NT) {
                         const int i = t % NU, j = t / NU;
-                        l_B[i + NU1 * j] = s_R[ip[i] + NU * (c0 + j)];
+                        l_B[i + NU1 * j] = s_R[ip[i] + L::LDR * (c0 + j)];
                     }
                     __syncthreads();
                     for (int k = 0; k < NU - 1; k++) {       // L y = P b (unit lower triangle)
@@ -918,20 +1192,23 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                         for (int t = tid; t < (k + 1) * nc; t += NT) {
                             const int i = t % (k + 1), j = t / (k + 1);
                             const double xk = l_B[k + NU1 * j] / ukk;
-                            if (i == k) s_R[k + NU * (c0 + j)] = xk;
+                            if (i == k) s_R[k + L::LDR * (c0 + j)] = xk;
                             else l_B[i + NU1 * j] -= l_LU[i + NU * k] * xk;
                         }
                         __syncthreads();
                     }
                 }
-            } else if (force_piv) {
-                gj_regs<NU, 1 + NH, NT, 8, true>(s_SD, s_R, s_pcol, s_diag, s_rowvar, s_gslot, s_bad);
+                } else {
+                    gj_regs<NU, 1 + NH, NT, 8, true, L::LDR>(s_SD, s_R, s_pcol, s_diag, s_rowvar, s_gslot, s_bad);
+                }
             } else {
             // Unpivoted elimination with the density unknowns last (in natural order interior
             // nodes have structurally zero density pivots: the continuity flux does not depend on
-            // the density), accepted when the backward error of the first column,
-            // |b0 - SD x0| / (|SD| |x0| + |b0|) (infinity norms), is below 1e-13; otherwise the
-            // element is redone with partial pivoting in FP64.
+            // the density; in the FP64 form the order set up above), accepted when the backward error of the first column,
+            // |b0 - SD x0| / (|SD| |x0| + |b0|) (infinity norms), is below kBackwardError (2e-15, where a
+            // sound elimination leaves 1.2e-16 at most; 1e-13 in the mixed form); otherwise the element
+            // is redone with partial pivoting in FP64.
+            constexpr double kBackwardError = MIXED ? 1e-13 : 2e-15;
             double *s_b0 = wk + L::d_b0;
             for (int i = tid; i < NU; i += NT) s_b0[i] = s_R[i];
             __syncthreads();
@@ -960,7 +1237,13 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                     __syncthreads();
                 }
             } else {
-                block_gj<NU, 1 + NH, NT, true, PairedOrder<NPV, NCU>>(s_SD, s_R, wk + L::p_pub, s_bad);
+                const TableOrder order{si + L::i_ord};
+                if constexpr (L::WS) {
+                    block_gj_factor<NU, NT>(s_SD, smd + L::ws_pub, s_bad, order);
+                    block_gj_apply<NU, 1 + NH, L::LDR, NT>(s_R, smd + L::ws_pub, order);
+                } else {
+                    block_gj<NU, 1 + NH, L::LDR, NT>(s_SD, s_R, wk + L::p_pub, s_bad, order);
+                }
             }
             {
                 double rmax = 0.0, amax = 0.0, xmax = 0.0, bmax = 0.0;
@@ -984,6 +1267,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                     bmax = fmax(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
                 }
                 double *red = s_pcol;   // free after the elimination
+                if constexpr (!MIXED) red = wk + L::d_red;
                 if ((tid & 31) == 0) {
                     red[4 * (tid >> 5) + 0] = rmax; red[4 * (tid >> 5) + 1] = amax;
                     red[4 * (tid >> 5) + 2] = xmax; red[4 * (tid >> 5) + 3] = bmax;
@@ -996,7 +1280,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                         X = fmax(X, red[4 * w + 2]); B = fmax(B, red[4 * w + 3]);
                     }
                     const double den = A * X + B;
-                    const bool ok = (*s_bad == bad_before) && (R <= 1e-13 * den) && isfinite(R);
+                    const bool ok = (*s_bad == bad_before) && (R <= kBackwardError * den) && isfinite(R);
                     s_gslot[0] = ok ? 0 : 1;
                     if (!ok) *s_bad = bad_before;
                 }
@@ -1135,7 +1419,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                 for (int g = 0; g < NGF; g++) {
                     const int gg = g + NGF * j;
                     double y = 0.0;
-                    for (int c = 0; c < NCG; c++) y += s_Gp[gg + NGT * (a + NCU * c)] * Xg[gg + NGT * c];
+                    for (int c = 0; c < NCG; c++) y += s_Gp[gg + NGT * a + L::CF * c] * Xg[gg + NGT * c];
                     t += t_fg[n + NPF * g] * y;
                 }
                 g_fe[i] = s_Rh[i] - t;
@@ -1143,14 +1427,111 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
             __syncthreads();
         }
 
-        // ============ DUDG_DUH and AE = H + GK DUDG_DUH in column tiles (schur_primal.m:136-147)
-        // Each column tile runs four batched small GEMMs with register tiles:
+        // ============ DUDG_DUH and AE = H + GK DUDG_DUH (schur_primal.m:136-147)
+        // The FP64 form: with DUDG_DUH = [dlu, Mi C dlu - Mi E] on the q rows,
+        //   AE = (H - GK_q Mi E) + G' dlu,   G' = GK_u + GK_q Mi C,
+        // both factors summed face by face like the face terms of SD and of the right-hand sides.
+        // First H - GK_q Mi E goes to AE, G' to the scratch and DUDG_DUH out; then AE += G' dlu.
+        auto mma_out = [&](auto nco_c) {
+            constexpr int NCO = decltype(nco_c)::value;
+            [[maybe_unused]] constexpr int KQ = NPF * NCU;
+            double *g_dd = Q.DUDG_DUH + (size_t)e * NPV * NCO * NH;     // [npv, nco, ncu, ndf]
+            double *g_ae = Q.AE + (size_t)e * NH * NH;
+            const bool wide = (((size_t)g_dd | (size_t)g_ae) & 15) == 0;
+            double *G = wk + L::x_start;
+            if constexpr (VISC) {
+                face_product<NCU, NPF, NFE, NGF, NU, NT>(
+                    t_fg, [&](int c, int j, int g, double (&w)[NCU]) { left_face(s_Gp, c % NPV, c / NPV, g + NGF * j, w); },
+                    [&](int c, int a, int n, int j, double v) { G[c * L::SG + a + NCU * (n + NPF * j)] = v; });
+                face_product<NCU, NPF, NFE, NGF, NH, NT>(
+                    t_fg,
+                    [&](int c, int j, int g, double (&w)[NCU]) {
+                        const int b = c % NCU, f = c / NCU, kf = g + NGF * j;
+                        if (f / NPF == j) {
+                            const double z = t_ft[g + NGF * (f % NPF)];
+#pragma unroll
+                            for (int a = 0; a < NCU; a++) w[a] = s_Hp[kf + NGT * (a + NCU * b)] * z;
+                        }
+#pragma unroll
+                        for (int d = 0; d < ND; d++) {
+                            const double z = x_ZFe[kf + L::ZF * (f + NDF * d)];
+#pragma unroll
+                            for (int a = 0; a < NCU; a++) w[a] -= s_Gp[kf + NGT * a + L::CF * (NCU + b + NCU * d)] * z;
+                        }
+                    },
+                    [&](int c, int a, int n, int j, double v) { g_ae[NH * c + a + NCU * (n + NPF * j)] = v; });
+            } else {
+                // inviscid: both are zero between a face's unknowns and what is not on the face
+                face_product<NCU, NPF, NFE, NGF, KQ, NT>(
+                    t_fg,
+                    [&](int c, int j, int g, double (&w)[NCU]) {
+                        const double z = t_ft[g + NGF * (c % NPF)];
+#pragma unroll
+                        for (int a = 0; a < NCU; a++) w[a] = s_Gp[g + NGF * j + NGT * a + L::CF * (c / NPF)] * z;
+                    },
+                    [&](int c, int a, int n, int j, double v) { G[(KQ * j + c) * L::SG + a + NCU * n] = v; });
+                face_product<NCU, NPF, NFE, NGF, KQ, NT>(
+                    t_fg,
+                    [&](int c, int j, int g, double (&w)[NCU]) {
+                        const double z = t_ft[g + NGF * (c / NCU)];
+#pragma unroll
+                        for (int a = 0; a < NCU; a++) w[a] = s_Hp[g + NGF * j + NGT * (a + NCU * (c % NCU))] * z;
+                    },
+                    [&](int c, int a, int n, int j, double v) { g_ae[NH * (c + KQ * j) + a + NCU * (n + NPF * j)] = v; });
+            }
+            for (int i = tid; i < NU * NH; i += NT) {
+                const int ru = i % NU, k = i / NU;
+                g_dd[(size_t)NPV * NCO * k + ru] = s_R[L::LDR * (1 + k) + ru];
+            }
+            if constexpr (NCO == NC) {
+                // q rows (r, a, d) of column k: columns (a, k), outputs (r, d)
+                matrix_product<NCU * NH, NPV * ND, NPV, NT>(
+                    0,
+                    [&](int ak, int o) {
+                        const int k = ak / NCU, r = o % NPV, d = o / NPV;
+                        return ak % NCU == k % NCU ? -s_MiE[r + NPV * (k / NCU + NDF * d)] : 0.0;
+                    },
+                    [&](int ak, int sx) { return s_R[L::LDR * (1 + ak / NCU) + NPV * (ak % NCU) + sx]; },
+                    [&](int sx, int o) { return s_MiC[o % NPV + NPV * (sx + NPV * (o / NPV))]; },
+                    [&](int ak, int o, double v0, double v1, int n) {
+                        double *to = g_dd + (size_t)NQ * (ak / NCU) + NPV * (NCU + ak % NCU);
+                        auto at = [&](int x) { return x % NPV + NPV * NCU * (x / NPV); };
+                        if constexpr (NPV % 2 == 0) {
+                            store2(to + at(o), v0, v1, wide);
+                        } else {
+                            to[at(o)] = v0;
+                            if (n == 2) to[at(o + 1)] = v1;
+                        }
+                    });
+            }
+            __syncthreads();
+            if constexpr (VISC) {
+                matrix_product<NH, NH, NU, NT>(
+                    0, [&](int c, int o) { return g_ae[NH * c + o]; },
+                    [&](int c, int k) { return s_R[L::LDR * (1 + c) + k]; }, [&](int k, int o) { return G[k * L::SG + o]; },
+                    [&](int c, int o, double v0, double v1, int) { store2(g_ae + NH * c + o, v0, v1, wide); });
+            } else {
+                int first = 0;
+                for (int j = 0; j < NFE; j++)
+                    first = matrix_product<NH, KQ, KQ, NT>(
+                        first, [&](int c, int o) { return c / KQ == j ? g_ae[NH * c + KQ * j + o] : 0.0; },
+                        [&](int c, int k) { return s_R[L::LDR * (1 + c) + perm[k % NPF + NPF * j] + NPV * (k / NPF)]; },
+                        [&](int k, int o) { return G[(KQ * j + k) * L::SG + o]; },
+                        [&](int c, int o, double v0, double v1, int n) {
+                            double *to = g_ae + NH * c + KQ * j + o;
+                            if (n == 2) store2(to, v0, v1, wide && KQ % 2 == 0);
+                            else *to = v0;
+                        });
+            }
+        };
+        // The mixed form, in column tiles.  Each column tile runs four batched small GEMMs with register tiles:
         //   X   = DUDG_DUH columns: u rows copied from the solve, q rows = MiC dlu - MiE
         //   Xg  = X at the face Gauss points (shapft through perm), per face
         //   Y   = Gp Xg, per face Gauss point (GK applied without forming it)
         //   AE  = shapfg Y (+ the face-block-diagonal H), per face
         // nco (components stored per row block) is a compile-time constant inside the tiles
         auto tiles = [&](auto nco_c) {
+            if constexpr (MIXED) {
             constexpr int NCO = decltype(nco_c)::value;
             constexpr int T = L::TILE;
             constexpr int TMQ = NPV <= 6 ? NPV : (NPV + 1) / 2;
@@ -1214,9 +1595,15 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                     });
                 __syncthreads();
             }
+            }
         };
-        if (Q.nco == NC) tiles(std::integral_constant<int, NC>{});
-        else tiles(std::integral_constant<int, NCU>{});
+        if constexpr (MIXED) {
+            if (Q.nco == NC) tiles(std::integral_constant<int, NC>{});
+            else tiles(std::integral_constant<int, NCU>{});
+        } else {
+            if (Q.nco == NC) mma_out(std::integral_constant<int, NC>{});
+            else mma_out(std::integral_constant<int, NCU>{});
+        }
         if (tid == 0 && Q.status) Q.status[e] = *s_bad;
         __syncthreads();
     }
@@ -1235,7 +1622,6 @@ template <class D, bool VISC, bool MIXED, class Arg>
 int launch_t(const Arg &p, int ne, cudaStream_t st, int grid_req) {
     constexpr int NT = cta_threads<D, VISC, MIXED>();
     using L = PlanSel<D, VISC, MIXED>;
-    static_assert(L::TILE >= 1, "tile");
     const size_t smem = L::smem_bytes;
     if (smem > 227 * 1024) return -3;
     auto kern = elemental_kernel<D, VISC, MIXED, NT, Arg>;

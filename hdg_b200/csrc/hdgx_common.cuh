@@ -470,7 +470,7 @@ __device__ void block_gauss_jordan(double *A, int lda, double *B, int ldb, int n
 }
 
 // Gauss-Jordan elimination of the augmented system [A | B] (A: N x N, B: N x NR, both
-// column-major with leading dimension N, in shared memory) with the matrix held in
+// column-major with leading dimensions N and LDB, in shared memory) with the matrix held in
 // REGISTERS: thread (tr, tc) = (tid % TR, tid / TR) owns rows tr + i*TR and columns
 // tc + jj*TC of the augmented matrix.  Per step k: the pivot row is broadcast inside each
 // TR-lane group with __shfl_sync, the multipliers come from a shared copy of column k that
@@ -480,7 +480,7 @@ __device__ void block_gauss_jordan(double *A, int lda, double *B, int ldb, int n
 // order.  PIVOT = false eliminates in natural order (SPD matrices).  *bad = k+1 for the
 // first zero or non-finite pivot.  Shared scratch: pcol[2N] (column copy, double-buffered),
 // diag[N], rowvar[N] (ints), slot[2] (ints).
-template <typename T, int N, int NR1, int NR2, bool IDENT2, int NT, int TR, bool PIVOT>
+template <typename T, int N, int NR1, int NR2, bool IDENT2, int NT, int TR, bool PIVOT, int LDB = N>
 __device__ __forceinline__ void gj_regs_t(const double *__restrict__ A, double *B, double *B2, T *pcol, T *diag,
                                           int *rowvar, int *slot, int *bad) {
     constexpr int NR = NR1 + NR2;
@@ -500,7 +500,7 @@ __device__ __forceinline__ void gj_regs_t(const double *__restrict__ A, double *
             double v = 0.0;
             if (r < N && j < NCOL) {
                 if (j < N) v = A[r + N * j];
-                else if (j < N + NR1) v = B[r + N * (j - N)];
+                else if (j < N + NR1) v = B[r + LDB * (j - N)];
                 else v = IDENT2 ? ((j - N - NR1 == r) ? 1.0 : 0.0) : B2[r + N * (j - N - NR1)];
             }
             a[i][jj] = (T)v;
@@ -581,16 +581,16 @@ __device__ __forceinline__ void gj_regs_t(const double *__restrict__ A, double *
             if (r < N && j >= N && j < NCOL) {
                 const int var = rowvar[r];
                 const double v = (double)(a[i][jj] / diag[var]);
-                if (j < N + NR1) B[var + N * (j - N)] = v;
+                if (j < N + NR1) B[var + LDB * (j - N)] = v;
                 else B2[var + N * (j - N - NR1)] = v;
             }
         }
     __syncthreads();
 }
-template <int N, int NR, int NT, int TR, bool PIVOT>
+template <int N, int NR, int NT, int TR, bool PIVOT, int LDB = N>
 __device__ __forceinline__ void gj_regs(const double *__restrict__ A, double *B, double *pcol, double *diag,
                                         int *rowvar, int *slot, int *bad) {
-    gj_regs_t<double, N, NR, 0, false, NT, TR, PIVOT>(A, B, nullptr, pcol, diag, rowvar, slot, bad);
+    gj_regs_t<double, N, NR, 0, false, NT, TR, PIVOT, LDB>(A, B, nullptr, pcol, diag, rowvar, slot, bad);
 }
 
 // Unpivoted Gauss-Jordan on [A | B] with the matrix in registers (layout as gj_regs), the
@@ -699,11 +699,6 @@ __device__ __forceinline__ void gj_regs_nopiv_t(const double *__restrict__ A, do
             }
         }
     __syncthreads();
-}
-
-template <int N, int NR, int NT, int TR, int ROT = 0>
-__device__ __forceinline__ void gj_regs_nopiv(const double *__restrict__ A, double *B, double *pcol, int *bad) {
-    gj_regs_nopiv_t<double, N, NR, 0, false, NT, TR, ROT>(A, B, nullptr, pcol, bad);
 }
 
 // Batched small GEMM with register tiles, spread over the NT threads of a CTA:
