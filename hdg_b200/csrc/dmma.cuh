@@ -44,8 +44,10 @@ __device__ __forceinline__ double fast_rcp(double x) {
 // Inverse of the 8 x 8 matrix held as a C fragment by a warp, in place: Gauss-Jordan over the four
 // diagonal 2 x 2 blocks in order (no pivoting).  One 2 x 2 block costs one shuffle round, one
 // reciprocal (of its determinant, the products with it formed meanwhile) and two multiply-adds in
-// sequence.  Returns false when a determinant is zero or not finite.
-__device__ __forceinline__ bool inv8(double (&z)[2]) {
+// sequence; between(b) is issued while block b's reciprocal is on its way.  Returns false when a
+// determinant is zero or not finite.
+template <class F>
+__device__ __forceinline__ bool inv8(double (&z)[2], F between) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, m = lane >> 2, h = lane & 3;
     bool ok = true;
@@ -60,6 +62,7 @@ __device__ __forceinline__ bool inv8(double (&z)[2]) {
         const double det = fma(a00, a11, -(a01 * a10));
         ok &= fabs(det) > 0.0 && isfinite(det);
         const double rd = fast_rcp(det);
+        between(b);
         // the block's rows become its inverse times them; row m loses (x0, x1) inverse times them
         const bool in0 = m == p, in1 = m == p + 1;
         const double u0 = in0 ? -a11 : (in1 ? a10 : fma(x0, a11, -(x1 * a10)));
@@ -97,8 +100,9 @@ struct TableOrder {
 // an A fragment of the columns 2 (l % 4) + s in step s, so no value is exchanged between lanes; the
 // right factors are the 8 columns of block k, which their owner has left in shared memory (inv(D)^T
 // and -L(i)^T; rows of ten doubles, so that the fragment reads are free of bank conflicts).  While
-// the others update, the owner of block k + 1 brings its tile up to date first and inverts the next
-// diagonal tile, so one barrier per 8 unknowns remains.
+// the others update, the owner of block k + 1 brings that block up to date and inverts the next diagonal
+// tile; its other columns wait until the next step (the published tiles go round three buffers), so
+// that an inversion and one barrier per 8 unknowns are all that is in sequence.
 // What bounds it: the chain of N / 8 inversions (about 1,300 cycles each), with the tensor work of
 // other resident elements beside it.  Measured in a loop, cycles per system against an elimination
 // of one unknown at a time in registers with a barrier each: N = 40, 49 right-hand sides, three
@@ -109,23 +113,8 @@ struct TableOrder {
 template <int N, int NR, int NT>
 struct BlockGJ {
     static constexpr int MT = (N + 7) / 8, RT = (NR + 7) / 8, CT = MT + RT, NW = NT / 32, CPT = (CT + NW - 1) / NW;
-    static constexpr int TS = 80, pub_doubles = 2 * MT * TS;
+    static constexpr int TS = 80, pub_doubles = 3 * MT * TS;
 };
-
-// The owner of column block k: the inverse of its diagonal tile and its other tiles, negated, into the
-// MT tiles at `to`.
-template <int k, int MT>
-__device__ __forceinline__ void publish_tiles(double (&z)[MT][2], double *to, int *bad) {
-    constexpr int TS = 80;
-    const int lane = threadIdx.x & 31, m = lane >> 2, n0 = 2 * (lane & 3);
-    to += 10 * m + n0;
-    const bool ok = inv8(z[k]);
-    if (!ok && lane == 0 && *bad == 0) *bad = 8 * k + 1;
-#pragma unroll
-    for (int i = 0; i < MT; i++)
-        *reinterpret_cast<double2 *>(to + i * TS) =
-            i == k ? make_double2(z[i][0], z[i][1]) : make_double2(-z[i][0], -z[i][1]);
-}
 
 // Block step k on one column block, with the tiles published at `from`
 template <int k, int MT>
@@ -146,17 +135,47 @@ __device__ __forceinline__ void apply_step(double (&z)[MT][2], const double *fro
         }
 }
 
+// The owner of column block k: block step k - 1 on its tiles, the diagonal one first, then the inverse
+// of the diagonal tile and the other tiles, negated, into the MT tiles at `to`.  The other tiles'
+// products are issued in the gaps of the inversion.
+template <int k, int MT>
+__device__ __forceinline__ void publish_tiles(double (&z)[MT][2], const double *from, double *to, int *bad) {
+    constexpr int TS = 80, k0 = k > 0 ? k - 1 : 0;
+    const int lane = threadIdx.x & 31;
+    to += 10 * (lane >> 2) + 2 * (lane & 3);
+    from += 20 * (lane & 3) + (lane >> 2);
+    double p[2] = {0.0, 0.0};
+    auto update = [&](int i) {
+        dmma(z[i], p[0], from[i * TS]);
+        dmma(z[i], p[1], from[i * TS + 10]);
+    };
+    if constexpr (k > 0) {
+        dmma(p, z[k0][0], from[k0 * TS]);
+        dmma(p, z[k0][1], from[k0 * TS + 10]);
+        z[k0][0] = p[0];
+        z[k0][1] = p[1];
+        update(k);
+    }
+    const bool ok = inv8(z[k], [&](int b) {
+        if constexpr (k > 0) {
+#pragma unroll
+            for (int i = 0; i < MT; i++)
+                if (i % 4 == b && i != k && i != k0) update(i);
+        }
+    });
+    if (!ok && lane == 0 && *bad == 0) *bad = 8 * k + 1;
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+        *reinterpret_cast<double2 *>(to + i * TS) =
+            i == k ? make_double2(z[i][0], z[i][1]) : make_double2(-z[i][0], -z[i][1]);
+}
+
 template <int N, int NR, int LDB, int NT, class Order>
 __device__ __forceinline__ void block_gj(const double *__restrict__ A, double *B, double *pub, int *bad, Order order) {
     using G = BlockGJ<N, NR, NT>;
     constexpr int MT = G::MT, CT = G::CT, NW = G::NW, CPT = G::CPT, TS = G::TS;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = lane >> 2, n0 = 2 * (lane & 3);
     double z[CPT][MT][2];
-    int at[MT][2];                                              // this lane's rows
-#pragma unroll
-    for (int i = 0; i < MT; i++)
-#pragma unroll
-        for (int t = 0; t < 2; t++) at[i][t] = 8 * i + n0 + t < N ? order(8 * i + n0 + t) : 0;
 #pragma unroll
     for (int s = 0; s < CPT; s++) {
         const int c = w + s * NW, col = 8 * c + m;
@@ -167,25 +186,26 @@ __device__ __forceinline__ void block_gj(const double *__restrict__ A, double *B
 #pragma unroll
             for (int t = 0; t < 2; t++) {
                 const int row = 8 * i + n0 + t;
-                z[s][i][t] = (in && row < N) ? src[at[i][t]] : (c < MT && col == row ? 1.0 : 0.0);
+                z[s][i][t] = (in && row < N) ? src[order(row)] : (c < MT && col == row ? 1.0 : 0.0);
             }
     }
     auto step = [&](auto kc) {
-        constexpr int k = decltype(kc)::value, kn = k + 1 < MT ? k + 1 : k, sn = kn / NW;   // the next block, its slot
-        const double *from = pub + (k & 1) * MT * TS;
-        const bool next = k + 1 < MT && w == kn % NW;
-        if (next) {
-            apply_step<k, MT>(z[sn], from);
-            publish_tiles<kn, MT>(z[sn], pub + (kn & 1) * MT * TS, bad);
-        }
+        constexpr int k = decltype(kc)::value, kn = k + 1 < MT ? k + 1 : k, kp = k > 0 ? k - 1 : 0;
+        const double *from = pub + k % 3 * MT * TS;
+        auto others = [&](auto jc, int except) {                // step j on the warp's live columns but one slot
+            constexpr int j = decltype(jc)::value;
 #pragma unroll
-        for (int s = 0; s < CPT; s++) {
-            const int c = w + s * NW;
-            if (c < CT && c > k && !(next && s == sn)) apply_step<k, MT>(z[s], from);
-        }
+            for (int s = 0; s < CPT; s++) {
+                const int c = w + s * NW;
+                if (c < CT && c > j && s != except) apply_step<j, MT>(z[s], pub + j % 3 * MT * TS);
+            }
+        };
+        if (k > 0 && w == k % NW) others(std::integral_constant<int, kp>{}, k / NW);   // what it put off as publisher
+        if (k + 1 < MT && w == kn % NW) publish_tiles<kn, MT>(z[kn / NW], from, pub + kn % 3 * MT * TS, bad);
+        else others(std::integral_constant<int, k>{}, -1);
         __syncthreads();
     };
-    if (w == 0) publish_tiles<0, MT>(z[0], pub, bad);
+    if (w == 0) publish_tiles<0, MT>(z[0], pub, pub, bad);
     __syncthreads();
     unroll_for<MT>(step);
 #pragma unroll
@@ -197,7 +217,7 @@ __device__ __forceinline__ void block_gj(const double *__restrict__ A, double *B
 #pragma unroll
                 for (int t = 0; t < 2; t++) {
                     const int row = 8 * i + n0 + t;
-                    if (row < N) B[at[i][t] + LDB * col] = z[s][i][t];
+                    if (row < N) B[order(row) + LDB * col] = z[s][i][t];
                 }
         }
     }
@@ -224,10 +244,9 @@ __device__ __forceinline__ void block_gj_factor(const double *A, double *steps, 
         }
     unroll_for<MT>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        double *step = steps + k * MT * TS;
-        if (w == k) publish_tiles<k, MT>(z, step, bad);
+        if (w == k) publish_tiles<k, MT>(z, steps + (k - 1) * MT * TS, steps + k * MT * TS, bad);
         __syncthreads();
-        if (w > k && w < MT) apply_step<k, MT>(z, step);
+        if (w > k + 1 && w < MT) apply_step<k, MT>(z, steps + k * MT * TS);
     });
 }
 

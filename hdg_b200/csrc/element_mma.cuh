@@ -114,62 +114,6 @@ __device__ __forceinline__ void face_product(const double *__restrict__ fg, LF l
     }
 }
 
-// Output tiles per job of matrix_product: the count (at most 6) that leaves the busiest warp the least
-// to do, a tile counted as one and the left fragment as one more.
-__host__ __device__ constexpr int tiles_per_job(int ct, int ot, int nw) {
-    int best = 1, cost = 1 << 30;
-    for (int t = 1; t <= 6 && t <= ot; t++) {
-        const int c = (ct * ((ot + t - 1) / t) + nw - 1) / nw * (t + 1);
-        if (c <= cost) { best = t; cost = c; }
-    }
-    return best;
-}
-
-// out(c, o) = init(c, o) + sum_{k < K} left(c, k) right(k, o) for c < NCOL, o < NOUT, in jobs of 8
-// columns by a few tiles of 8 outputs.  store(c, o, v0, v1, n) consumes the outputs o and (n == 2) o + 1;
-// init is read when the job begins.  first: the warp that takes job 0 (several products share the
-// warps evenly); returns the next one's.
-template <int NCOL, int NOUT, int K, int NT, class FI, class FL, class FR, class ST>
-__device__ __forceinline__ int matrix_product(int first, FI init, FL left, FR right, ST store) {
-    constexpr int CT = (NCOL + 7) / 8, OT = (NOUT + 7) / 8, NW = NT / 32, TO = tiles_per_job(CT, OT, NW),
-                  GO = (OT + TO - 1) / TO;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = lane >> 2, q = lane & 3;
-    for (int job = (w + NW - first) % NW; job < CT * GO; job += NW) {
-        const int c = 8 * (job % CT) + m, o0 = 8 * TO * (job / CT);
-        const bool in = NCOL % 8 == 0 || c < NCOL;
-        double acc[TO][2], ini[TO][2];
-#pragma unroll
-        for (int t = 0; t < TO; t++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int o = o0 + 8 * t + 2 * q + h;
-                ini[t][h] = in && (NOUT % (8 * TO) == 0 || o < NOUT) ? init(c, o) : 0.0;
-                acc[t][h] = 0.0;
-            }
-#pragma unroll 4
-        for (int s = 0; s < (K + 3) / 4; s++) {
-            const int k = 4 * s + q;
-            const bool ink = K % 4 == 0 || k < K;
-            const double l = in && ink ? left(c, k) : 0.0;
-#pragma unroll
-            for (int t = 0; t < TO; t++) {
-                const int o = o0 + 8 * t + m;
-                const double r = ink && (NOUT % (8 * TO) == 0 || o < NOUT) ? right(k, o) : 0.0;
-                dmma(acc[t], l, r);
-            }
-        }
-        if (in) {
-#pragma unroll
-            for (int t = 0; t < TO; t++) {
-                const int o = o0 + 8 * t + 2 * q;
-                if (NOUT % (8 * TO) == 0 || o < NOUT)
-                    store(c, o, acc[t][0] + ini[t][0], acc[t][1] + ini[t][1], NOUT % 2 == 0 || o + 1 < NOUT ? 2 : 1);
-            }
-        }
-    }
-    return (first + CT * GO) % NW;
-}
-
 // two values to consecutive addresses, as one 16-byte store where `wide` says that they are aligned to it
 __device__ __forceinline__ void store2(double *p, double v0, double v1, bool wide) {
     if (wide) {
@@ -177,6 +121,119 @@ __device__ __forceinline__ void store2(double *p, double v0, double v1, bool wid
     } else {
         p[0] = v0;
         p[1] = v1;
+    }
+}
+
+// The trace Jacobian, face by face: for columns c < NH and the unknowns o = (a, n) of face j
+//   AE(o, j, c) = sum_{k < K} left(c, k, j) right(k, o, j) + sum_{a', g} face(c, j, g, a') [a == a'] fg(n, g)
+// (the second sum is H - GK_q Mi E, whose left factor depends on the component).  A job is 8 columns and
+// a face; on(c, j) says whether the second sum has anything for column c.
+template <int NCU, int NPF, int NFE, int NGF, int NH, int K, int NT, class FL, class FR, class FF, class FO>
+__device__ __forceinline__ void trace_jacobian(const double *__restrict__ fg, double *ae, bool wide, FL left, FR right, FF face,
+                                               FO on) {
+    constexpr int KQ = NPF * NCU, OT = (KQ + 7) / 8, NJ = (NH + 7) / 8 * NFE, NW = NT / 32;
+    const int lane = threadIdx.x & 31, m = lane >> 2, q = lane & 3;
+    for (int job = threadIdx.x >> 5; job < NJ; job += NW) {
+        const int j = job % NFE, c = 8 * (job / NFE) + m;
+        const bool in = NH % 8 == 0 || c < NH;
+        double acc[OT][2];
+#pragma unroll
+        for (int t = 0; t < OT; t++) acc[t][0] = acc[t][1] = 0.0;
+#pragma unroll 4
+        for (int s = 0; s < (K + 3) / 4; s++) {
+            const int k = 4 * s + q;
+            const bool ink = K % 4 == 0 || k < K;
+            const double l = in && ink ? left(c, k, j) : 0.0;
+#pragma unroll
+            for (int t = 0; t < OT; t++) dmma(acc[t], l, ink && (KQ % 8 == 0 || 8 * t + m < KQ) ? right(k, 8 * t + m, j) : 0.0);
+        }
+        if (__any_sync(0xffffffffu, in && on(c, j))) {
+#pragma unroll
+            for (int s = 0; s < (NGF + 3) / 4; s++) {
+                const int g = 4 * s + q;
+                const bool ing = NGF % 4 == 0 || g < NGF;
+                double w[NCU] = {};
+                if (in && ing) face(c, j, g, w);
+#pragma unroll
+                for (int t = 0; t < OT; t++) {
+                    const int o = 8 * t + m, n = o / NCU, ao = o - NCU * n;
+                    const double p = ing && (KQ % 8 == 0 || o < KQ) ? fg[n + NPF * g] : 0.0;
+#pragma unroll
+                    for (int a = 0; a < NCU; a++) dmma(acc[t], w[a], a == ao ? p : 0.0);
+                }
+            }
+        }
+        if (in) {
+            double *to = ae + NH * c + KQ * j + 2 * q;
+#pragma unroll
+            for (int t = 0; t < OT; t++) {
+                if (KQ % 2 == 0) {
+                    if (KQ % 8 == 0 || 8 * t + 2 * q < KQ) store2(to + 8 * t, acc[t][0], acc[t][1], wide);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                        if (8 * t + 2 * q + h < KQ) to[8 * t + h] = acc[t][h];
+                }
+            }
+        }
+    }
+}
+
+// The q rows of DUDG_DUH: for column k = (b, f), component a, direction d, node r
+//   dd(r, a, d, k) = sum_s MiC(r, s, d) dlu(s, a, k) - (a == b) MiE(r, f, d)
+// R: dlu [LDR, NH], dd: row (r, a, d) of column k at dd[NQ k + r + NPV (a + NCU d)].  Rows of the
+// fragments are (a, k); the right factor Mi C stays in registers for every job, and so do a lane's
+// offsets in the output: with them computed per value, the index arithmetic took most of the time.
+template <int NPV, int ND, int NCU, int NDF, int NH, int LDR, int NQ, int NT>
+__device__ __forceinline__ void q_rows(const double *R, const double *MiC, const double *MiE, double *dd, bool wide) {
+    constexpr int KS = (NPV + 3) / 4, OT = (NPV * ND + 7) / 8, TO = OT <= 4 ? OT : 4, CT = (NCU * NH + 7) / 8, NW = NT / 32;
+    const int lane = threadIdx.x & 31, m = lane >> 2, q = lane & 3;
+    for (int o0 = 0; o0 < 8 * OT; o0 += 8 * TO) {
+        double right[TO][KS];
+        int to[TO][2], me[TO][2];                                // offsets in a column of dd, in MiE; -1: no output
+#pragma unroll
+        for (int t = 0; t < TO; t++) {
+            const int o = o0 + 8 * t + m, r = o % NPV, d = o / NPV;
+#pragma unroll
+            for (int s = 0; s < KS; s++)
+                right[t][s] = o < NPV * ND && 4 * s + q < NPV ? MiC[r + NPV * (4 * s + q + NPV * d)] : 0.0;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int oo = o0 + 8 * t + 2 * q + h, rr = oo % NPV, de = oo / NPV;
+                to[t][h] = oo < NPV * ND ? rr + NPV * NCU * de : -1;
+                me[t][h] = rr + NPV * NDF * de;
+            }
+        }
+        for (int job = threadIdx.x >> 5; job < CT; job += NW) {
+            const int ak = 8 * job + m;
+            const bool in = (NCU * NH) % 8 == 0 || ak < NCU * NH;
+            const int k = ak / NCU, a = ak - NCU * k, f = k / NCU;
+            double acc[TO][2], left[KS];
+#pragma unroll
+            for (int s = 0; s < KS; s++)
+                left[s] = in && (NPV % 4 == 0 || 4 * s + q < NPV) ? R[LDR * k + NPV * a + 4 * s + q] : 0.0;
+#pragma unroll
+            for (int t = 0; t < TO; t++)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    acc[t][h] = in && a == k - NCU * f && to[t][h] >= 0 ? -MiE[me[t][h] + NPV * f] : 0.0;
+#pragma unroll
+            for (int s = 0; s < KS; s++)
+#pragma unroll
+                for (int t = 0; t < TO; t++) dmma(acc[t], left[s], right[t][s]);
+            if (in) {
+                double *col = dd + (size_t)NQ * k + NPV * a;
+#pragma unroll
+                for (int t = 0; t < TO; t++) {
+                    if (NPV % 2 == 0) {
+                        if (to[t][0] >= 0) store2(col + to[t][0], acc[t][0], acc[t][1], wide);
+                    } else {
+                        if (to[t][0] >= 0) col[to[t][0]] = acc[t][0];
+                        if (to[t][1] >= 0) col[to[t][1]] = acc[t][1];
+                    }
+                }
+            }
+        }
     }
 }
 

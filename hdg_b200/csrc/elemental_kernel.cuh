@@ -340,13 +340,25 @@ constexpr int blocks_for(size_t bytes) {
 template <class D, bool VISC, bool MIXED>
 using PlanSel = std::conditional_t<MIXED, Plan<D, VISC, blocks_for(Plan<D, VISC, false>::bytes) <= blocks_for(Plan<D, VISC, true>::bytes)>,
                                    PlanMma<D, VISC>>;
-template <class D, bool VISC, bool MIXED>
-constexpr int min_blocks() { return blocks_for(PlanSel<D, VISC, MIXED>::bytes); }
-template <class D, bool VISC, bool MIXED>
-constexpr int cta_threads() {
-    return PlanSel<D, VISC, MIXED>::WS ? 512
-                                       : (min_blocks<D, VISC, MIXED>() == 4 ? 128
-                                                                            : (min_blocks<D, VISC, MIXED>() == 3 ? 192 : 256));
+// Threads per CTA and CTAs per SM of a launch.  WIDE: the launch has at most one element per slot of
+// this shape, so what counts is the time of one element (2D Euler p = 2, 512 elements: 23.9 us with 128
+// threads an element, LATENCY_NARROW with 64); otherwise the elements in flight count, and the small
+// plans of the FP64 form trade threads for them.
+struct LaunchShape {
+    int threads, blocks;
+};
+template <class D, bool VISC, bool MIXED, bool WIDE>
+constexpr LaunchShape launch_shape() {
+    using L = PlanSel<D, VISC, MIXED>;
+    if (L::WS) return {512, 1};
+    if (!MIXED && !WIDE) {
+        if (L::bytes <= 27 * 1024) return {64, 8};
+        if (L::bytes <= 36 * 1024) return {96, 6};
+        if (L::bytes <= 44 * 1024) return {96, 5};
+        if (L::bytes <= 56 * 1024) return {128, 4};
+    }
+    const int n = blocks_for(L::bytes);
+    return {n == 4 ? 128 : (n == 3 ? 192 : 256), n};
 }
 
 // MIXED: the local elimination of the Jacobian columns runs in FP32 (with the identity
@@ -357,8 +369,8 @@ constexpr int cta_threads() {
 // Tensor-core Schur product also in plans that run several CTAs per SM (see USE_TC below).
 constexpr bool kTcMultiCta = false;
 
-template <class D, bool VISC, bool MIXED, int NT, class Arg = ElemParams>
-__global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_kernel(const __grid_constant__ Arg A) {
+template <class D, bool VISC, bool MIXED, int NT, int BLOCKS, class Arg = ElemParams>
+__global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_constant__ Arg A) {
     constexpr bool SEG = !std::is_same<Arg, ElemParams>::value;
     const ElemParams &P = base_params(A);
     using L = PlanSel<D, VISC, MIXED>;
@@ -440,7 +452,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
     // kernel's occupancy to 1), while the smaller plans run three or four elements per SM and
     // are bound by the latency of their elimination chain: the tensor-core Schur product is used
     // where the plan runs one CTA per SM anyway (3D p = 2).
-    constexpr bool USE_TC = L::TC && (min_blocks<D, VISC, MIXED>() == 1 || kTcMultiCta);
+    constexpr bool USE_TC = L::TC && (BLOCKS == 1 || kTcMultiCta);
     uint64_t *s_mbar = reinterpret_cast<uint64_t *>(wk + L::d_mbar);
     uint32_t tmem = 0, tc_phases = 0;          // bit b: the phase parity mbarrier b waits for next
     if constexpr (USE_TC) {
@@ -476,6 +488,31 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
 
     int seg = 0;                                 // segmented launches: the segment of element eg
     const int ne_launch = launch_ne(A);
+    // an element's nodes, state, trace and q source (SH_q), one value per thread and slot
+    constexpr int NPRE = (NPV * ND + NQ + NH + NPV * NCU * ND + NT - 1) / NT;
+    [[maybe_unused]] double pre[NPRE] = {};
+    [[maybe_unused]] int pre_bf = 0, fetched = -1;
+    [[maybe_unused]] auto fetch = [&](int at) {
+        const ElemParams *F = &P;
+        int el = at;
+        if constexpr (SEG) {
+            int sg = seg;
+            while (at >= A.seg_start[sg + 1]) sg++;
+            F = &A.seg[sg];
+            el = at - A.seg_start[sg];
+        }
+        const double *__restrict__ sh = F->SH ? F->SH + (size_t)el * NQ + NPV * NCU : nullptr;
+#pragma unroll
+        for (int k = 0; k < NPRE; k++) {
+            int i = tid + k * NT;
+            if (i < NPV * ND) pre[k] = __ldg(F->dgnodes + (size_t)el * NPV * ND + i);
+            else if ((i -= NPV * ND) < NQ) pre[k] = __ldg(F->UDG + (size_t)el * NQ + i);
+            else if ((i -= NQ) < NH) pre[k] = __ldg(F->UH + (size_t)el * NH + i);
+            else if ((i -= NH) < NPV * NCU * ND) pre[k] = sh ? __ldg(sh + i) : 0.0;
+        }
+        if (tid < NFE) pre_bf = F->bf[(size_t)el * NFE + tid];
+        fetched = at;
+    };
     for (int eg = blockIdx.x; eg < ne_launch; eg += gridDim.x) {
         const ElemParams *Qp = &P;
         int e = eg;
@@ -489,7 +526,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                                      // the scratch: the element is then evaluated again, pivoted
     elem_start:
         // ================================================================ load
-        {
+        if constexpr (MIXED) {
             const double *g_dg = Q.dgnodes + (size_t)e * NPV * ND;
             const double *g_udg = Q.UDG + (size_t)e * NPV * NC;
             const double *g_uh = Q.UH + (size_t)e * NCU * NDF;
@@ -497,14 +534,22 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
             for (int i = tid; i < NPV * NC; i += NT) s_udg[i] = g_udg[i];
             for (int i = tid; i < NCU * NDF; i += NT) s_uh[i] = g_uh[i];
             if (tid < NFE) s_bf[tid] = Q.bf[(size_t)e * NFE + tid];
-            if (tid == 0) *s_bad = 0;
-            if constexpr (!MIXED) {
-                const double *__restrict__ g_sh = Q.SH + (size_t)e * NPV * NC;
-                const bool no_q = Q.QDG || Q.RU;                     // getq: q does not enter
-                for (int i = NPV * NCU + tid; i < NPV * NC; i += NT)
-                    wk[L::p_rqs + i - NPV * NCU] = (Q.SH ? g_sh[i] / Q.fc_q : 0.0) - (no_q ? 0.0 : g_udg[i]);
+        } else {
+            // the element's inputs were read while the one before it was written out (the first ones, and
+            // those of an element that is evaluated again, here)
+            if (fetched != eg) fetch(eg);
+            fetched = -1;
+#pragma unroll
+            for (int k = 0; k < NPRE; k++) {
+                int i = tid + k * NT;
+                if (i < NPV * ND) s_dg[i] = pre[k];
+                else if ((i -= NPV * ND) < NQ) s_udg[i] = pre[k];
+                else if ((i -= NQ) < NH) s_uh[i] = pre[k];
+                else if ((i -= NH) < NPV * NCU * ND) wk[L::p_rqs + i] = Q.fc_q == 1.0 ? pre[k] : pre[k] / Q.fc_q;
             }
+            if (tid < NFE) s_bf[tid] = pre_bf;
         }
+        if (tid == 0) *s_bad = 0;
         __syncthreads();
 
         // ====================================================== geometry, traces
@@ -630,6 +675,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
         }
         __syncthreads();
         // Rq = M (SH/fc_q - q) + C u - E uh   (volint.m:57-60, faceint.m:49-51)
+        [[maybe_unused]] const bool no_q = Q.QDG || Q.RU;       // getq: q does not enter
         const double *__restrict__ g_shq = Q.SH + (size_t)e * NPV * NC + NPV * NCU;   // q part of SH
         for (int i = tid; i < NPV * NCU * ND; i += NT) {
             const int r = i % NPV, a = (i / NPV) % NCU, d = i / (NPV * NCU);
@@ -638,7 +684,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
 #pragma unroll
             for (int s = 0; s < NPV; s++) {
                 double v;
-                if constexpr (!MIXED) v = wk[L::p_rqs + s + NPV * (a + NCU * d)];
+                if constexpr (!MIXED) v = wk[L::p_rqs + s + NPV * (a + NCU * d)] - (no_q ? 0.0 : s_udg[s + NPV * cq]);
                 else v = (Q.SH ? g_shq[s + NPV * (a + NCU * d)] / Q.fc_q : 0.0) -
                          ((Q.QDG || Q.RU) ? 0.0 : s_udg[s + NPV * cq]);   // getq: q does not enter
                 t += s_M[r + NPV * s] * v;
@@ -1412,16 +1458,20 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                 Xg[i] = t;
             }
             __syncthreads();
-            double *g_fe = Q.FE + (size_t)e * NH;
+            double *g_fe = Q.FE + (size_t)e * NH, *Y = Xg + NGT * NCG;
+            for (int i = tid; i < NGT * NCU; i += NT) {
+                const int gg = i % NGT, a = i / NGT;
+                double y = 0.0;
+#pragma unroll
+                for (int c = 0; c < NCG; c++) y += s_Gp[gg + NGT * a + L::CF * c] * Xg[gg + NGT * c];
+                Y[i] = y;
+            }
+            __syncthreads();
             for (int i = tid; i < NH; i += NT) {
                 const int a = i % NCU, nf = i / NCU, n = nf % NPF, j = nf / NPF;
                 double t = 0.0;
-                for (int g = 0; g < NGF; g++) {
-                    const int gg = g + NGF * j;
-                    double y = 0.0;
-                    for (int c = 0; c < NCG; c++) y += s_Gp[gg + NGT * a + L::CF * c] * Xg[gg + NGT * c];
-                    t += t_fg[n + NPF * g] * y;
-                }
+#pragma unroll
+                for (int g = 0; g < NGF; g++) t += t_fg[n + NPF * g] * Y[g + NGF * j + NGT * a];
                 g_fe[i] = s_Rh[i] - t;
             }
             __syncthreads();
@@ -1431,7 +1481,6 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
         // The FP64 form: with DUDG_DUH = [dlu, Mi C dlu - Mi E] on the q rows,
         //   AE = (H - GK_q Mi E) + G' dlu,   G' = GK_u + GK_q Mi C,
         // both factors summed face by face like the face terms of SD and of the right-hand sides.
-        // First H - GK_q Mi E goes to AE, G' to the scratch and DUDG_DUH out; then AE += G' dlu.
         auto mma_out = [&](auto nco_c) {
             constexpr int NCO = decltype(nco_c)::value;
             [[maybe_unused]] constexpr int KQ = NPF * NCU;
@@ -1443,25 +1492,8 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                 face_product<NCU, NPF, NFE, NGF, NU, NT>(
                     t_fg, [&](int c, int j, int g, double (&w)[NCU]) { left_face(s_Gp, c % NPV, c / NPV, g + NGF * j, w); },
                     [&](int c, int a, int n, int j, double v) { G[c * L::SG + a + NCU * (n + NPF * j)] = v; });
-                face_product<NCU, NPF, NFE, NGF, NH, NT>(
-                    t_fg,
-                    [&](int c, int j, int g, double (&w)[NCU]) {
-                        const int b = c % NCU, f = c / NCU, kf = g + NGF * j;
-                        if (f / NPF == j) {
-                            const double z = t_ft[g + NGF * (f % NPF)];
-#pragma unroll
-                            for (int a = 0; a < NCU; a++) w[a] = s_Hp[kf + NGT * (a + NCU * b)] * z;
-                        }
-#pragma unroll
-                        for (int d = 0; d < ND; d++) {
-                            const double z = x_ZFe[kf + L::ZF * (f + NDF * d)];
-#pragma unroll
-                            for (int a = 0; a < NCU; a++) w[a] -= s_Gp[kf + NGT * a + L::CF * (NCU + b + NCU * d)] * z;
-                        }
-                    },
-                    [&](int c, int a, int n, int j, double v) { g_ae[NH * c + a + NCU * (n + NPF * j)] = v; });
             } else {
-                // inviscid: both are zero between a face's unknowns and what is not on the face
+                // inviscid: zero but for the unknowns on the face
                 face_product<NCU, NPF, NFE, NGF, KQ, NT>(
                     t_fg,
                     [&](int c, int j, int g, double (&w)[NCU]) {
@@ -1470,59 +1502,35 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
                         for (int a = 0; a < NCU; a++) w[a] = s_Gp[g + NGF * j + NGT * a + L::CF * (c / NPF)] * z;
                     },
                     [&](int c, int a, int n, int j, double v) { G[(KQ * j + c) * L::SG + a + NCU * n] = v; });
-                face_product<NCU, NPF, NFE, NGF, KQ, NT>(
-                    t_fg,
-                    [&](int c, int j, int g, double (&w)[NCU]) {
-                        const double z = t_ft[g + NGF * (c / NCU)];
-#pragma unroll
-                        for (int a = 0; a < NCU; a++) w[a] = s_Hp[g + NGF * j + NGT * (a + NCU * (c % NCU))] * z;
-                    },
-                    [&](int c, int a, int n, int j, double v) { g_ae[NH * (c + KQ * j) + a + NCU * (n + NPF * j)] = v; });
             }
-            for (int i = tid; i < NU * NH; i += NT) {
-                const int ru = i % NU, k = i / NU;
-                g_dd[(size_t)NPV * NCO * k + ru] = s_R[L::LDR * (1 + k) + ru];
-            }
-            if constexpr (NCO == NC) {
-                // q rows (r, a, d) of column k: columns (a, k), outputs (r, d)
-                matrix_product<NCU * NH, NPV * ND, NPV, NT>(
-                    0,
-                    [&](int ak, int o) {
-                        const int k = ak / NCU, r = o % NPV, d = o / NPV;
-                        return ak % NCU == k % NCU ? -s_MiE[r + NPV * (k / NCU + NDF * d)] : 0.0;
-                    },
-                    [&](int ak, int sx) { return s_R[L::LDR * (1 + ak / NCU) + NPV * (ak % NCU) + sx]; },
-                    [&](int sx, int o) { return s_MiC[o % NPV + NPV * (sx + NPV * (o / NPV))]; },
-                    [&](int ak, int o, double v0, double v1, int n) {
-                        double *to = g_dd + (size_t)NQ * (ak / NCU) + NPV * (NCU + ak % NCU);
-                        auto at = [&](int x) { return x % NPV + NPV * NCU * (x / NPV); };
-                        if constexpr (NPV % 2 == 0) {
-                            store2(to + at(o), v0, v1, wide);
-                        } else {
-                            to[at(o)] = v0;
-                            if (n == 2) to[at(o + 1)] = v1;
-                        }
-                    });
-            }
+            for (int k = tid >> 5; k < NH; k += NT / 32)
+                for (int ru = tid & 31; ru < NU; ru += 32) g_dd[(size_t)NPV * NCO * k + ru] = s_R[L::LDR * (1 + k) + ru];
+            if constexpr (NCO == NC)
+                q_rows<NPV, ND, NCU, NDF, NH, L::LDR, NQ, NT>(s_R + L::LDR, s_MiC, s_MiE, g_dd + NPV * NCU, wide);
             __syncthreads();
-            if constexpr (VISC) {
-                matrix_product<NH, NH, NU, NT>(
-                    0, [&](int c, int o) { return g_ae[NH * c + o]; },
-                    [&](int c, int k) { return s_R[L::LDR * (1 + c) + k]; }, [&](int k, int o) { return G[k * L::SG + o]; },
-                    [&](int c, int o, double v0, double v1, int) { store2(g_ae + NH * c + o, v0, v1, wide); });
-            } else {
-                int first = 0;
-                for (int j = 0; j < NFE; j++)
-                    first = matrix_product<NH, KQ, KQ, NT>(
-                        first, [&](int c, int o) { return c / KQ == j ? g_ae[NH * c + KQ * j + o] : 0.0; },
-                        [&](int c, int k) { return s_R[L::LDR * (1 + c) + perm[k % NPF + NPF * j] + NPV * (k / NPF)]; },
-                        [&](int k, int o) { return G[(KQ * j + k) * L::SG + o]; },
-                        [&](int c, int o, double v0, double v1, int n) {
-                            double *to = g_ae + NH * c + KQ * j + o;
-                            if (n == 2) store2(to, v0, v1, wide && KQ % 2 == 0);
-                            else *to = v0;
-                        });
-            }
+            trace_jacobian<NCU, NPF, NFE, NGF, NH, (VISC ? NU : KQ), NT>(
+                t_fg, g_ae, wide,
+                [&](int c, int k, int j) {
+                    return s_R[L::LDR * (1 + c) + (VISC ? k : perm[k % NPF + NPF * j] + NPV * (k / NPF))];
+                },
+                [&](int k, int o, int j) { return VISC ? G[k * L::SG + KQ * j + o] : G[(KQ * j + k) * L::SG + o]; },
+                [&](int c, int j, int g, double (&w)[NCU]) {
+                    const int b = c % NCU, f = c / NCU, kf = g + NGF * j;
+                    if (f / NPF == j) {
+                        const double z = t_ft[g + NGF * (f % NPF)];
+#pragma unroll
+                        for (int a = 0; a < NCU; a++) w[a] = s_Hp[kf + NGT * (a + NCU * b)] * z;
+                    }
+                    if constexpr (VISC) {
+#pragma unroll
+                        for (int d = 0; d < ND; d++) {
+                            const double z = x_ZFe[kf + L::ZF * (f + NDF * d)];
+#pragma unroll
+                            for (int a = 0; a < NCU; a++) w[a] -= s_Gp[kf + NGT * a + L::CF * (NCU + b + NCU * d)] * z;
+                        }
+                    }
+                },
+                [&](int c, int j) { return VISC || c / KQ == j; });
         };
         // The mixed form, in column tiles.  Each column tile runs four batched small GEMMs with register tiles:
         //   X   = DUDG_DUH columns: u rows copied from the solve, q rows = MiC dlu - MiE
@@ -1601,6 +1609,7 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
             if (Q.nco == NC) tiles(std::integral_constant<int, NC>{});
             else tiles(std::integral_constant<int, NCU>{});
         } else {
+            if (eg + (int)gridDim.x < ne_launch) fetch(eg + gridDim.x);
             if (Q.nco == NC) mma_out(std::integral_constant<int, NC>{});
             else mma_out(std::integral_constant<int, NCU>{});
         }
@@ -1618,13 +1627,14 @@ __global__ void __launch_bounds__(NT, (min_blocks<D, VISC, MIXED>())) elemental_
 inline ElemParams &base_of(ElemParams &a) { return a; }
 inline ElemParams &base_of(SegTable &a) { return a.seg[0]; }
 
-template <class D, bool VISC, bool MIXED, class Arg>
-int launch_t(const Arg &p, int ne, cudaStream_t st, int grid_req) {
-    constexpr int NT = cta_threads<D, VISC, MIXED>();
+template <class D, bool VISC, bool MIXED, bool WIDE, class Arg>
+int launch_shaped(const Arg &p, int ne, cudaStream_t st, int grid_req) {
+    constexpr LaunchShape S = launch_shape<D, VISC, MIXED, WIDE>();
+    constexpr int NT = S.threads;
     using L = PlanSel<D, VISC, MIXED>;
     const size_t smem = L::smem_bytes;
     if (smem > 227 * 1024) return -3;
-    auto kern = elemental_kernel<D, VISC, MIXED, NT, Arg>;
+    auto kern = elemental_kernel<D, VISC, MIXED, NT, S.blocks, Arg>;
     cudaError_t err = allow_dynamic_smem((const void *)kern, smem);
     if (err != cudaSuccess) return -10;
     // resident CTAs per SM of this instantiation, once per device
@@ -1659,6 +1669,16 @@ int launch_t(const Arg &p, int ne, cudaStream_t st, int grid_req) {
         err = cudaGetLastError();
     }
     return err == cudaSuccess ? 0 : -12;
+}
+
+// One wave of the wide shape, or less: that shape; more elements: the other, where it differs.
+template <class D, bool VISC, bool MIXED, class Arg>
+int launch_t(const Arg &p, int ne, cudaStream_t st, int grid_req) {
+    constexpr LaunchShape W = launch_shape<D, VISC, MIXED, true>(), M = launch_shape<D, VISC, MIXED, false>();
+    if constexpr (W.threads != M.threads || W.blocks != M.blocks) {
+        if (ne > sm_count_of(current_device()) * W.blocks) return launch_shaped<D, VISC, MIXED, false, Arg>(p, ne, st, grid_req);
+    }
+    return launch_shaped<D, VISC, MIXED, true, Arg>(p, ne, st, grid_req);
 }
 
 // The compiled element shapes: (nd, npv, npf, ngv, ngf) of 2D p = 1..4 and 3D p = 1..3 at the
