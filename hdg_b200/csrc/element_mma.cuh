@@ -20,13 +20,17 @@ __host__ __device__ constexpr int pad4(int x) { return x + ((4 - x % 8) + 8) % 8
 // For every column c < NCOL of a local matrix and every component a, over rows r < NPV:
 //   out(a, r, c) = sum_{k < KV} left_v(c, k, a) right_v(r, k) + sum_{k < KF} left_f(c, k, a) right_f(r, k)
 // left_*(c, k, w) fills w[0 .. NCU) for all a; store(c, a, r, value) consumes.
+//
+// Here and below, lanes past the last column, row or point read the last one instead (what comes of it
+// is not stored, or its factor is set to zero): a branch around a read keeps the reads from being
+// issued together, which cost more than the products.
 template <int NCU, int NPV, int KV, int KF, int NCOL, int NT, class LV, class RV, class LF, class RF, class ST>
 __device__ __forceinline__ void column_product(LV left_v, RV right_v, LF left_f, RF right_f, ST store) {
     constexpr int TN = (NPV + 7) / 8, NW = NT / 32;
     const int lane = threadIdx.x & 31, m = lane >> 2, q = lane & 3;
     for (int ct = threadIdx.x >> 5; ct < (NCOL + 7) / 8; ct += NW) {
-        const int c = 8 * ct + m;
-        const bool in = c < NCOL;
+        const bool in = NCOL % 8 == 0 || 8 * ct + m < NCOL;
+        const int c = in ? 8 * ct + m : NCOL - 1;
         double acc[NCU][TN][2];
 #pragma unroll
         for (int a = 0; a < NCU; a++)
@@ -40,22 +44,34 @@ __device__ __forceinline__ void column_product(LV left_v, RV right_v, LF left_f,
         };
 #pragma unroll 2
         for (int s = 0; s < (KV + 3) / 4; s++) {
-            const int k = 4 * s + q;
+            const bool ink = KV % 4 == 0 || 4 * s + q < KV;
+            const int k = ink ? 4 * s + q : KV - 1;
             double w[NCU] = {}, p[TN];
-            const bool ink = KV % 4 == 0 || k < KV;
-            if (in && ink) left_v(c, k, w);
+            left_v(c, k, w);
 #pragma unroll
-            for (int t = 0; t < TN; t++) p[t] = ink && (NPV % 8 == 0 || 8 * t + m < NPV) ? right_v(8 * t + m, k) : 0.0;
+            for (int t = 0; t < TN; t++) p[t] = right_v(NPV % 8 == 0 || 8 * t + m < NPV ? 8 * t + m : NPV - 1, k);
+            if constexpr (KV % 4 != 0) {
+#pragma unroll
+                for (int a = 0; a < NCU; a++) w[a] = ink ? w[a] : 0.0;
+#pragma unroll
+                for (int t = 0; t < TN; t++) p[t] = ink ? p[t] : 0.0;
+            }
             accumulate(w, p);
         }
 #pragma unroll 2
         for (int s = 0; s < (KF + 3) / 4; s++) {
-            const int k = 4 * s + q;
+            const bool ink = KF % 4 == 0 || 4 * s + q < KF;
+            const int k = ink ? 4 * s + q : KF - 1;
             double w[NCU] = {}, p[TN];
-            const bool ink = KF % 4 == 0 || k < KF;
-            if (in && ink) left_f(c, k, w);
+            left_f(c, k, w);
 #pragma unroll
-            for (int t = 0; t < TN; t++) p[t] = ink && (NPV % 8 == 0 || 8 * t + m < NPV) ? right_f(8 * t + m, k) : 0.0;
+            for (int t = 0; t < TN; t++) p[t] = right_f(NPV % 8 == 0 || 8 * t + m < NPV ? 8 * t + m : NPV - 1, k);
+            if constexpr (KF % 4 != 0) {
+#pragma unroll
+                for (int a = 0; a < NCU; a++) w[a] = ink ? w[a] : 0.0;
+#pragma unroll
+                for (int t = 0; t < TN; t++) p[t] = ink ? p[t] : 0.0;
+            }
             accumulate(w, p);
         }
         if (in) {
@@ -80,8 +96,9 @@ __device__ __forceinline__ void face_product(const double *__restrict__ fg, LF l
     const int lane = threadIdx.x & 31, m = lane >> 2, q = lane & 3;
     constexpr int NJ = (NCOL + 7) / 8 * NFE;                 // a job is a face of a block of 8 columns
     for (int job = threadIdx.x >> 5; job < NJ; job += NW) {
-        const int j = job % NFE, c = 8 * (job / NFE) + m;
-        const bool in = c < NCOL;
+        const int j = job % NFE, c0 = 8 * (job / NFE) + m;
+        const bool in = NCOL % 8 == 0 || c0 < NCOL;
+        const int c = in ? c0 : NCOL - 1;
         double acc[NCU][TN][2];
 #pragma unroll
         for (int a = 0; a < NCU; a++)
@@ -89,13 +106,18 @@ __device__ __forceinline__ void face_product(const double *__restrict__ fg, LF l
             for (int t = 0; t < TN; t++) acc[a][t][0] = acc[a][t][1] = 0.0;
 #pragma unroll
         for (int s = 0; s < (NGF + 3) / 4; s++) {
-            const int g = 4 * s + q;
+            const bool ing = NGF % 4 == 0 || 4 * s + q < NGF;
+            const int g = ing ? 4 * s + q : NGF - 1;
             double w[NCU] = {};
-            const bool ing = NGF % 4 == 0 || g < NGF;
-            if (in && ing) left(c, j, g, w);
+            left(c, j, g, w);
+            if constexpr (NGF % 4 != 0) {
+#pragma unroll
+                for (int a = 0; a < NCU; a++) w[a] = ing ? w[a] : 0.0;
+            }
 #pragma unroll
             for (int t = 0; t < TN; t++) {
-                const double p = ing && (NPF % 8 == 0 || 8 * t + m < NPF) ? fg[8 * t + m + NPF * g] : 0.0;
+                double p = fg[(NPF % 8 == 0 || 8 * t + m < NPF ? 8 * t + m : NPF - 1) + NPF * g];
+                if constexpr (NGF % 4 != 0) p = ing ? p : 0.0;
 #pragma unroll
                 for (int a = 0; a < NCU; a++) dmma(acc[a][t], w[a], p);
             }
@@ -114,13 +136,18 @@ __device__ __forceinline__ void face_product(const double *__restrict__ fg, LF l
     }
 }
 
+// Stores of the outputs, which the element does not read again, past L1: it is left to the tables and to
+// spilled registers (3D p = 2, two CTAs in 225 KB of shared memory: 1,060 -> 900 us on 3,072 elements).
+__device__ __forceinline__ void store_out(double *p, double v) {
+    asm volatile("st.global.L1::no_allocate.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
 // two values to consecutive addresses, as one 16-byte store where `wide` says that they are aligned to it
 __device__ __forceinline__ void store2(double *p, double v0, double v1, bool wide) {
     if (wide) {
-        *reinterpret_cast<double2 *>(p) = make_double2(v0, v1);
+        asm volatile("st.global.L1::no_allocate.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v0), "d"(v1) : "memory");
     } else {
-        p[0] = v0;
-        p[1] = v1;
+        store_out(p, v0);
+        store_out(p + 1, v1);
     }
 }
 
@@ -134,30 +161,43 @@ __device__ __forceinline__ void trace_jacobian(const double *__restrict__ fg, do
     constexpr int KQ = NPF * NCU, OT = (KQ + 7) / 8, NJ = (NH + 7) / 8 * NFE, NW = NT / 32;
     const int lane = threadIdx.x & 31, m = lane >> 2, q = lane & 3;
     for (int job = threadIdx.x >> 5; job < NJ; job += NW) {
-        const int j = job % NFE, c = 8 * (job / NFE) + m;
-        const bool in = NH % 8 == 0 || c < NH;
+        const int j = job % NFE, c0 = 8 * (job / NFE) + m;
+        const bool in = NH % 8 == 0 || c0 < NH;
+        const int c = in ? c0 : NH - 1;
         double acc[OT][2];
 #pragma unroll
         for (int t = 0; t < OT; t++) acc[t][0] = acc[t][1] = 0.0;
 #pragma unroll 4
         for (int s = 0; s < (K + 3) / 4; s++) {
-            const int k = 4 * s + q;
-            const bool ink = K % 4 == 0 || k < K;
-            const double l = in && ink ? left(c, k, j) : 0.0;
+            const bool ink = K % 4 == 0 || 4 * s + q < K;
+            const int k = ink ? 4 * s + q : K - 1;
+            double l = left(c, k, j), r[OT];
 #pragma unroll
-            for (int t = 0; t < OT; t++) dmma(acc[t], l, ink && (KQ % 8 == 0 || 8 * t + m < KQ) ? right(k, 8 * t + m, j) : 0.0);
+            for (int t = 0; t < OT; t++) r[t] = right(k, KQ % 8 == 0 || 8 * t + m < KQ ? 8 * t + m : KQ - 1, j);
+            if constexpr (K % 4 != 0) {
+                l = ink ? l : 0.0;
+#pragma unroll
+                for (int t = 0; t < OT; t++) r[t] = ink ? r[t] : 0.0;
+            }
+#pragma unroll
+            for (int t = 0; t < OT; t++) dmma(acc[t], l, r[t]);
         }
         if (__any_sync(0xffffffffu, in && on(c, j))) {
 #pragma unroll
             for (int s = 0; s < (NGF + 3) / 4; s++) {
-                const int g = 4 * s + q;
-                const bool ing = NGF % 4 == 0 || g < NGF;
+                const bool ing = NGF % 4 == 0 || 4 * s + q < NGF;
+                const int g = ing ? 4 * s + q : NGF - 1;
                 double w[NCU] = {};
-                if (in && ing) face(c, j, g, w);
+                face(c, j, g, w);
+                if constexpr (NGF % 4 != 0) {
+#pragma unroll
+                    for (int a = 0; a < NCU; a++) w[a] = ing ? w[a] : 0.0;
+                }
 #pragma unroll
                 for (int t = 0; t < OT; t++) {
-                    const int o = 8 * t + m, n = o / NCU, ao = o - NCU * n;
-                    const double p = ing && (KQ % 8 == 0 || o < KQ) ? fg[n + NPF * g] : 0.0;
+                    const int o = KQ % 8 == 0 || 8 * t + m < KQ ? 8 * t + m : KQ - 1, n = o / NCU, ao = o - NCU * n;
+                    double p = fg[n + NPF * g];
+                    if constexpr (NGF % 4 != 0) p = ing ? p : 0.0;
 #pragma unroll
                     for (int a = 0; a < NCU; a++) dmma(acc[t], w[a], a == ao ? p : 0.0);
                 }
@@ -172,7 +212,7 @@ __device__ __forceinline__ void trace_jacobian(const double *__restrict__ fg, do
                 } else {
 #pragma unroll
                     for (int h = 0; h < 2; h++)
-                        if (8 * t + 2 * q + h < KQ) to[8 * t + h] = acc[t][h];
+                        if (8 * t + 2 * q + h < KQ) store_out(to + 8 * t + h, acc[t][h]);
                 }
             }
         }
@@ -201,22 +241,26 @@ __device__ __forceinline__ void q_rows(const double *R, const double *MiC, const
             for (int h = 0; h < 2; h++) {
                 const int oo = o0 + 8 * t + 2 * q + h, rr = oo % NPV, de = oo / NPV;
                 to[t][h] = oo < NPV * ND ? rr + NPV * NCU * de : -1;
-                me[t][h] = rr + NPV * NDF * de;
+                me[t][h] = oo < NPV * ND ? rr + NPV * NDF * de : 0;
             }
         }
         for (int job = threadIdx.x >> 5; job < CT; job += NW) {
             const int ak = 8 * job + m;
             const bool in = (NCU * NH) % 8 == 0 || ak < NCU * NH;
-            const int k = ak / NCU, a = ak - NCU * k, f = k / NCU;
+            const int k = in ? ak / NCU : 0, a = in ? ak - NCU * k : 0, f = k / NCU;
+            const bool same = in && a == k - NCU * f;
             double acc[TO][2], left[KS];
 #pragma unroll
             for (int s = 0; s < KS; s++)
-                left[s] = in && (NPV % 4 == 0 || 4 * s + q < NPV) ? R[LDR * k + NPV * a + 4 * s + q] : 0.0;
+                left[s] = R[LDR * k + NPV * a + (NPV % 4 == 0 || 4 * s + q < NPV ? 4 * s + q : NPV - 1)];
+            if constexpr (NPV % 4 != 0) left[KS - 1] = 4 * (KS - 1) + q < NPV ? left[KS - 1] : 0.0;
 #pragma unroll
             for (int t = 0; t < TO; t++)
 #pragma unroll
-                for (int h = 0; h < 2; h++)
-                    acc[t][h] = in && a == k - NCU * f && to[t][h] >= 0 ? -MiE[me[t][h] + NPV * f] : 0.0;
+                for (int h = 0; h < 2; h++) {
+                    const double v = MiE[me[t][h] + NPV * f];    // read without a branch: one took half the time
+                    acc[t][h] = same ? -v : 0.0;
+                }
 #pragma unroll
             for (int s = 0; s < KS; s++)
 #pragma unroll
@@ -228,8 +272,8 @@ __device__ __forceinline__ void q_rows(const double *R, const double *MiC, const
                     if (NPV % 2 == 0) {
                         if (to[t][0] >= 0) store2(col + to[t][0], acc[t][0], acc[t][1], wide);
                     } else {
-                        if (to[t][0] >= 0) col[to[t][0]] = acc[t][0];
-                        if (to[t][1] >= 0) col[to[t][1]] = acc[t][1];
+                        if (to[t][0] >= 0) store_out(col + to[t][0], acc[t][0]);
+                        if (to[t][1] >= 0) store_out(col + to[t][1], acc[t][1]);
                     }
                 }
             }

@@ -931,12 +931,14 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
         auto right_v = [&](int r, int kk) { return t_vg[r + NPV * (kk + NGV)]; };   // shapvg(r, g, id + 1), kk = g + NGV id
         auto right_f = [&](int r, int kf) {
             const int m = invp[r + NPV * (kf / NGF)];
-            return m >= 0 ? t_fg[m + NPF * (kf % NGF)] : 0.0;
+            const double v = t_fg[max(m, 0) + NPF * (kf % NGF)];
+            return m >= 0 ? v : 0.0;
         };
         // the face point's factor for local unknown (k, b), J = FHu (SD) or Gp (trace Jacobian)
         auto left_face = [&](const double *J, int k, int b, int kf, double (&w)[NCU]) {
             const int nk = invp[k + NPV * (kf / NGF)];
-            left_node(J + kf + L::CF * b, nk >= 0 ? t_ft[kf % NGF + NGF * nk] : 0.0, x_ZFc + kf + L::ZF * k, L::ZF * NPV, NGT,
+            const double v = t_ft[kf % NGF + NGF * max(nk, 0)];
+            left_node(J + kf + L::CF * b, nk >= 0 ? v : 0.0, x_ZFc + kf + L::ZF * k, L::ZF * NPV, NGT,
                       L::CF, w);
         };
         double *x_w0 = wk + L::p_dudg;
@@ -1023,11 +1025,9 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
                     right_v,
                     [&](int c, int kf, double (&w)[NCU]) {
                         const int b = c % NCU, f = c / NCU;
-                        if (f / NPF == kf / NGF) {
-                            const double z = t_ft[kf % NGF + NGF * (f % NPF)];
+                        const double ft = t_ft[kf % NGF + NGF * (f % NPF)], z0 = f / NPF == kf / NGF ? ft : 0.0;
 #pragma unroll
-                            for (int a = 0; a < NCU; a++) w[a] = -x_FHh[kf + NGT * (a + NCU * b)] * z;
-                        }
+                        for (int a = 0; a < NCU; a++) w[a] = -x_FHh[kf + NGT * (a + NCU * b)] * z0;
                         const double *J = x_FHu + kf + L::CF * (NCU + b), *Z = x_ZFe + kf + L::ZF * f;
 #pragma unroll
                         for (int d = 0; d < ND; d++) {
@@ -1504,7 +1504,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
                     [&](int c, int a, int n, int j, double v) { G[(KQ * j + c) * L::SG + a + NCU * n] = v; });
             }
             for (int k = tid >> 5; k < NH; k += NT / 32)
-                for (int ru = tid & 31; ru < NU; ru += 32) g_dd[(size_t)NPV * NCO * k + ru] = s_R[L::LDR * (1 + k) + ru];
+                for (int ru = tid & 31; ru < NU; ru += 32) store_out(g_dd + (size_t)NPV * NCO * k + ru, s_R[L::LDR * (1 + k) + ru]);
             if constexpr (NCO == NC)
                 q_rows<NPV, ND, NCU, NDF, NH, L::LDR, NQ, NT>(s_R + L::LDR, s_MiC, s_MiE, g_dd + NPV * NCU, wide);
             __syncthreads();
@@ -1516,11 +1516,9 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
                 [&](int k, int o, int j) { return VISC ? G[k * L::SG + KQ * j + o] : G[(KQ * j + k) * L::SG + o]; },
                 [&](int c, int j, int g, double (&w)[NCU]) {
                     const int b = c % NCU, f = c / NCU, kf = g + NGF * j;
-                    if (f / NPF == j) {
-                        const double z = t_ft[g + NGF * (f % NPF)];
+                    const double ft = t_ft[g + NGF * (f % NPF)], z0 = f / NPF == j ? ft : 0.0;
 #pragma unroll
-                        for (int a = 0; a < NCU; a++) w[a] = s_Hp[kf + NGT * (a + NCU * b)] * z;
-                    }
+                    for (int a = 0; a < NCU; a++) w[a] = s_Hp[kf + NGT * (a + NCU * b)] * z0;
                     if constexpr (VISC) {
 #pragma unroll
                         for (int d = 0; d < ND; d++) {
