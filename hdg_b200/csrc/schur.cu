@@ -6,20 +6,15 @@
 //   DUDG = [du, Mi Rq + Mi C du]; DUDG_DUH = [dlu, Mi C dlu - Mi E (x) I]
 //   FE = Rh - GK DUDG; AE = H + GK DUDG_DUH.
 // hdgx_schur_u replaces kernel/schur_u.c (:42-163; MATLAB twin schur_primal.m:13-49).
-// One CTA per element (grid-stride), runtime sizes, operands staged in shared memory; the
-// inputs are never modified (the reference MEX overwrites M, C, E, BD, F, Rq, Ru).
+// The (u,q) form of the elemental kernel's shapes runs schur_uq_mma_kernel (schur_mma.cuh); schur_kernel
+// here takes any other sizes and the u form: one CTA per element (grid-stride), runtime sizes, operands
+// staged in shared memory.  The inputs are never modified (the reference MEX overwrites M, C, E, BD, F,
+// Rq, Ru).
 #include <cuda_runtime.h>
 #include "hdgx_common.cuh"
+#include "schur_mma.cuh"
 
 namespace hdgx {
-
-struct SchurParams {
-    int nd, npv, ncu, nc, ndf, ne, qform;   // qform 1: (u,q) form, 0: u only
-    const double *M, *C, *E, *BD, *F, *GK, *H, *Rq, *Ru, *Rh;
-    double *DUDG, *DUDG_DUH, *AE, *FE;
-    int *status;
-    int tile;
-};
 
 struct SchurPlan {
     size_t M, Mi, SD, R, dudg, X, ints, bytes;
@@ -158,6 +153,16 @@ __global__ void __launch_bounds__(NT) schur_kernel(const __grid_constant__ Schur
     }
 }
 
+template <int ND, int NPV, int NCU, int NDF>
+static int launch_mma(const SchurParams &p, cudaStream_t st) {
+    using S = SchurShape<ND, NPV, NCU, NDF>;
+    auto kern = schur_uq_mma_kernel<ND, NPV, NCU, NDF>;
+    if (allow_dynamic_smem((const void *)kern, S::bytes) != cudaSuccess) return -10;
+    const int slots = sm_count_of(current_device()) * S::blocks;
+    kern<<<p.ne < slots ? p.ne : slots, S::threads, S::bytes, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -12;
+}
+
 int schur_launch(int qform, int nd, int npv, int ncu, int nc, int ndf, int ne, const double *M,
                  const double *C, const double *E, const double *BD, const double *F, const double *GK,
                  const double *H, const double *Rq, const double *Ru, const double *Rh, double *DUDG,
@@ -165,6 +170,16 @@ int schur_launch(int qform, int nd, int npv, int ncu, int nc, int ndf, int ne, c
     constexpr int NT = 256;
     SchurParams p{nd, npv, ncu, nc, ndf, ne, qform, M, C, E, BD, F, GK, H, Rq, Ru, Rh,
                   DUDG, DUDG_DUH, AE, FE, status, 1};
+    if (ne < 1) return 0;
+    if (qform && nc == ncu * (nd + 1)) {
+        auto is = [&](int d, int v, int u, int f) { return nd == d && npv == v && ncu == u && ndf == f; };
+        if (is(2, 3, 4, 6)) return launch_mma<2, 3, 4, 6>(p, st);
+        if (is(2, 6, 4, 9)) return launch_mma<2, 6, 4, 9>(p, st);
+        if (is(2, 10, 4, 12)) return launch_mma<2, 10, 4, 12>(p, st);
+        if (is(2, 15, 4, 15)) return launch_mma<2, 15, 4, 15>(p, st);
+        if (is(3, 4, 5, 12)) return launch_mma<3, 4, 5, 12>(p, st);
+        if (is(3, 10, 5, 24)) return launch_mma<3, 10, 5, 24>(p, st);
+    }
     int tile = ncu * ndf;
     SchurPlan L = SchurPlan::make(nd, npv, ncu, nc, ndf, tile);
     while (L.bytes > 200 * 1024 && tile > 1) {
