@@ -86,6 +86,7 @@ static void sweep_color(const hdgx_bsr *A, int dir, const int *rows, int nr, con
                                                                                   A->pos, Mg, in, out);
 }
 
+int factor_level(const hdgx_bsr *A, const int *rows, int nr, double *Mg, int *status, bool first, cudaStream_t st);
 int level_sweep_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, cudaStream_t st);
 int level_sweep_apply_f32(const hdgx_bsr *A, const float *Mg, const double *x, double *y, double *v, cudaStream_t st);
 
@@ -218,9 +219,14 @@ int hdgx_bilu0_factor(const hdgx_bsr *A, double *Mg, int *status, hdgx_stream_t 
     }
     if (allow_dynamic_smem((const void *)bilu0_color_kernel<NT>, smem) != cudaSuccess)
         return -10;
+    bool first = true;
     for (int c = 0; c < A->ncolors; c++) {
         const int r0 = A->color_ptr[c], nr = A->color_ptr[c + 1] - r0;
         if (nr <= 0) continue;
+        const int rc = factor_level(A, A->color_rows + r0, nr, Mg, status, first, st);
+        first = false;
+        if (rc < 0) return rc;
+        if (rc == 0) continue;
         unsigned grid = (unsigned)(nr < sm_count() * 8 ? nr : sm_count() * 8);
         bilu0_color_kernel<NT><<<grid, NT, smem, st>>>(A->bs, A->color_rows + r0, nr, A->rowpts, A->colind, A->pos, Mg,
                                                        status);

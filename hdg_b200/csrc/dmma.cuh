@@ -284,4 +284,38 @@ __device__ __forceinline__ void block_gj_apply(double *B, const double *steps, O
     __syncthreads();
 }
 
+// Largest |b - A x| / (max row sum |A| max |x| + max |b|) of one column over the CTA, b read through bval;
+// every thread returns whether it is at most tol (NaN is not).  red: 4 doubles a warp.
+template <int N, int NT, class FB>
+__device__ __forceinline__ bool backward_error_ok(const double *A, const double *x, FB bval, double tol, double *red) {
+    double v[4] = {};
+    for (int r = threadIdx.x; r < N; r += NT) {
+        const double b = bval(r);
+        double res = b, as = 0.0;
+        for (int c = 0; c < N; c++) {
+            const double a = A[r + N * c];
+            res -= a * x[c];
+            as += fabs(a);
+        }
+        if (!(res == res)) res = INFINITY;
+        v[0] = fmax(v[0], fabs(res));
+        v[1] = fmax(v[1], as);
+        v[2] = fmax(v[2], fabs(x[r]));
+        v[3] = fmax(v[3], fabs(b));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        for (int o = 16; o > 0; o >>= 1) v[k] = fmax(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+        if ((threadIdx.x & 31) == 0) red[4 * (threadIdx.x >> 5) + k] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        v[k] = 0.0;
+        for (int w = 0; w < NT / 32; w++) v[k] = fmax(v[k], red[4 * w + k]);
+    }
+    __syncthreads();
+    return v[0] <= tol * (v[1] * v[2] + v[3]) && isfinite(v[0]);
+}
+
 }  // namespace hdgx
