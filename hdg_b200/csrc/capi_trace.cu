@@ -136,23 +136,26 @@ int trace_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, doub
     return launched();
 }
 
-__global__ void mgs_coop_kernel(size_t, int, const double *, double *, double *, double *, unsigned *, int *);
+constexpr int kMgsThreads = 512;         // as in trace_system.cu
+constexpr int kMgsBlocks = 256;          // packets of a half
+template <int R>
+__global__ void mgs_coop_kernel(size_t, int, const double *, double *, unsigned long long *, unsigned, int *, GmresState, int);
 
-// The Arnoldi orthogonalisation of w against V(:, 0:nv) and its normalisation as one cooperative
-// launch (mgs_coop_kernel); false when the device cannot hold the grid at once (the caller then
-// issues the separate products).  part: 2 * 1024 doubles; bar: 2 unsigned (bar[0] == 0 on entry).
-static bool mgs_fused(size_t n, int nv, const double *V, double *w, double *hcol, double *part, unsigned *bar, int *err,
-                      cudaStream_t st) {
-    unsigned grid = grid_for(n, 256);
-    if (grid > 1024) grid = 1024;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)mgs_coop_kernel, 256, 0) != cudaSuccess ||
-        (long long)per_sm * sm_count() < (long long)grid) {
-        cudaGetLastError();
-        return false;
-    }
-    void *args[] = {&n, &nv, &V, &w, &hcol, &part, &bar, &err};
-    if (cudaLaunchCooperativeKernel((const void *)mgs_coop_kernel, dim3(grid), dim3(256), args, 0, st) != cudaSuccess) {
+// The Arnoldi orthogonalisation of w against V(:, 0:nv), its normalisation and the rotation of column
+// nv - 1 of H as one cooperative launch (mgs_coop_kernel); false when the device cannot hold the grid at
+// once (the caller then issues the separate products).  packets: 4 * kMgsBlocks words, zero before the first
+// call; tag: above every tag of earlier calls on them by more than nv.
+static bool mgs_fused(size_t n, int nv, const double *V, double *w, unsigned long long *packets, unsigned tag, int *err,
+                      GmresState gs, int m, cudaStream_t st) {
+    size_t grid = (n + kMgsThreads - 1) / kMgsThreads;
+    const size_t cap = sm_count() < kMgsBlocks ? sm_count() : kMgsBlocks;
+    if (grid > cap) grid = cap;
+    const size_t per = (n + grid * kMgsThreads - 1) / (grid * kMgsThreads);
+    const void *kern = per <= 1 ? (const void *)mgs_coop_kernel<1>
+                                : (per <= 4 ? (const void *)mgs_coop_kernel<4>
+                                            : (per <= 12 ? (const void *)mgs_coop_kernel<12> : (const void *)mgs_coop_kernel<0>));
+    void *args[] = {&n, &nv, &V, &w, &packets, &tag, &err, &gs, &m};
+    if (cudaLaunchCooperativeKernel(kern, dim3((unsigned)grid), dim3(kMgsThreads), args, 0, st) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -265,7 +268,7 @@ size_t hdgx_gmres_workspace_bytes(const hdgx_bsr *A, int restart) {
     if (!A || restart < 1) return 0;
     const size_t N = (size_t)A->bs * A->nf;
     const size_t m = (size_t)restart;
-    return sizeof(double) * (N * (m + 1) + 3 * N + (m + 1) * m + 4 * (m + 1) + 8 + 2048 + 2 + m) + 256;
+    return sizeof(double) * (N * (m + 1) + 3 * N + (m + 1) * m + 4 * (m + 1) + 8 + 1024 + 2 + m + 4 * kMgsBlocks) + 256;
 }
 
 }  // extern "C"
@@ -294,11 +297,14 @@ int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const
     gs.g = gs.sn + (m + 1);
     gs.y = gs.g + (m + 1);
     gs.scal = gs.y + (m + 1);
-    double *part = gs.scal + 8;                   // [2048] partial sums
-    unsigned *bar = reinterpret_cast<unsigned *>(part + 2048);   // grid barrier of the fused step
-    int *bar_err = reinterpret_cast<int *>(bar + 1) + 1;         // [0] count, [1] generation, err
-    gs.hist = part + 2048 + 2;                    // [m] residual norm after each step of a cycle
-    cudaMemsetAsync(bar, 0, 3 * sizeof(unsigned), st);
+    double *part = gs.scal + 8;                   // [1024] partial sums
+    int *mgs_flag = reinterpret_cast<int *>(part + 1024);        // error flag of the fused step
+    gs.hist = part + 1024 + 2;                    // [m] residual norm after each step of a cycle
+    // [4 kMgsBlocks] packets of the fused step, on a 16-byte boundary
+    unsigned long long *packets = reinterpret_cast<unsigned long long *>(((size_t)(gs.hist + m) + 15) & ~(size_t)15);
+    unsigned mgs_tag = 1;                         // tags run on over the whole solve
+    cudaMemsetAsync(mgs_flag, 0, sizeof(int), st);
+    cudaMemsetAsync(packets, 0, sizeof(unsigned long long) * 4 * kMgsBlocks, st);
     // host scalars on the stack (pageable copies are stream-ordered and, unlike freeing
     // pinned memory, never synchronise the other streams of the device)
     double h_scal[1 + kGmresBatch] = {};
@@ -344,15 +350,17 @@ int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const
                 if (int r = trace_matvec(A, Hg, vj, t, st)) rc = rc ? rc : r;
                 if (int r = prec(t, w2, w)) rc = rc ? rc : r;
                 double *hc = gs.H + (size_t)(m + 1) * j;
-                if (!mgs_fused(N, j + 1, V, w, hc, part, bar, bar_err, st)) {
+                const bool fused = mgs_fused(N, j + 1, V, w, packets, mgs_tag, mgs_flag, gs, m, st);
+                mgs_tag += (unsigned)j + 3;
+                if (!fused) {
                     for (int i = 0; i <= j; i++) {        // modified Gram-Schmidt (gmres_bilu0.m:59-63)
                         dot(N, V + N * i, w, hc + i, part, 0, st);
                         axpy_kernel<<<grid_for(N, 256), 256, 0, st>>>(N, hc + i, -1.0, V + N * i, w);
                     }
                     dot(N, w, w, hc + j + 1, part, 1, st);
                     scale_div_kernel<<<grid_for(N, 256), 256, 0, st>>>(N, hc + j + 1, w, w);
+                    givens_kernel<<<1, 1, 0, st>>>(gs, m, j);
                 }
-                givens_kernel<<<1, 1, 0, st>>>(gs, m, j);
             }
             wait(st);
             cudaMemcpyAsync(h_hist, gs.hist + j0, sizeof(double) * kb, cudaMemcpyDeviceToHost, st);
@@ -380,7 +388,7 @@ int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const
     if (flag) *flag = fl;
     if (relres) *relres = res_rel;
     int mgs_err = 0;
-    cudaMemcpyAsync(&mgs_err, bar_err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&mgs_err, mgs_flag, sizeof(int), cudaMemcpyDeviceToHost, st);
     synced();
     int sched_err = 0;
     if (A->ncolors == 0 && A->sched) {

@@ -11,8 +11,8 @@
 // with a barrier per unknown, and a launch.  Here a warp looks up all neighbours of all neighbours
 // at once; the row's own blocks, which no other row changes, are fetched while the level before
 // still runs (programmatic dependent launch), and neighbour s + 1's blocks while s's are used.
-// Factorisation: 2D p = 3, 12,416 faces, 440 levels: 11.4 -> TIME1 ms; 3D p = 2, 6,528 faces, 282
-// levels: 37.7 -> TIME2 ms.
+// Factorisation: 2D p = 3, 12,416 faces, 440 levels: 11.4 -> 2.83 ms; 3D p = 2, 6,528 faces, 282
+// levels: 37.7 -> 5.25 ms.
 #include <cuda_runtime.h>
 #include "dmma.cuh"
 #include "hdgx_common.cuh"

@@ -342,23 +342,27 @@ __global__ void axpby_kernel(size_t n, double a, const double *__restrict__ x, d
 // GMRES state on the device: H[(m+1) x m] column-major, cs, sn, g[m+1], scalars.
 
 // Apply the previous rotations to column j of H, form the new one, update g.  One thread.
-__global__ void givens_kernel(GmresState s, int m, int j) {
+// hin, cs, sn: the column and the rotations as read (they may be the arrays of s themselves).
+__device__ void givens_column(const GmresState &s, int m, int j, const double *hin, const double *cs, const double *sns) {
     double *h = s.H + (size_t)(m + 1) * j;
+    double a = hin[0];
     for (int i = 0; i < j; i++) {
-        const double a = h[i], b = h[i + 1];
-        h[i] = s.cs[i] * a + s.sn[i] * b;
-        h[i + 1] = -s.sn[i] * a + s.cs[i] * b;
+        const double b = hin[i + 1], c = cs[i], sn = sns[i];
+        h[i] = c * a + sn * b;
+        a = -sn * a + c * b;
     }
-    const double a = h[j], b = h[j + 1];
+    const double b = hin[j + 1];
     const double den = sqrt(a * a + b * b);
     const double c = (den != 0.0) ? a / den : 1.0, sn = (den != 0.0) ? b / den : 0.0;
     s.cs[j] = c; s.sn[j] = sn;
     h[j] = den; h[j + 1] = 0.0;
-    s.g[j + 1] = -sn * s.g[j];
-    s.g[j] = c * s.g[j];
-    s.scal[1] = fabs(s.g[j + 1]);
+    const double g = s.g[j];
+    s.g[j + 1] = -sn * g;
+    s.g[j] = c * g;
+    s.scal[1] = fabs(-sn * g);
     if (s.hist) s.hist[j] = s.scal[1];
 }
+__global__ void givens_kernel(GmresState s, int m, int j) { givens_column(s, m, j, s.H + (size_t)(m + 1) * j, s.cs, s.sn); }
 
 // Back substitution of the triangular Hessenberg system for y[0:k].  One thread.
 __global__ void hess_solve_kernel(GmresState s, int m, int k) {
@@ -433,81 +437,134 @@ __device__ __forceinline__ int poll_limit(const int *sched) {
 }
 
 // ------------------------------------------------------------- fused Gram-Schmidt step
-// Blocks of one cooperative launch meet here.  Thread 0 of each block arrives on a counter; the
-// last one resets it and advances the generation; the others poll the generation with a bounded
-// wait (after HDGX_SPIN_LIMIT polls the error flag is raised and the block goes on).
-__device__ __forceinline__ void grid_barrier(unsigned *bar, unsigned nblocks, int *err) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *gen = bar + 1;
-        const unsigned g = *gen;
-        __threadfence();
-        if (atomicAdd(bar, 1u) == nblocks - 1) {
-            bar[0] = 0;
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            int n = 0;
-            while (*gen == g) {
-                if (++n > HDGX_SPIN_LIMIT) { atomicExch(err, 1); break; }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
+// One Arnoldi orthogonalisation of GMRES (modified Gram-Schmidt, gmres_bilu0.m:59-63: for
+// i < nv, h_i = v_i . w, w -= h_i v_i; then h_nv = |w|, w /= h_nv) and the Givens rotation of its
+// column as ONE cooperative launch of at most one block per SM.  A product ends in an exchange of
+// one partial sum per block: every block leaves its sum in a packet (two 8-byte words, each half of
+// the value beside the step's tag, so that no fence or counter is needed) and adds up all blocks'
+// packets in block order, so every block has the same bits.  Packets alternate between two
+// halves: a block writes step s + 2 only after it has every packet of step s + 1, which the others
+// send after they have read step s.  Waits are bounded (HDGX_SPIN_LIMIT polls, then the error flag).
+// Bound by that exchange, about 0.9 us a product; w stays in registers (R values a thread, or R = 0:
+// in memory) and v_{i+1} is read while product i is exchanged.  198,656 unknowns, 10.5 products on
+// average: 82 us with a counter barrier over 776 blocks -> 44 us.
+constexpr int kMgsThreads = 512, kMgsMaxRestart = 64;
+
+__device__ __forceinline__ void packet_store(unsigned long long *p, double v, unsigned tag) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | (b & 0xffffffffull)), "l"(t | (b >> 32))
+                 : "memory");
 }
 
-// One Arnoldi orthogonalisation of GMRES (modified Gram-Schmidt, gmres_bilu0.m:59-63: for
-// i < nv, h_i = v_i . w, w -= h_i v_i; then h_nv = |w|, w /= h_nv) as ONE cooperative launch
-// instead of 3 (nv + 1) small ones.  The grid is that of the two-pass dot product it replaces,
-// each block forms its partial sums over the same grid-stride elements and every block adds the
-// partials in the order of dot_final_kernel (256 threads), so the results are the same bit for
-// bit; every element of w is read and written by the same thread throughout, so one grid
-// barrier per product suffices (partials alternate between two halves of part[2 * grid]).
-__global__ void __launch_bounds__(256) mgs_coop_kernel(size_t n, int nv, const double *__restrict__ V, double *w,
-                                                       double *hcol, double *part, unsigned *bar, int *err) {
-    __shared__ double red[32];
-    __shared__ double hval;
+template <int R>
+__global__ void __launch_bounds__(kMgsThreads)
+    mgs_coop_kernel(size_t n, int nv, const double *__restrict__ V, double *w, unsigned long long *packets, unsigned tag0,
+                    int *err, GmresState gs, int m) {
+    __shared__ double red[kMgsThreads / 32], sum[kMgsThreads / 32];
+    const int pollers = ((int)gridDim.x + 31) / 32;          // warps that wait for packets (at most 8)
+    constexpr int RR = R > 0 ? R : 1;
     const unsigned G = gridDim.x;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const size_t t0 = blockIdx.x * (size_t)kMgsThreads + tid, step = (size_t)G * kMgsThreads;
+    double *hcol = gs.H + (size_t)(m + 1) * (nv - 1);
+    double wr[RR], vr[RR], vn[RR];
+    if constexpr (R > 0) {
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            const size_t t = t0 + k * step;
+            wr[k] = t < n ? w[t] : 0.0;
+            vn[k] = t < n ? V[t] : 0.0;
+        }
+    }
     for (int i = 0; i <= nv; i++) {
-        const double *a = i < nv ? V + n * i : w;
-        double *pp = part + (size_t)(i & 1) * G;
+        const double *a = V + n * i;
         double s = 0.0;
-        for (size_t t = blockIdx.x * (size_t)blockDim.x + tid; t < n; t += (size_t)G * blockDim.x) s += a[t] * w[t];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((tid & 31) == 0) red[tid >> 5] = s;
-        __syncthreads();
-        if (tid < 32) {
-            s = (tid < (int)(blockDim.x >> 5)) ? red[tid] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (tid == 0) pp[blockIdx.x] = s;
+        if constexpr (R > 0) {
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                vr[k] = i < nv ? vn[k] : wr[k];
+                s += vr[k] * wr[k];
+            }
+            if (i + 1 < nv) {                                // the next vector, while this product is exchanged
+#pragma unroll
+                for (int k = 0; k < R; k++) {
+                    const size_t t = t0 + k * step;
+                    vn[k] = t < n ? a[n + t] : 0.0;
+                }
+            }
+        } else {
+            const double *u = i < nv ? a : w;
+            for (size_t t = t0; t < n; t += step) s += u[t] * w[t];
         }
-        grid_barrier(bar, G, err);
-        s = 0.0;
-        for (int t = tid; t < (int)G; t += blockDim.x) s += __ldcg(pp + t);
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((tid & 31) == 0) red[tid >> 5] = s;
+        if (lane == 0) red[wp] = s;
         __syncthreads();
-        if (tid == 0) {
+        if (wp < pollers) {                                  // a lane a packet; warp 0 sends this block's first
+            unsigned long long *pk = packets + (size_t)(i & 1) * 2 * G;
+            const unsigned tag = tag0 + (unsigned)i, b = 32 * wp + lane;
+            if (wp == 0) {
+                s = lane < kMgsThreads / 32 ? red[lane] : 0.0;
+                for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) packet_store(pk + 2 * blockIdx.x, s, tag);
+            }
             double r = 0.0;
-            for (int q = 0; q < (int)(blockDim.x >> 5); q++) r += red[q];
-            hval = (i < nv) ? r : sqrt(r);
-            if (blockIdx.x == 0) hcol[i] = hval;
+            if (b < G) {
+                unsigned long long lo, hi;
+                int c = 0;
+                do {
+                    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(pk + 2 * b) : "memory");
+                } while (((unsigned)(lo >> 32) != tag || (unsigned)(hi >> 32) != tag) && ++c < HDGX_SPIN_LIMIT);
+                if (c >= HDGX_SPIN_LIMIT) atomicExch(err, 1);
+                r = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
+            }
+            __syncwarp();
+            for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+            if (lane == 0) sum[wp] = r;
         }
         __syncthreads();
-        const double h = hval;
+        double h = 0.0;
+        for (int k = 0; k < pollers; k++) h += sum[k];
+        if (i == nv) h = sqrt(h);
+        if (blockIdx.x == 0 && tid == 0) hcol[i] = h;
         if (i < nv) {
-            const double al = -1.0 * h;
-            for (size_t t = blockIdx.x * (size_t)blockDim.x + tid; t < n; t += (size_t)G * blockDim.x) w[t] += al * a[t];
+            if constexpr (R > 0) {
+#pragma unroll
+                for (int k = 0; k < R; k++) wr[k] -= h * vr[k];
+            } else {
+                for (size_t t = t0; t < n; t += step) w[t] -= h * a[t];
+            }
         } else {
             const double sc = (h != 0.0) ? 1.0 / h : 0.0;
-            for (size_t t = blockIdx.x * (size_t)blockDim.x + tid; t < n; t += (size_t)G * blockDim.x) w[t] = w[t] * sc;
+            if constexpr (R > 0) {
+#pragma unroll
+                for (int k = 0; k < R; k++)
+                    if (t0 + k * step < n) w[t0 + k * step] = wr[k] * sc;
+            } else {
+                for (size_t t = t0; t < n; t += step) w[t] *= sc;
+            }
         }
-        __syncthreads();
+    }
+    if (blockIdx.x == 0 && wp == 0) {
+        // the rotation's operands side by side first: one after another from memory they take 0.3 us each
+        __shared__ double col[3][kMgsMaxRestart + 1];
+        if (nv <= kMgsMaxRestart) {
+            __syncwarp();
+            for (int k = lane; k <= nv; k += 32) {
+                col[0][k] = __ldcg(hcol + k);
+                col[1][k] = k < nv - 1 ? gs.cs[k] : 0.0;
+                col[2][k] = k < nv - 1 ? gs.sn[k] : 0.0;
+            }
+            __syncwarp();
+            if (lane == 0) givens_column(gs, m, nv - 1, col[0], col[1], col[2]);
+        } else if (lane == 0) {
+            givens_column(gs, m, nv - 1, hcol, gs.cs, gs.sn);
+        }
     }
 }
+template __global__ void mgs_coop_kernel<0>(size_t, int, const double *, double *, unsigned long long *, unsigned, int *, GmresState, int);
+template __global__ void mgs_coop_kernel<1>(size_t, int, const double *, double *, unsigned long long *, unsigned, int *, GmresState, int);
+template __global__ void mgs_coop_kernel<4>(size_t, int, const double *, double *, unsigned long long *, unsigned, int *, GmresState, int);
+template __global__ void mgs_coop_kernel<12>(size_t, int, const double *, double *, unsigned long long *, unsigned, int *, GmresState, int);
 
 __device__ __forceinline__ int load_acquire(const int *p) {
     int v;
@@ -741,24 +798,47 @@ __global__ void bilu0_bwd_bs_kernel(const int *__restrict__ rows, int nrows, con
     }
 }
 
+// y = Hg x, a warp per row: the row's neighbours and their values of x are read at once (lane b the block
+// index b, then lane r the values r, into shared memory), and PARTS = 32 / BS groups of lanes take every
+// PARTS-th block.  DRAM-bound; with one group of lanes and x read by every lane, 2D p = 3, 12,416 faces
+// (102 MB): 45.5 us; now 26.9 us.
 template <int BS>
-__global__ void bsr_matvec_bs_kernel(int nf, const long long *__restrict__ rowpts, const int *__restrict__ colind,
-                                     const double *__restrict__ Hg, const double *__restrict__ x,
-                                     double *__restrict__ y) {
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (int i = blockIdx.x * warps + (threadIdx.x >> 5); i < nf; i += gridDim.x * warps) {
-        for (int r = lane; r < BS; r += 32) {
-            double acc = 0.0;
-            for (long long k = rowpts[i]; k < rowpts[i + 1]; k++) {
-                const double *H = Hg + (size_t)BS * BS * k, *xj = x + (size_t)BS * (colind[k] - 1);
-                double hv[BS], xv[BS];
-#pragma unroll
-                for (int c = 0; c < BS; c++) { hv[c] = H[r + BS * c]; xv[c] = xj[c]; }
-#pragma unroll
-                for (int c = 0; c < BS; c++) acc += hv[c] * xv[c];
+__global__ void __launch_bounds__(256, BS >= 20 ? 2 : 4) bsr_matvec_bs_kernel(int nf, const long long *__restrict__ rowpts,
+                                                            const int *__restrict__ colind, const double *__restrict__ Hg,
+                                                            const double *__restrict__ x, double *__restrict__ y) {
+    constexpr int PARTS = 32 / BS, NB = 8, BSP = (BS + 1) / 2 * 2;
+    __shared__ double xs[8][NB][BSP];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int part = lane / BS, r = lane - part * BS;
+    for (int i = blockIdx.x * warps + w; i < nf; i += gridDim.x * warps) {
+        const long long k0 = rowpts[i], k1 = rowpts[i + 1];
+        double acc = 0.0;
+        for (long long kb = k0; kb < k1; kb += NB) {
+            const int nb = k1 - kb < NB ? (int)(k1 - kb) : NB;
+            const int col = lane < nb ? colind[kb + lane] - 1 : 0;
+            for (int b = part; b - part < nb; b += PARTS) {
+                const int cb = __shfl_sync(0xffffffffu, col, b < nb ? b : 0);
+                if (part < PARTS && b < nb) xs[w][b][r] = x[(size_t)BS * cb + r];
             }
-            y[(size_t)BS * i + r] = acc;
+            __syncwarp();
+            if (part < PARTS) {
+#pragma unroll 1
+                for (int b = part; b < nb; b += PARTS) {
+                    const double *H = Hg + (size_t)BS * BS * (kb + b) + r;
+                    double hv[BS], s[2] = {0.0, 0.0};
+#pragma unroll
+                    for (int c = 0; c < BS; c++) hv[c] = H[BS * c];
+#pragma unroll
+                    for (int c = 0; c < BS; c++) s[c & 1] += hv[c] * xs[w][b][c];
+                    acc += s[0] + s[1];
+                }
+            }
+            __syncwarp();
         }
+        double t = acc;
+#pragma unroll
+        for (int p = 1; p < PARTS; p++) t += __shfl_down_sync(0xffffffffu, acc, p * BS);
+        if (part == 0) y[(size_t)BS * i + r] = t;
     }
 }
 
