@@ -22,7 +22,9 @@
 //
 // What bounds a level is then the store-to-load time through L2 (0.47 us measured between two SMs)
 // and the arithmetic after it, so both are kept short: the row's factor blocks are staged in
-// shared memory before its inputs arrive, lane r of part p (PARTS = 32 / BS parts) adds up only
+// shared memory before its inputs arrive, by one bulk copy a block (16-byte copies by all lanes cost
+// a warp about 2,500 cycles a row of 30 x 30 blocks; blocks that are no multiple of 16 bytes, those of 15 x 15,
+// still take them: apply 600 -> 577 us at 12,416 faces of 16, 597 -> 567 us at 6,528 of 30), lane r of part p (PARTS = 32 / BS parts) adds up only
 // the neighbours p, p + PARTS, .. in CH independent chains (a dependent FP64 multiply-add takes
 // 17.6 cycles), and the parts are added with shuffles.
 #include <cuda_runtime.h>
@@ -54,12 +56,30 @@ __device__ __forceinline__ void store_value(double *p, double v) {
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void *dst, const void *src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+// One warp's mbarrier for its bulk copies
+__device__ __forceinline__ void stage_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void stage_bulk(void *dst, const void *src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ bool stage_wait(unsigned bar, unsigned parity, int limit) {
+    unsigned done = 0;
+    for (int n = 0; !done && n < limit; n++)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+    return done;
 }
 
 // Shared memory of one warp: MAXD neighbour blocks and the diagonal block of its row, the
-// neighbours' values and the row's intermediate t; as many warps per CTA as fit (at most 16).
+// neighbours' values, the row's intermediate t and the mbarrier; as many warps per CTA as fit (at most 16).
 template <int BS, int MAXD, class MT>
 struct SweepShape {
     static constexpr int PARTS = 32 / BS, DP = (MAXD + PARTS - 1) / PARTS;
@@ -68,10 +88,15 @@ struct SweepShape {
     static constexpr int CH = BS == 30 ? 6 : (BS == 15 ? 5 : 4);             // chains of a row sum
     static constexpr size_t stage = (sizeof(MT) * BLK * (MAXD + 1) + 15) / 16 * 16;
     static constexpr int BSP = (BS + 1) / 2 * 2;                             // 16-byte aligned value rows
-    static constexpr size_t warp_bytes = stage + sizeof(double) * BSP * (MAXD + 1);
+    static constexpr size_t warp_bytes = stage + sizeof(double) * BSP * (MAXD + 1) + 16;
     static constexpr int fit = (int)(216 * 1024 / warp_bytes);
     static constexpr int WPC = fit > 16 ? 16 : fit;
     static constexpr size_t smem = warp_bytes * WPC;
+    // Products of the neighbours that have arrived, while the last one is waited for: pays where a block's product
+    // is long.  Apply in us, all at once / as they arrive: blocks of 30, 6,528 faces in 282 levels, 702 / 597; of 20, 1,776
+    // in 160, 251 / 255; of 16, 12,416 in 440, 592 / 623; of 12, 800 in 104, 129 / 133.
+    static constexpr bool EARLY = BS > 20;
+    static_assert(!EARLY || PARTS == 1, "the slots of a warp are one row's");
     static_assert(BS <= 32 && RW <= 32 && WPC >= 1, "one lane per row component and per record entry");
 };
 
@@ -102,11 +127,18 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
     MT *blk = reinterpret_cast<MT *>(mine);                          // [MAXD + 1][BS, BS]
     double *val = reinterpret_cast<double *>(mine + S::stage);       // [MAXD][BSP], then t [BSP]
     double *tsh = val + MAXD * BSP;
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(tsh + BSP);
     const int part = lane / BS, r = lane - part * BS;
     const bool on = part < PARTS;
     const int W = gridDim.x * S::WPC, w = warp * gridDim.x + blockIdx.x;   // neighbouring slots on different SMs
-    const bool wide = sizeof(MT) * BLK % 16 == 0 && ((size_t)Mg & 15) == 0;
-    int limit = kPollLimit;
+    const bool wide = sizeof(MT) * BLK % 16 == 0 && ((size_t)Mg & 15) == 0;   // a bulk copy's addresses and sizes
+    int limit = kPollLimit, stage_limit = kPollLimit;
+    unsigned parity = 0;                                             // of the row staged next
+    if (lane == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
 
     // slot record, one entry per lane: (row, diagonal block, MAXD (block, column) of the earlier
     // neighbours, MAXD of the later ones)
@@ -114,12 +146,7 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
     auto stage_block = [&](int slot, int k) {
         const MT *src = Mg + (size_t)BLK * k;
         MT *dst = blk + slot * BLK;
-        if (wide) {
-            constexpr int PER = 16 / sizeof(MT);
-            for (int t = lane * PER; t < BLK; t += 32 * PER) cp_async<16>(dst + t, src + t);
-        } else {
-            for (int t = lane; t < BLK; t += 32) cp_async<sizeof(MT)>(dst + t, src + t);
-        }
+        for (int t = lane; t < BLK; t += 32) cp_async<sizeof(MT)>(dst + t, src + t);
     };
     auto add_parts = [&](double s) {
         double t = s;
@@ -137,8 +164,16 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
         int q = BWD ? nf - 1 - w : w;
         int cur = record(q), nxt = record(q + step), nxt2 = record(q + 2 * step);
         auto begin_row = [&](int R) {                                    // stage the row's blocks
-            const int i = __shfl_sync(0xffffffffu, R, 0);
-            if (i < 0) return;
+            if (__shfl_sync(0xffffffffu, R, 0) < 0) return;
+            if (wide) {                                                  // lane d: block d
+                const int k = __shfl_sync(0xffffffffu, R, lane < MAXD ? OFF + 2 * lane : 1);
+                const bool has = (lane < MAXD || (BWD && lane == MAXD)) && k >= 0;
+                const unsigned n = __popc(__ballot_sync(0xffffffffu, has));
+                if (lane == 0) stage_expect(bar, n * (unsigned)(sizeof(MT) * BLK));
+                __syncwarp();
+                if (has) stage_bulk(blk + lane * BLK, Mg + (size_t)BLK * k, sizeof(MT) * BLK, bar);
+                return;
+            }
 #pragma unroll
             for (int d = 0; d < MAXD; d++) {
                 const int k = __shfl_sync(0xffffffffu, R, OFF + 2 * d);
@@ -171,34 +206,54 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
             }
             prefetch_row(nxt2);
             const int nxt3 = record(q + 3 * step);
-            asm volatile("cp.async.wait_all;" ::: "memory");
+            bool staged = true;
+            if (wide) {
+                staged = stage_wait(bar, parity, stage_limit);
+                if (!staged) stage_limit = 1;
+                parity ^= 1;
+            } else {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+            }
             // wait for the neighbours' values (and, backward, for the row's own y)
             unsigned long long got[DP], own = 0;
-            bool ready;
-            int n = 0;
-            do {
-                ready = true;
+            double acc[CH] = {};
+            unsigned todo = 0;                                           // slots whose product is to be added
+#pragma unroll
+            for (int s = 0; s < DP; s++) todo |= k[s] >= 0 ? 1u << s : 0u;
+            auto use = [&](unsigned which) {
+#pragma unroll
+                for (int s = 0; s < DP; s++)
+                    if (which >> s & 1) val[(part + s * PARTS) * BSP + r] = __longlong_as_double((long long)got[s]);
+                __syncwarp();
 #pragma unroll
                 for (int s = 0; s < DP; s++) {
-                    got[s] = k[s] >= 0 ? load_value(in + (size_t)BS * j[s] + r) : 0ull;
-                    ready &= got[s] != kPending;
+                    const int d = part + s * PARTS;
+                    if (which >> s & 1) dot_cols<BS, BS, CH>(blk + d * BLK + r, val + d * BSP, 0, acc);
                 }
-                if (BWD) {
-                    own = part == 0 ? load_value(y + (size_t)BS * i + r) : 0ull;
-                    ready &= own != kPending;
+            };
+            for (int n = 0;;) {
+                unsigned miss = 0;
+#pragma unroll
+                for (int s = 0; s < DP; s++) got[s] = todo >> s & 1 ? load_value(in + (size_t)BS * j[s] + r) : 0ull;
+                if (BWD) own = part == 0 ? load_value(y + (size_t)BS * i + r) : 0ull;
+#pragma unroll
+                for (int s = 0; s < DP; s++) miss |= got[s] == kPending ? 1u << s : 0u;
+                if (BWD) miss |= own == kPending ? 1u << DP : 0u;
+                if (__all_sync(0xffffffffu, !miss)) break;
+                if (++n >= limit) {                                      // NaN (kPending is one) from here on
+                    limit = 1;
+                    break;
                 }
-            } while (!__all_sync(0xffffffffu, ready) && ++n < limit);
-            if (n >= limit) limit = 1;                                   // NaN (kPending is one) from here on
-#pragma unroll
-            for (int s = 0; s < DP; s++)
-                if (k[s] >= 0) val[(part + s * PARTS) * BSP + r] = __longlong_as_double((long long)got[s]);
-            __syncwarp();
-            double acc[CH] = {};
-#pragma unroll
-            for (int s = 0; s < DP; s++) {
-                const int d = part + s * PARTS;
-                if (k[s] >= 0) dot_cols<BS, BS, CH>(blk + d * BLK + r, val + d * BSP, 0, acc);
+                if constexpr (S::EARLY) {
+                    const unsigned here = __reduce_and_sync(0xffffffffu, ~miss) & todo;
+                    if (__any_sync(0xffffffffu, here != 0)) {
+                        use(here);
+                        todo &= ~here;
+                    }
+                }
             }
+            use(todo);
+            if (!staged) xv = __longlong_as_double((long long)(own = kPending));
             const double sum = add_parts(chain_sum(acc));
             if (!BWD) {
                 if (part == 0) store_value(out + (size_t)BS * i + r, xv - sum);
@@ -247,9 +302,11 @@ static int launch_sweep(const hdgx_bsr *A, const MT *Mg, const double *x, double
     const int nf = A->nf;
     const size_t n = (size_t)BS * nf;
     // four warps per row of an average level, so that a row's warp is there, its blocks staged, when
-    // the values arrive (2D p = 3, 12,416 faces in 440 levels: 1,322, 769, 611 and 641 us per apply
-    // with 1, 2, 4 and 8; 3D p = 2, 6,528 faces in 282 levels: 1,153, 900, 720 and 680)
-    const long long want = (4ll * nf / A->ncolors + S::WPC - 1) / S::WPC;
+    // the values arrive; six where a block takes long to stage.  Apply in us with 2, 3, 4 and 6 (clusters of
+    // at most 8 CTAs): 2D p = 3, 12,416 faces in 440 levels, 692, 577, 577, 559; 49,408 in 888, 1,507, 1,318, 1,237 to 1,333, 1,289;
+    // 3D p = 2, 6,528 faces in 282 levels, 705, 603, 567, 533.  More warps take SMs from other solves:
+    // 32 queued 2D requests on 16 slots ran at 34 to 43 solves/s with four, 16 to 29 with eight.
+    const long long want = ((S::EARLY ? 6ll : 4ll) * nf / A->ncolors + S::WPC - 1) / S::WPC;
     const int nsm = sm_count_of(current_device());
     int G = want < 1 ? 1 : (want > nsm ? nsm : (int)want);
     if (G <= 8) G = G > 4 ? 8 : (G > 2 ? 4 : G);

@@ -81,3 +81,53 @@ def test_not_a_number_in_is_not_a_number_out(oracle):
     v, w = ts.empty_vec(), ts.empty_vec()
     ts.bilu0_apply(dM, x, v, w)
     assert bool(torch.isnan(v.t).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,kw", [("c1", dict(n=5, porder=2)), ("c4", dict(n=3, porder=2))])
+def test_factors_at_8_byte_alignment(oracle, name, kw):
+    """Factors that no 16-byte copy can read: each value is staged by itself."""
+    import torch
+    from hdg_b200._lib import check, lib
+    P, ts, dM, DArray = _system(oracle, name, kw)
+    x = np.random.default_rng(5).standard_normal((ts.bs, ts.nf))
+    ref = oracle.bilu0_apply(P.mesh, dM.numpy(), x, ts.o2u, ts.u2o)
+    M = torch.empty(dM.t.numel() + 1, dtype=torch.float64, device="cuda")[1:]
+    M.copy_(dM.t.view(-1))
+    assert M.data_ptr() % 16 == 8
+    d, v, w = DArray.from_numpy(x), ts.empty_vec(), ts.empty_vec()
+    check(lib().hdgx_bilu0_apply(ct.byref(ts.bsr), M.data_ptr(), d.ptr, v.ptr, w.ptr, None), "hdgx_bilu0_apply")
+    torch.cuda.synchronize()
+    assert _rel(v.numpy(), ref) < 1e-12
+
+
+@pytest.mark.gpu
+def test_vectors_that_share_storage_in_part(oracle):
+    """The work vector over the right-hand side: one launch per level instead."""
+    P, ts, dM, DArray = _system(oracle, "c1", dict(n=5, porder=2))
+    x = np.random.default_rng(6).standard_normal((ts.bs, ts.nf))
+    ref = oracle.bilu0_apply(P.mesh, dM.numpy(), x, ts.o2u, ts.u2o)
+    d, v = DArray.from_numpy(x), ts.empty_vec()
+    ts.bilu0_apply(dM, d, v, d)
+    assert _rel(v.numpy(), ref) < 1e-12
+
+
+@pytest.mark.gpu
+def test_plan_that_is_no_schedule_ends_in_nan(oracle):
+    """A row that is said to need itself: its wait runs out, the result is NaN, and the next call is right."""
+    import torch
+    P, ts, dM, DArray = _system(oracle, "c1", dict(n=3, porder=2))
+    x = np.random.default_rng(7).standard_normal((ts.bs, ts.nf))
+    good, plan = ts.bsr.sweep_plan, ts.d["sweep_plan"].numpy().copy().ravel()
+    rec = plan[ts.bsr.ncolors + 1:].reshape(ts.nf, 2 + 4 * ts.bsr.sweep_maxd)
+    q = int(np.flatnonzero(rec[:, 2] >= 0)[0])
+    rec[q, 3] = rec[q, 0]
+    bad = DArray.from_numpy(plan, dtype=torch.int32)
+    v, w = ts.empty_vec(), ts.empty_vec()
+    ts.bsr.sweep_plan = bad.ptr
+    ts.bilu0_apply(dM, DArray.from_numpy(x), v, w)
+    torch.cuda.synchronize()
+    ts.bsr.sweep_plan = good
+    assert np.isnan(v.numpy()).any()
+    ts.bilu0_apply(dM, DArray.from_numpy(x), v, w)
+    assert _rel(v.numpy(), oracle.bilu0_apply(P.mesh, dM.numpy(), x, ts.o2u, ts.u2o)) < 1e-12
