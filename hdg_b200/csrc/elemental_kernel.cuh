@@ -341,9 +341,10 @@ template <class D, bool VISC, bool MIXED>
 using PlanSel = std::conditional_t<MIXED, Plan<D, VISC, blocks_for(Plan<D, VISC, false>::bytes) <= blocks_for(Plan<D, VISC, true>::bytes)>,
                                    PlanMma<D, VISC>>;
 // Threads per CTA and CTAs per SM of a launch.  WIDE: the launch has at most one element per slot of
-// this shape, so what counts is the time of one element (2D Euler p = 2, 512 elements: 23.9 us with 128
-// threads an element, LATENCY_NARROW with 64); otherwise the elements in flight count, and the small
-// plans of the FP64 form trade threads for them.
+// this shape, so what counts is the time of one element, and it gets all the threads that its share of the
+// SM allows; otherwise the elements in flight count, and the small plans of the FP64 form trade threads
+// for them (2D Euler p = 1, 13,122 elements: 316 us with four CTAs of 128, 187 with eight of 64; p = 2,
+// 8,192: 349 us with four of 128, 288 with the shape below).
 struct LaunchShape {
     int threads, blocks;
 };

@@ -18,15 +18,18 @@ from hdg_b200.mesh import mkmesh_cube, mkmesh_square
 
 SHAPES = [(nd, p, v) for nd, ps in ((2, (1, 2, 3, 4)), (3, (1, 2, 3))) for p in ps for v in (False, True)]
 
+# launches of more elements than one wave of the shape for few elements: the narrower CTAs of the small plans
+NARROW = [(2, 1, False), (2, 1, True), (2, 2, False), (2, 2, True), (2, 3, False), (3, 1, False), (3, 1, True)]
+
 
 class _Elements(Problem):
     def uh_elem(self, UH=None):
         return self.UH if UH is None else UH
 
 
-def _state(nd, p, visc, tdep=False):
+def _state(nd, p, visc, tdep=False, n=None):
     r = np.random.default_rng(100 * nd + 10 * p + visc)
-    mesh = mkmesh_square(4, 4, p) if nd == 2 else mkmesh_cube(2, 2, 2, p)
+    mesh = mkmesh_square(n or 4, n or 4, p) if nd == 2 else mkmesh_cube(n or 2, n or 2, n or 2, p)
     master = mkmaster(nd, p, 2 * p)
     app = make_app(nd, re=300.0 if visc else np.inf, minf=0.5)
     if tdep:
@@ -66,6 +69,14 @@ def test_every_shape_matches_oracle(oracle, nd, p, visc, getdqdg, tdep):
     from hdg_b200.elemental import hdg_elemental
     P = _state(nd, p, visc, tdep)
     P.app.getdqdg = getdqdg
+    _check(oracle, P, hdg_elemental(P.master, P.app, P.mesh.dgnodes, P.mesh.bf, P.UDG, P.UH, P.SH))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nd,p,visc", NARROW)
+def test_many_elements_match_oracle(oracle, nd, p, visc):
+    from hdg_b200.elemental import hdg_elemental
+    P = _state(nd, p, visc, n=25 if nd == 2 else 6)                      # 1,249 and 1,079 elements
     _check(oracle, P, hdg_elemental(P.master, P.app, P.mesh.dgnodes, P.mesh.bf, P.UDG, P.UH, P.SH))
 
 
