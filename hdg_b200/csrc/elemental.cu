@@ -15,6 +15,9 @@ HDGX_ELEM_LAUNCHERS_FP64(extern, hdgx::Tet3)
 namespace hdgx {
 
 template <class D>
+int residual_launch(const ElemParams &p, cudaStream_t st);   // residual.cu
+
+template <class D>
 static int launch_v(const ElemParams &p, bool visc, bool mixed, cudaStream_t st, int grid) {
     if constexpr (PlanSel<D, true, false>::WS || PlanSel<D, false, false>::WS) {
         // plans in the global workspace are built in FP64 only: the mixed form runs the FP64 kernel
@@ -104,6 +107,7 @@ int elemental_launch(const hdgx_master *m, const hdgx_app *app, int ne, const do
     const ElemParams p = fill_params(m, app, ne, dgnodes, bf, UDG, UH, SH, AE, FE, DUDG, DUDG_DUH, status, QDG, RU);
     if (int rc = elemental_check_master(m)) return rc;   // nothing is launched for a foreign master
     return with_dims(m->nd, m->porder, [&](auto d) -> int {
+        if (QDG || RU) return residual_launch<decltype(d)>(p, st);
         return launch_v<decltype(d)>(p, is_viscous(app), mixed, st, grid);
     });
 }

@@ -45,9 +45,9 @@ struct ElemParams {
     const int *bf;
     double *AE, *FE, *DUDG, *DUDG_DUH;
     int *status;
-    double *QDG;               // non-NULL: getq mode (kernel/getq.m), the element stops after inv(M)
+    double *QDG;               // getq (residual.cu): its result
     int nco;                   // components stored in DUDG / DUDG_DUH: nc, or ncu when app.getdqdg = 0
-    double *RU;                // non-NULL: residual mode (kernel/cuda_residual.m), Ru at q = getq(u, uh)
+    double *RU;                // the element residual (residual.cu): Ru at q = getq(u, uh)
     double *ws;                // global workspace of plans beyond shared memory (set by the launcher)
 };
 
@@ -362,6 +362,48 @@ constexpr LaunchShape launch_shape() {
     return {n == 4 ? 128 : (n == 3 ? 192 : 256), n};
 }
 
+// The adjugate of J, entry (i, j) at X[ld (i + ND j)]; returns det J (volgeom.m:18-61)
+template <int ND>
+__device__ __forceinline__ double adjugate(const double (&J)[ND][ND], double *X, int ld) {
+    double jac;
+    if constexpr (ND == 2) {
+        jac = J[0][0] * J[1][1] - J[0][1] * J[1][0];
+        X[ld * (0 + 2 * 0)] = J[1][1];
+        X[ld * (1 + 2 * 0)] = -J[1][0];
+        X[ld * (0 + 2 * 1)] = -J[0][1];
+        X[ld * (1 + 2 * 1)] = J[0][0];
+    } else {
+        jac = J[0][0] * J[1][1] * J[2][2] - J[0][0] * J[2][1] * J[1][2] + J[1][0] * J[2][1] * J[0][2]
+                 - J[1][0] * J[0][1] * J[2][2] + J[2][0] * J[0][1] * J[1][2] - J[2][0] * J[1][1] * J[0][2];
+        X[ld * (0 + 3 * 0)] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+        X[ld * (1 + 3 * 0)] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+        X[ld * (2 + 3 * 0)] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+        X[ld * (0 + 3 * 1)] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
+        X[ld * (1 + 3 * 1)] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
+        X[ld * (2 + 3 * 1)] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
+        X[ld * (0 + 3 * 2)] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
+        X[ld * (1 + 3 * 2)] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
+        X[ld * (2 + 3 * 2)] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
+    }
+    return jac;
+}
+
+// The normal v, with the area factor as its length, of a face point with the tangents dp(:, k); returns that
+// length (facegeom.m:20-52)
+template <int ND>
+__device__ __forceinline__ double face_normal(const double (&dp)[ND][ND > 1 ? ND - 1 : 1], double (&v)[ND]) {
+    if constexpr (ND == 2) {
+        v[0] = dp[1][0];
+        v[1] = -dp[0][0];
+        return sqrt(v[1] * v[1] + v[0] * v[0]);
+    } else {
+        v[0] = dp[1][0] * dp[2][1] - dp[2][0] * dp[1][1];
+        v[1] = dp[2][0] * dp[0][1] - dp[0][0] * dp[2][1];
+        v[2] = dp[0][0] * dp[1][1] - dp[1][0] * dp[0][1];
+        return sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+    }
+}
+
 // MIXED: the local elimination of the Jacobian columns runs in FP32 (with the identity
 // appended so that the FP32 inverse of SD comes out too); the local residual solve (DUDG)
 // is then refined against the FP64 SD to FP64 accuracy, and every residual (Ru, Rq, Rh, FE)
@@ -566,26 +608,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
                     for (int n = 0; n < NPV; n++) t += t_mv[g + NGV * (n + NPV * (k + 1))] * s_dg[n + NPV * m];
                     J[k][m] = t;
                 }
-            double *X = x_Xx + g;   // X(i,j) at X[NGV*(i + ND*j)]
-            if constexpr (ND == 2) {
-                x_jac[g] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
-                X[NGV * (0 + 2 * 0)] = J[1][1];
-                X[NGV * (1 + 2 * 0)] = -J[1][0];
-                X[NGV * (0 + 2 * 1)] = -J[0][1];
-                X[NGV * (1 + 2 * 1)] = J[0][0];
-            } else {
-                x_jac[g] = J[0][0] * J[1][1] * J[2][2] - J[0][0] * J[2][1] * J[1][2] + J[1][0] * J[2][1] * J[0][2]
-                         - J[1][0] * J[0][1] * J[2][2] + J[2][0] * J[0][1] * J[1][2] - J[2][0] * J[1][1] * J[0][2];
-                X[NGV * (0 + 3 * 0)] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
-                X[NGV * (1 + 3 * 0)] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
-                X[NGV * (2 + 3 * 0)] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-                X[NGV * (0 + 3 * 1)] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
-                X[NGV * (1 + 3 * 1)] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
-                X[NGV * (2 + 3 * 1)] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
-                X[NGV * (0 + 3 * 2)] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
-                X[NGV * (1 + 3 * 2)] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
-                X[NGV * (2 + 3 * 2)] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
-            }
+            x_jac[g] = adjugate<ND>(J, x_Xx + g, NGV);
         }
         for (int gg = tid; gg < NGT; gg += NT) {
             const int g = gg % NGF, j = gg / NGF;
@@ -600,21 +623,11 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
                         t += t_mf[g + NGF * (n + NPF * (k + 1))] * s_dg[perm[n + NPF * j] + NPV * m];
                     dp[m][k] = t;
                 }
-            if constexpr (ND == 2) {
-                const double jc = sqrt(dp[0][0] * dp[0][0] + dp[1][0] * dp[1][0]);
-                x_jf[gg] = jc;
-                x_nl[gg + NGT * 0] = dp[1][0] / jc;
-                x_nl[gg + NGT * 1] = -dp[0][0] / jc;
-            } else {
-                const double n0 = dp[1][0] * dp[2][1] - dp[2][0] * dp[1][1];
-                const double n1 = dp[2][0] * dp[0][1] - dp[0][0] * dp[2][1];
-                const double n2 = dp[0][0] * dp[1][1] - dp[1][0] * dp[0][1];
-                const double jc = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
-                x_jf[gg] = jc;
-                x_nl[gg + NGT * 0] = n0 / jc;
-                x_nl[gg + NGT * 1] = n1 / jc;
-                x_nl[gg + NGT * 2] = n2 / jc;
-            }
+            double v[ND];
+            const double jc = face_normal<ND>(dp, v);
+            x_jf[gg] = jc;
+#pragma unroll
+            for (int d = 0; d < ND; d++) x_nl[gg + NGT * d] = v[d] / jc;
         }
         // volint.m:31-33 / faceint.m:55-61: solution and trace at the Gauss points
         for (int i = tid; i < NGV * NC; i += NT) {
@@ -676,7 +689,6 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
         }
         __syncthreads();
         // Rq = M (SH/fc_q - q) + C u - E uh   (volint.m:57-60, faceint.m:49-51)
-        [[maybe_unused]] const bool no_q = Q.QDG || Q.RU;       // getq: q does not enter
         const double *__restrict__ g_shq = Q.SH + (size_t)e * NPV * NC + NPV * NCU;   // q part of SH
         for (int i = tid; i < NPV * NCU * ND; i += NT) {
             const int r = i % NPV, a = (i / NPV) % NCU, d = i / (NPV * NCU);
@@ -685,9 +697,8 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
 #pragma unroll
             for (int s = 0; s < NPV; s++) {
                 double v;
-                if constexpr (!MIXED) v = wk[L::p_rqs + s + NPV * (a + NCU * d)] - (no_q ? 0.0 : s_udg[s + NPV * cq]);
-                else v = (Q.SH ? g_shq[s + NPV * (a + NCU * d)] / Q.fc_q : 0.0) -
-                         ((Q.QDG || Q.RU) ? 0.0 : s_udg[s + NPV * cq]);   // getq: q does not enter
+                if constexpr (!MIXED) v = wk[L::p_rqs + s + NPV * (a + NCU * d)] - s_udg[s + NPV * cq];
+                else v = (Q.SH ? g_shq[s + NPV * (a + NCU * d)] / Q.fc_q : 0.0) - s_udg[s + NPV * cq];
                 t += s_M[r + NPV * s] * v;
             }
 #pragma unroll
@@ -705,44 +716,10 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
         block_gj<NPV, NPV * ND + NDF * ND + NCU * ND, NPV, NT>(s_M, s_MiC, pub, s_bad, NaturalOrder{});
         if (tid == 0 && *s_bad) *s_bad = 1;
         __syncthreads();
-        if (Q.QDG) {
-            // getq.m:37-104: the q that zeroes Rq for this u and uh; with q left out of Rq above,
-            // Mi Rq = inv(fc_q Mu) (fc_q Mu SH_q / fc_q + C u - E uh)
-            double *g_q = Q.QDG + (size_t)e * NPV * NCU * ND;
-            for (int i = tid; i < NPV * NCU * ND; i += NT) g_q[i] = s_MiRq[i];
-            if (tid == 0 && Q.status) Q.status[e] = *s_bad;
-            __syncthreads();
-            continue;
-        }
-        if (Q.RU) {
-            // cuda_residual.m:3-4: q from getq, then the u residual is evaluated at that q; Rq is
-            // zero at that q, so Mi Rq (and its Gauss-point values below) are set to exact zeros
-            for (int i = tid; i < NPV * NCU * ND; i += NT) {
-                s_udg[NPV * NCU + i] = s_MiRq[i];
-                s_MiRq[i] = 0.0;
-            }
-            __syncthreads();
-            for (int i = tid; i < NGV * NCU * ND; i += NT) {
-                const int g = i % NGV, c = NCU + i / NGV;
-                double t = 0.0;
-#pragma unroll
-                for (int n = 0; n < NPV; n++) t += t_vt[g + NGV * n] * s_udg[n + NPV * c];
-                x_ug[g + NGV * c] = t;
-            }
-            for (int i = tid; i < NGT * NCU * ND; i += NT) {
-                const int gg = i % NGT, c = NCU + i / NGT, g = gg % NGF, j = gg / NGF;
-                double t = 0.0;
-#pragma unroll
-                for (int n = 0; n < NPF; n++) t += t_ft[g + NGF * n] * s_udg[perm[n + NPF * j] + NPV * c];
-                x_fu[gg + NGT * c] = t;
-            }
-            __syncthreads();
-        }
 
         // ================================ flux / fhat / fbou at the Gauss points
         // volume: thread (g, seed); volint.m:81, 241-254
-        const int nseed = !MIXED && Q.RU ? 1 : NSEED;      // the residual alone needs no derivatives
-        for (int i = tid; i < NGV * nseed; i += NT) {
+        for (int i = tid; i < NGV * NSEED; i += NT) {
             const int g = i % NGV, sd = i / NGV;
             D1 u[NCU], q[NCU * ND], f[NCU * ND];
 #pragma unroll
@@ -769,7 +746,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
             for (int i = tid; i < NGV * ND * NCU * (NC - NCU); i += NT) x_wrl[NGV * ND * NCU * NCU + i] = 0.0;
         }
         // faces: thread (gg, seed); fhat.m:49-67 = f(uh,q).n + tau (u - uh)
-        for (int i = tid; i < NGT * nseed; i += NT) {
+        for (int i = tid; i < NGT * NSEED; i += NT) {
             const int gg = i % NGT, sd = i / NGT;
             D1 u[NCU], q[NCU * ND], f[NCU * ND];
 #pragma unroll
@@ -857,7 +834,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
             }
         }
         // Mi C, Mi E, Mi Rq at the volume and face Gauss points (only B couples through them)
-        if (VISC && (MIXED || !Q.RU)) {
+        if constexpr (VISC) {
             for (int i = tid; i < NGV * NPV * ND; i += NT) {
                 const int g = i % NGV, kd = i / NGV;
                 double t = 0.0;
@@ -998,7 +975,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
             for (int i = tid; i < (KV + NGT) * NCU; i += NT) {
                 const int kk = i % (KV + NGT), a = i / (KV + NGT), kf = kk - KV;
                 double w = kk < KV ? x_wrk[kk + KV * a] : -x_FH[kf + NGT * a];
-                if (VISC && !Q.RU) {
+                if constexpr (VISC) {
                     const double *J = kk < KV ? x_wrl + kk + NGV * ND * a + L::CW * NCU : x_FHu + kf + NGT * a + L::CF * NCU;
                     const double *Zr = kk < KV ? x_Zr + kk % NGV : x_ZFr + kf;
                     const int js = kk < KV ? L::CW : L::CF, zs = kk < KV ? NGV : NGT;
@@ -1009,7 +986,6 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
                 }
                 x_w0[i] = w;
             }
-            if (Q.RU) return;
             // RHS((r,a), (b,f)) = B Mi E - F   (schur_primal.m:98,118; faceint.m:319-333)
             if constexpr (VISC) {
                 column_product<NCU, NPV, KV, NGT, NH, NT>(
@@ -1172,18 +1148,6 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
         };
         if constexpr (MIXED) build_rhs();
         else mma_rhs();
-        if (Q.RU) {
-            // cuda_residual.m: the element u residual Ru (volume and face terms, time source)
-            __syncthreads();
-            if constexpr (!MIXED) {
-                mma_residual();
-                __syncthreads();
-            }
-            for (int i = tid; i < NU; i += NT) Q.RU[(size_t)e * NU + i] = s_R[i];
-            if (tid == 0 && Q.status) Q.status[e] = *s_bad;
-            __syncthreads();
-            continue;
-        }
         // Rh = -(fbou or fhat) integrated on each face (faceint.m:335-339)
         for (int i = tid; i < NH; i += NT) {
             const int a = i % NCU, mf = i / NCU, m = mf % NPF, j = mf / NPF;

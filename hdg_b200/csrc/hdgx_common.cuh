@@ -88,31 +88,40 @@ __device__ __forceinline__ D1 operator/(D1 a, D1 b) {
     double q = a.v * ib;
     return {q, (a.d - q * b.d) * ib};
 }
+// a value alone, by the same operations
+struct D0 {
+    double v;
+};
+__device__ __forceinline__ D0 operator+(D0 a, D0 b) { return {a.v + b.v}; }
+__device__ __forceinline__ D0 operator-(D0 a, D0 b) { return {a.v - b.v}; }
+__device__ __forceinline__ D0 operator*(D0 a, D0 b) { return {a.v * b.v}; }
+__device__ __forceinline__ D0 operator*(D0 a, double s) { return {a.v * s}; }
+__device__ __forceinline__ D0 operator/(D0 a, D0 b) { return {a.v * (1.0 / b.v)}; }
 
 // Compressible Navier-Stokes flux in all ND directions at one point (Euler when rinv = 0).
 // u[NCU] conserved state, q[NCU*ND] gradient slots (component fastest, the reference's
 // sign convention q = -grad u is carried through unchanged).  f[a + NCU*j].
 // Physics: application/FM/ns/flux2d.m / flux3d.m (flux_ns2d.c / flux_ns3d.c).
-template <int ND>
-__device__ __forceinline__ void ns_flux(const PhysConst &pc, const D1 *u, const D1 *q, D1 *f) {
+template <int ND, class S>
+__device__ __forceinline__ void ns_flux(const PhysConst &pc, const S *u, const S *q, S *f) {
     constexpr int NCU = ND + 2;
-    const D1 r = u[0], rE = u[NCU - 1];
-    D1 vel[ND];
-    D1 ke = dc(0.0);
+    const S r = u[0], rE = u[NCU - 1];
+    S vel[ND];
+    S ke = S{0.0};
 #pragma unroll
     for (int i = 0; i < ND; i++) {
         vel[i] = u[1 + i] / r;
         ke = ke + vel[i] * u[1 + i];
     }
-    const D1 p = (rE - ke * 0.5) * pc.gam1;
-    const D1 h = (rE + p) / r;
+    const S p = (rE - ke * 0.5) * pc.gam1;
+    const S h = (rE + p) / r;
     if (pc.rinv == 0.0) {
 #pragma unroll
         for (int j = 0; j < ND; j++) {
             f[0 + NCU * j] = u[1 + j];
 #pragma unroll
             for (int i = 0; i < ND; i++) {
-                D1 t = u[1 + i] * vel[j];
+                S t = u[1 + i] * vel[j];
                 if (i == j) t = t + p;
                 f[(1 + i) + NCU * j] = t;
             }
@@ -120,38 +129,38 @@ __device__ __forceinline__ void ns_flux(const PhysConst &pc, const D1 *u, const 
         }
         return;
     }
-    const D1 ri = dc(1.0) / r;
-    D1 gv[ND][ND];
+    const S ri = S{1.0} / r;
+    S gv[ND][ND];
 #pragma unroll
     for (int i = 0; i < ND; i++)
 #pragma unroll
         for (int j = 0; j < ND; j++) gv[i][j] = (q[(1 + i) + NCU * j] - vel[i] * q[NCU * j]) * ri;
-    D1 div = dc(0.0);
+    S div = S{0.0};
 #pragma unroll
     for (int i = 0; i < ND; i++) div = div + gv[i][i];
-    D1 v2 = dc(0.0);
+    S v2 = S{0.0};
 #pragma unroll
     for (int i = 0; i < ND; i++) v2 = v2 + vel[i] * vel[i];
 #pragma unroll
     for (int j = 0; j < ND; j++) {
-        D1 tauj[ND];
+        S tauj[ND];
 #pragma unroll
         for (int i = 0; i < ND; i++) {
-            D1 t = gv[i][j] + gv[j][i];
+            S t = gv[i][j] + gv[j][i];
             if (i == j) t = t - div * (2.0 / 3.0);
             tauj[i] = t * pc.rinv;
         }
-        D1 vdv = dc(0.0);
+        S vdv = S{0.0};
 #pragma unroll
         for (int i = 0; i < ND; i++) vdv = vdv + vel[i] * gv[i][j];
-        const D1 qr = q[NCU * j];
-        const D1 pj = (q[(NCU - 1) + NCU * j] - v2 * 0.5 * qr - r * vdv) * pc.gam1;
-        const D1 Tj = (pj * r - p * qr) / (r * r);
+        const S qr = q[NCU * j];
+        const S pj = (q[(NCU - 1) + NCU * j] - v2 * 0.5 * qr - r * vdv) * pc.gam1;
+        const S Tj = (pj * r - p * qr) / (r * r);
         f[0 + NCU * j] = u[1 + j];
-        D1 e = h * u[1 + j];
+        S e = h * u[1 + j];
 #pragma unroll
         for (int i = 0; i < ND; i++) {
-            D1 t = u[1 + i] * vel[j] + tauj[i];
+            S t = u[1 + i] * vel[j] + tauj[i];
             if (i == j) t = t + p;
             f[(1 + i) + NCU * j] = t;
             e = e + vel[i] * tauj[i];
@@ -218,6 +227,11 @@ __device__ __forceinline__ void roe_apply(double gam, double eps, const double *
 #pragma unroll
     for (int i = 0; i < ND; i++) y[1 + i] = l[2] * x[1 + i] + v[i] * w1 + dscale(w2, nl[i]);
     y[NCU - 1] = l[2] * x[NCU - 1] + h * w1 + un * w2;
+}
+
+// Whether fbou_point knows the boundary type
+__device__ __forceinline__ bool fbou_known(const FbouConst &fc, int ib) {
+    return ib == 1 || ib == 4 || ((fc.fam == 0 || fc.fam == 1) && (ib == 2 || ib == 3)) || (fc.fam == 1 && ib == 5);
 }
 
 // The boundary flux fh[NCU] of fbou.m at one face point, from the interior state u, its gradient

@@ -1,0 +1,280 @@
+// residual.cu -- getq (kernel/getq.m:37-104) and the element residual (kernel/cuda_residual.m:3-4) for
+// sm_100a: q solves its own equation for the given u and uh, Ru is evaluated at that q.
+//
+// No Jacobian is needed, so nothing of the local system is formed: C u and E uh are integrals of the
+// state and the trace at the quadrature points (C and E themselves are not built), and inv(M) is applied
+// to the NCU ND columns of q instead of to those of C, E and Rq (8 instead of 52 in 2D p = 3).  The
+// interpolations and integrals are products on FP64 fragments (column_product), one for all components;
+// with a thread a value they took half again as long (57 -> 42 us in the case below).
+//
+// What bounds it: the chain of some ten short phases an element (loads, geometry, inv(M), fluxes,
+// integrals), a few hundred to 3,000 cycles each; the DRAM traffic of an element is a few KB.  So a CTA is
+// one warp wherever an element's data is small (a barrier is then a warp's own, and 24 elements are in
+// flight on an SM), and launches of few elements give each of them four warps.
+// 2D NS p = 3, 8,450 elements: 205 us in the elemental kernel, 42 us here.  Error of Ru against extended
+// precision over 27 states (2D p = 1 .. 4, 3D p = 1 .. 3, Euler and NS), largest of the RMS: 8.1e-13 in both.
+#include "elemental_kernel.cuh"
+
+namespace hdgx {
+
+// Shared memory (in doubles): the tables, then one element.  The tiles that inv(M) publishes lie on what is
+// dead before it or written after it; a point's fluxes replace the gradient values they come from.
+template <class D>
+struct ResidualPlan {
+    static constexpr int NQD = D::NCU * D::ND, MT = (D::NPV + 7) / 8;
+    static constexpr int t_vt = 0, t_ft = t_vt + D::NGV * D::NPV, t_fg = t_ft + D::NGF * D::NPF;   // values
+    static constexpr int u = t_fg + D::NPF * D::NGF, Xx = u + D::NU, jac = Xx + D::NGV * D::ND * D::ND;
+    static constexpr int nl = jac + D::NGV, jf = nl + D::NGT * D::ND, ug = jf + D::NGT, fu = ug + D::NGV * D::NCU;
+    static constexpr int fuh = fu + D::NGT * D::NCU, M = fuh + D::NGT * D::NCU, R = M + D::NPV * D::NPV;
+    static constexpr int pub = ev(R + D::NPV * NQD), pub_doubles = (MT < 3 ? MT : 3) * MT * BlockGJ<D::NPV, NQD, 32>::TS;
+    static constexpr int gq = pub, wrk = gq, fq = gq + D::NGV * NQD, FH = fq;
+    static constexpr int qs = fq + D::NGT * NQD;                 // SH_q / fc_q, later the time source at the points
+    static constexpr int dg = qs + D::NPV * NQD, uh = dg + D::NPV * D::ND;
+    static constexpr int n_doubles = uh + D::NH > pub + pub_doubles ? uh + D::NH : pub + pub_doubles;
+    static constexpr int i_perm = 0, i_invp = D::NPF * D::NFE, i_bf = i_invp + D::NPV * D::NFE, i_bad = i_bf + D::NFE;
+    static constexpr size_t bytes = sizeof(double) * n_doubles + sizeof(int) * (i_bad + 2);
+    // one warp an element up to 12 KB, two up to 24 KB, four beyond
+    static constexpr int threads = bytes <= 12 * 1024 ? 32 : (bytes <= 24 * 1024 ? 64 : 128);
+    static_assert(D::NGV <= D::NPV * D::ND, "the time source fits the q source");
+};
+// CTAs per SM: what fits, at most `warps` warps.  24 of them leave a thread 80 registers: 2D NS p = 3, 8,450
+// elements: 48 us with 16, 42 with 24, 43 with 32; 3D p = 2, 24,576: 276, 258 and 260 us.
+template <class D>
+constexpr int residual_blocks(int nt, int warps) {
+    const int fit = (int)(227 * 1024 / (ResidualPlan<D>::bytes + 1024)), most = warps * 32 / nt;
+    return fit < most ? fit : most;
+}
+
+template <class D, int NT, int WARPS>
+__global__ void __launch_bounds__(NT, residual_blocks<D>(NT, WARPS)) residual_kernel(const __grid_constant__ ElemParams P) {
+    using L = ResidualPlan<D>;
+    constexpr int ND = D::ND, NPV = D::NPV, NPF = D::NPF, NGV = D::NGV, NGF = D::NGF, NFE = D::NFE, NCU = D::NCU;
+    constexpr int NC = D::NC, NDF = D::NDF, NU = D::NU, NH = D::NH, NGT = D::NGT, NQD = NCU * ND;
+    extern __shared__ __align__(16) double sm[];
+    double *t_vt = sm + L::t_vt, *t_ft = sm + L::t_ft, *t_fg = sm + L::t_fg;
+    double *s_dg = sm + L::dg, *s_u = sm + L::u, *s_uh = sm + L::uh, *s_Xx = sm + L::Xx, *s_jac = sm + L::jac;
+    double *s_nl = sm + L::nl, *s_jf = sm + L::jf, *s_ug = sm + L::ug, *s_fu = sm + L::fu, *s_fuh = sm + L::fuh;
+    double *s_gq = sm + L::gq, *s_fq = sm + L::fq, *s_M = sm + L::M, *s_R = sm + L::R, *s_qs = sm + L::qs, *s_wrk = sm + L::wrk, *s_FH = sm + L::FH;
+    int *si = reinterpret_cast<int *>(sm + L::n_doubles);
+    int *perm = si + L::i_perm, *invp = si + L::i_invp, *s_bf = si + L::i_bf, *s_bad = si + L::i_bad;
+    const double *__restrict__ t_vg = P.shapvg, *__restrict__ t_mv = P.shapmv, *__restrict__ t_mf = P.shapmf;
+    const int tid = threadIdx.x;
+
+    for (int i = tid; i < NGV * NPV; i += NT) t_vt[i] = P.shapvt[i];
+    for (int i = tid; i < NGF * NPF; i += NT) {
+        t_ft[i] = P.shapft[i];
+        t_fg[i] = P.shapfg[i];
+    }
+    for (int i = tid; i < NPF * NFE; i += NT) perm[i] = P.perm[i] - 1;
+    for (int i = tid; i < NPV * NFE; i += NT) invp[i] = -1;
+    __syncthreads();
+    for (int i = tid; i < NPF * NFE; i += NT) invp[perm[i] + NPV * (i / NPF)] = i % NPF;
+
+    // the right factors of the products (column_product): shape functions at the volume points, of the element's
+    // nodes at the face points, of the face nodes there; gradients at the volume points by row, face shape functions by row
+    auto at_volume = [&](int g, int n) { return t_vt[g + NGV * n]; };
+    auto at_faces = [&](int gg, int n) {
+        const int m = invp[n + NPV * (gg / NGF)];
+        return m >= 0 ? t_ft[gg % NGF + NGF * (m >= 0 ? m : 0)] : 0.0;
+    };
+    auto trace = [&](int gg, int f) { return f / NPF == gg / NGF ? t_ft[gg % NGF + NGF * (f % NPF)] : 0.0; };
+    auto gradient = [&](int r, int kk) { return __ldg(t_vg + r + NPV * (kk + NGV)); };
+    auto on_face = [&](int r, int gg) {
+        const int m = invp[r + NPV * (gg / NGF)];
+        return m >= 0 ? t_fg[(m >= 0 ? m : 0) + NPF * (gg % NGF)] : 0.0;
+    };
+    auto none = [](int, int, double (&)[1]) {};
+    auto zero = [](int, int) { return 0.0; };
+
+    for (int e = blockIdx.x; e < P.ne; e += gridDim.x) {
+        // ---- the element's nodes, u, trace and q source
+        const double *__restrict__ g_dg = P.dgnodes + (size_t)e * NPV * ND, *__restrict__ g_u = P.UDG + (size_t)e * NPV * NC;
+        const double *__restrict__ g_uh = P.UH + (size_t)e * NH, *__restrict__ g_sh = P.SH ? P.SH + (size_t)e * NPV * NC : nullptr;
+        for (int i = tid; i < NPV * ND; i += NT) s_dg[i] = __ldg(g_dg + i);
+        for (int i = tid; i < NU; i += NT) s_u[i] = __ldg(g_u + i);
+        for (int i = tid; i < NH; i += NT) s_uh[i] = __ldg(g_uh + i);
+        if (g_sh)
+            for (int i = tid; i < NPV * NQD; i += NT) s_qs[i] = __ldg(g_sh + NU + i) / P.fc_q;
+        if (tid < NFE) s_bf[tid] = P.bf[(size_t)e * NFE + tid];
+        if (tid < 2) s_bad[tid] = 0;
+        __syncthreads();
+
+        // ---- volgeom.m:18-61 (Jg(k,m) = dx_m/dxi_k; Xx = adj(Jg)), facegeom.m:20-52; u and uh at the points
+        for (int i = tid; i < NGV + NGT; i += NT) {
+            if (i < NGV) {
+                const int g = i;
+                double J[ND][ND] = {};
+#pragma unroll
+                for (int n = 0; n < NPV; n++)
+#pragma unroll
+                    for (int k = 0; k < ND; k++)
+#pragma unroll
+                        for (int m = 0; m < ND; m++) J[k][m] += __ldg(t_mv + g + NGV * (n + NPV * (k + 1))) * s_dg[n + NPV * m];
+                s_jac[g] = adjugate<ND>(J, s_Xx + g, NGV);
+            } else {
+                const int gg = i - NGV, g = gg % NGF, j = gg / NGF;
+                double dp[ND][ND - 1] = {};
+#pragma unroll
+                for (int n = 0; n < NPF; n++) {
+                    const int v = perm[n + NPF * j];
+#pragma unroll
+                    for (int k = 0; k < ND - 1; k++)
+#pragma unroll
+                        for (int m = 0; m < ND; m++) dp[m][k] += __ldg(t_mf + g + NGF * (n + NPF * (k + 1))) * s_dg[v + NPV * m];
+                }
+                double v[ND];
+                s_jf[gg] = face_normal<ND>(dp, v);
+#pragma unroll
+                for (int d = 0; d < ND; d++) s_nl[gg + NGT * d] = v[d];    // (area factor) n: one rounding instead of three
+            }
+        }
+        column_product<1, NGV, NPV, 0, NCU, NT>([&](int a, int n, double (&w)[1]) { w[0] = s_u[n + NPV * a]; }, at_volume, none,
+                                                zero, [&](int a, int, int g, double v) { s_ug[g + NGV * a] = v; });
+        column_product<1, NGT, NPV, 0, NCU, NT>(
+            [&](int a, int n, double (&w)[1]) { w[0] = s_u[n + NPV * a]; }, at_faces, none, zero,
+            [&](int a, int, int gg, double v) { s_fu[gg + NGT * a] = v; });
+        column_product<1, NGT, NDF, 0, NCU, NT>([&](int a, int f, double (&w)[1]) { w[0] = s_uh[a + NCU * f]; }, trace, none,
+                                                zero, [&](int a, int, int gg, double v) { s_fuh[gg + NGT * a] = v; });
+        __syncthreads();
+
+        // ---- M (volint.m:43), C u and E uh (volint.m:44-55, faceint.m:37-51) from the values at the points
+        column_product<1, NPV, NGV, 0, NPV, NT>(
+            [&](int s, int g, double (&w)[1]) { w[0] = t_vt[g + NGV * s] * s_jac[g]; },
+            [&](int r, int g) { return __ldg(t_vg + r + NPV * g); }, none, zero,
+            [&](int s, int, int r, double v) { s_M[r + NPV * s] = P.fc_q * v; });
+        column_product<1, NPV, NGV * ND, NGT, NQD, NT>(
+            [&](int c, int kk, double (&w)[1]) {
+                const int g = kk % NGV, jd = kk / NGV, a = c % NCU, d = c / NCU;
+                w[0] = s_ug[g + NGV * a] * s_Xx[g + NGV * (d + ND * jd)];
+            },
+            gradient,
+            [&](int c, int gg, double (&w)[1]) {
+                const int a = c % NCU, d = c / NCU;
+                w[0] = -s_nl[gg + NGT * d] * s_fuh[gg + NGT * a];
+            },
+            on_face, [&](int c, int, int r, double v) { s_R[r + NPV * c] = v; });
+        __syncthreads();
+        if (g_sh) {
+            column_product<1, NPV, NPV, 0, NQD, NT>([&](int c, int n, double (&w)[1]) { w[0] = s_qs[n + NPV * c]; },
+                                                    [&](int r, int n) { return s_M[r + NPV * n]; }, none, zero,
+                                                    [&](int c, int, int r, double v) { s_R[r + NPV * c] += v; });
+            __syncthreads();
+        }
+
+        // ---- q = inv(M) (M SH_q / fc_q + C u - E uh): M is SPD, eliminated without pivoting
+        block_gj<NPV, NQD, NPV, NT>(s_M, s_R, sm + L::pub, s_bad, NaturalOrder{});
+        __syncthreads();
+        if (P.QDG) {
+            for (int i = tid; i < NPV * NQD; i += NT) P.QDG[(size_t)e * NPV * NQD + i] = s_R[i];
+            if (tid == 0 && P.status) P.status[e] = *s_bad ? 1 : 0;
+            __syncthreads();
+            continue;
+        }
+        if (P.pc.rinv != 0.0) {                        // (the inviscid flux does not depend on q)
+            auto gradients = [&](int c, int n, double (&w)[1]) { w[0] = s_R[n + NPV * c]; };
+            column_product<1, NGV, NPV, 0, NQD, NT>(gradients, at_volume, none, zero,
+                                                    [&](int c, int, int g, double v) { s_gq[g + NGV * c] = v; });
+            column_product<1, NGT, NPV, 0, NQD, NT>(gradients, at_faces, none, zero,
+                                                    [&](int c, int, int gg, double v) { s_fq[gg + NGT * c] = v; });
+            __syncthreads();
+        }
+
+        // ---- fluxes: volint.m:81, 241-254, and fhat.m:49-67 = f(uh,q).n + tau (u - uh)
+        for (int i = tid; i < NGV + NGT; i += NT) {
+            const bool vol = i < NGV;
+            const int gg = i - NGV;
+            const double *pu = vol ? s_ug + i : s_fuh + gg, *pq = vol ? s_gq + i : s_fq + gg;
+            const int stride = vol ? NGV : NGT;
+            D0 u[NCU], q[NQD] = {}, f[NQD];
+#pragma unroll
+            for (int c = 0; c < NCU; c++) u[c] = {pu[stride * c]};
+            if (P.pc.rinv != 0.0) {
+#pragma unroll
+                for (int c = 0; c < NQD; c++) q[c] = {pq[stride * c]};
+            }
+            ns_flux<ND>(P.pc, u, q, f);
+            if (vol) {
+#pragma unroll
+                for (int id = 0; id < ND; id++)
+#pragma unroll
+                    for (int a = 0; a < NCU; a++) {
+                        double w = 0.0;
+#pragma unroll
+                        for (int jd = 0; jd < ND; jd++) w += f[a + NCU * jd].v * s_Xx[i + NGV * (jd + ND * id)];
+                        s_wrk[i + NGV * (id + ND * a)] = w;
+                    }
+            } else {
+                const int b = s_bf[gg / NGF], ib = -b - 1;
+                // the boundary flux enters Rh only; an unknown type is still reported
+                if (b < 0) {
+                    const int type = ib < P.nbnd ? P.bcm[ib] : -1;
+                    if (type != 6 && !(type == 5 && P.fb.fam == 0) && !fbou_known(P.fb, type)) s_bad[1] = 3;
+                }
+#pragma unroll
+                for (int a = 0; a < NCU; a++) {
+                    double fn = s_jf[gg] * (P.pc.tau * (s_fu[gg + NGT * a] - s_fuh[gg + NGT * a]));
+#pragma unroll
+                    for (int jd = 0; jd < ND; jd++) fn += f[a + NCU * jd].v * s_nl[gg + NGT * jd];
+                    s_FH[gg + NGT * a] = fn;
+                }
+            }
+        }
+        if (P.tdep) {
+            // s = SH_u - fc_u u at the points, times jac (volint.m:180-221 with dtcoef = 1 and no axisymmetry)
+            column_product<1, NGV, NPV, 0, NCU, NT>(
+                [&](int a, int n, double (&w)[1]) { w[0] = g_sh ? __ldg(g_sh + n + NPV * a) : 0.0; }, at_volume, none, zero,
+                [&](int a, int, int g, double v) { s_qs[g + NGV * a] = (v - s_ug[g + NGV * a] * P.fc_u) * s_jac[g]; });
+        }
+        __syncthreads();
+
+        // ---- Ru (volint.m:241-258, faceint.m:306-331); the source's part waits in R, for the lane that adds it
+        if (P.tdep) {
+            column_product<1, NPV, NGV, 0, NCU, NT>([&](int a, int g, double (&w)[1]) { w[0] = s_qs[g + NGV * a]; },
+                                                    [&](int r, int g) { return __ldg(t_vg + r + NPV * g); }, none, zero,
+                                                    [&](int a, int, int r, double v) { s_R[r + NPV * a] = v; });
+        }
+        column_product<1, NPV, NGV * ND, NGT, NCU, NT>(
+            [&](int a, int kk, double (&w)[1]) { w[0] = s_wrk[kk + NGV * ND * a]; }, gradient,
+            [&](int a, int gg, double (&w)[1]) { w[0] = -s_FH[gg + NGT * a]; }, on_face,
+            [&](int a, int, int r, double v) { P.RU[(size_t)e * NU + r + NPV * a] = P.tdep ? v + s_R[r + NPV * a] : v; });
+        if (tid == 0 && P.status) P.status[e] = s_bad[1] ? s_bad[1] : (s_bad[0] ? 1 : 0);
+        __syncthreads();
+    }
+}
+
+template <class D, int NT, int WARPS>
+static int launch(const ElemParams &p, cudaStream_t st) {
+    using L = ResidualPlan<D>;
+    auto kern = residual_kernel<D, NT, WARPS>;
+    if (allow_dynamic_smem((const void *)kern, L::bytes) != cudaSuccess) return -10;
+    static std::atomic<int> per_sm_cache[kMaxDevices];
+    const int dev = current_device(), nsm = sm_count_of(dev);
+    std::atomic<int> &cached = per_sm_cache[dev < kMaxDevices ? dev : 0];
+    int per_sm = cached.load(std::memory_order_relaxed);
+    if (per_sm < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, L::bytes) != cudaSuccess || per_sm < 1) return -11;
+        cached.store(per_sm, std::memory_order_relaxed);
+    }
+    const int grid = p.ne < nsm * per_sm ? p.ne : nsm * per_sm;
+    kern<<<grid, NT, L::bytes, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -12;
+}
+
+// getq (p.QDG set) or the residual (p.RU set) of one element set
+template <class D>
+int residual_launch(const ElemParams &p, cudaStream_t st) {
+    if (p.ne < 1) return 0;
+    // Up to four elements an SM: four warps each (2D NS p = 3, 512 elements: 11.5 us with one, 9.2 with four;
+    // 1,152 elements: 12.4 and 16.1; 3D NS p = 3, 162 elements: 17.9 us with 128 registers a thread, 21.2 with 80).
+    if (p.ne <= sm_count_of(current_device()) * 4) return launch<D, 128, 16>(p, st);
+    return launch<D, ResidualPlan<D>::threads, 24>(p, st);
+}
+template int residual_launch<Tri1>(const ElemParams &, cudaStream_t);
+template int residual_launch<Tri2>(const ElemParams &, cudaStream_t);
+template int residual_launch<Tri3>(const ElemParams &, cudaStream_t);
+template int residual_launch<Tri4>(const ElemParams &, cudaStream_t);
+template int residual_launch<Tet1>(const ElemParams &, cudaStream_t);
+template int residual_launch<Tet2>(const ElemParams &, cudaStream_t);
+template int residual_launch<Tet3>(const ElemParams &, cudaStream_t);
+
+}  // namespace hdgx
