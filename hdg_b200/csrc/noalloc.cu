@@ -104,8 +104,8 @@ extern "C" int hdgx_gmres_bilu0_noalloc(const hdgx_bsr *A, const double *Hg, con
     if (int rc = scratch_address(&base)) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     // The array keeps the previous call's contents: clear it up to the end of this call's
-    // workspace, so that nothing of an earlier solve (Hessenberg columns, rotations, the grid
-    // barrier of the fused Gram-Schmidt step) can leak into this one.
+    // workspace, so that nothing of an earlier solve (Hessenberg columns, rotations, the tagged
+    // packets of the fused Gram-Schmidt step) can leak into this one.
     if (cudaMemsetAsync(base, 0, need, st) != cudaSuccess) return -12;
     return hdgx::gmres_bilu0_run(A, Hg, Mg, nullptr, b, x, restart, tol, maxit, iters, flag, relres, history, base,
                                  st);
