@@ -14,8 +14,9 @@
 //     sum_g sum_i shapvg(r,g,i) sum_d wrl_i(g,a,(b,d)) Z(g,.,d) where Z is Mi C / Mi E / Mi Rq
 //     interpolated to the Gauss points (sum factorisation; cf. the BMiCvol/BMiCface
 //     experiments at kernel/hdg_elemental.m:206-520).
-//   * GK = dRh/d(u,q) is applied to DUDG and DUDG_DUH at the face Gauss points:
+//   * GK = dRh/d(u,q) is applied to DUDG and (mixed form) DUDG_DUH at the face Gauss points:
 //     (GK X)(a,(n,j)) = sum_g shapfg(n,g) jac_g sum_c FHu(g,a,c) sum_m shapft(g,m) X(perm(m,j),c).
+//     The FP64 form writes AE = (H - GK_q Mi E) + (GK_u + GK_q Mi C) dlu and does not read DUDG_DUH back.
 // H is face-block diagonal and is added directly.  Results equal the reference's up to
 // floating-point summation order.
 #pragma once
@@ -327,13 +328,13 @@ struct PlanMma {
     static_assert(smem_bytes <= 227 * 1024, "the shared-memory part of the plan fits");
 };
 
-// Resident elements per SM: the kernel is latency-bound (barrier-separated phases, a 40-step
-// elimination), so more elements in flight per SM beat more threads per element.  A plan that
-// fits four CTAs per SM runs four of 128 threads, one that fits three runs three of 192 (up to
-// 112 registers each); the larger plans run two or one of 256.  (C2, 2D NS p = 3: 6.84 ms
-// with two CTAs of 256, 6.21 ms with three of 192; 2D p = 2: 3.01 -> 1.80 ms with four of 128.)
-// The volume tables shapvt / shapvg move from shared to global memory (read through L1) only
-// when that raises the number of resident CTAs (2D p = 4: 119 -> 108 KB, one -> two per SM).
+// Resident elements per SM: the kernel is latency-bound (barrier-separated phases), so more elements in
+// flight per SM beat more threads per element.  A plan that fits four CTAs per SM runs four of 128
+// threads, one that fits three runs three of 192 (up to 112 registers each); the larger plans run two or
+// one of 256.  (With scalar products, 2D NS p = 3, 32,768 elements: 6.84 ms with two CTAs of 256, 6.21 ms with
+// three of 192; 2D Euler p = 2: 3.01 -> 1.80 ms with four of 128.)  In the mixed form the volume tables shapvt /
+// shapvg move from shared to global memory (read through L1) only when that raises the number of resident
+// CTAs (2D p = 4: 119 -> 108 KB, one -> two per SM).
 constexpr int blocks_for(size_t bytes) {
     return bytes <= 45 * 1024 ? 4 : (bytes <= 74 * 1024 ? 3 : (bytes <= 113 * 1024 ? 2 : 1));
 }
