@@ -318,4 +318,39 @@ __device__ __forceinline__ bool backward_error_ok(const double *A, const double 
     return v[0] <= tol * (v[1] * v[2] + v[3]) && isfinite(v[0]);
 }
 
+// Whether X is the inverse of A (N x N, column-major, leading dimension N) as a stable elimination leaves it: for
+// every column j and row r, |(A x_j - e_j)_r| <= tol |A_r| |x_j| (row sum, largest entry; not a number is not).
+// Every column is looked at, as one of them says nothing about the unknowns that it does not reach.  Tiles of A X
+// over the warps, with the norms from the fragments; one barrier, every thread returns the answer.
+template <int N, int NT>
+__device__ __forceinline__ bool inverse_ok(const double *A, const double *X, double tol) {
+    constexpr int TN = (N + 7) / 8, NW = NT / 32;
+    const int lane = threadIdx.x & 31, m = lane >> 2, q = lane & 3;
+    bool ok = true;
+    for (int t = threadIdx.x >> 5; t < TN * TN; t += NW) {
+        const int r = 8 * (t % TN) + m, c = 8 * (t / TN) + m;
+        double acc[2] = {0.0, 0.0}, as = 0.0, xm = 0.0;
+#pragma unroll
+        for (int s = 0; s < (N + 3) / 4; s++) {
+            const int k = 4 * s + q;
+            const double a = r < N && k < N ? A[r + N * k] : 0.0, x = c < N && k < N ? X[k + N * c] : 0.0;
+            as += fabs(a);
+            xm = fmax(xm, fabs(x));
+            dmma(acc, a, x);
+        }
+        for (int o = 1; o < 4; o <<= 1) {                               // row r's sum, column c's largest entry
+            as += __shfl_xor_sync(0xffffffffu, as, o);
+            xm = fmax(xm, __shfl_xor_sync(0xffffffffu, xm, o));
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const double xc = __shfl_sync(0xffffffffu, xm, 4 * (2 * q + h));
+            const int j = 8 * (t / TN) + 2 * q + h;
+            const double res = fabs(acc[h] - (r == j ? 1.0 : 0.0));
+            if (r < N && j < N) ok &= isfinite(res) && res <= tol * as * xc;
+        }
+    }
+    return __syncthreads_and(ok);
+}
+
 }  // namespace hdgx
