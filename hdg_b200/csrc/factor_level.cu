@@ -90,6 +90,8 @@ __global__ void __launch_bounds__(FactorShape<BS>::NT)
             for (int s = 0; s < S::NP / 4; s++) dmma(acc, Am[r0 + m + LD * (4 * s + q)], Bm[4 * s + q + LD * (c0 + m)]);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
+                // the padding stays zero: what a singular block puts there would reach the CTA's next row
+                if (BS % 8 != 0 && (r0 + m >= BS || c0 + 2 * q + h >= BS)) continue;
                 double *c = Cm + r0 + m + LD * (c0 + 2 * q + h);
                 *c = subtract ? *c - acc[h] : acc[h];
             }
