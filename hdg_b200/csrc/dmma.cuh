@@ -284,38 +284,50 @@ __device__ __forceinline__ void block_gj_apply(double *B, const double *steps, O
     __syncthreads();
 }
 
-// Largest |b - A x| / (max row sum |A| max |x| + max |b|) of one column over the CTA, b read through bval;
-// every thread returns whether it is at most tol (NaN is not).  red: 4 doubles a warp.
-template <int N, int NT, class FB>
-__device__ __forceinline__ bool backward_error_ok(const double *A, const double *x, FB bval, double tol, double *red) {
-    double v[4] = {};
+// A fixed right-hand side without a zero, entries 1 to 2 in size: solved beside the others (the last tile of 8
+// columns has room for it in every shape), it shows what an elimination without pivoting did to all unknowns,
+// whichever of them the other right-hand sides reach, and also when those are zero.
+__device__ __forceinline__ double probe_rhs(int r) {
+    const int h = (37 * r + 11) & 63;
+    return h < 32 ? 1.0 + h / 32.0 : -1.0 - (h - 32) / 32.0;
+}
+
+// Whether x solves A x = probe_rhs as a stable elimination leaves it, over the CTA: for every row the residual is at
+// most kProbeError (|A| |x| + |b|) in the largest row sum and entries, and at most kProbeRow of the row's own
+// sum_c |a_rc x_c| + |b_r| (where a part of x is large it hides the rows of the others in the first measure; the
+// second allows more, since a sound elimination's fill-in exceeds a sparse row's own entries).  Not a number does not
+// pass.  red: 4 doubles a warp; every thread returns the answer.
+constexpr double kProbeError = 2e-15, kProbeRow = 1e-12;
+template <int N, int NT>
+__device__ __forceinline__ bool probe_ok(const double *A, const double *x, double *red) {
+    double v[3] = {};
+    bool row_ok = true;
     for (int r = threadIdx.x; r < N; r += NT) {
-        const double b = bval(r);
-        double res = b, as = 0.0;
+        double res = probe_rhs(r), own = fabs(res), as = 0.0;
         for (int c = 0; c < N; c++) {
-            const double a = A[r + N * c];
-            res -= a * x[c];
+            const double a = A[r + N * c], xc = x[c];
+            res -= a * xc;
+            own += fabs(a * xc);
             as += fabs(a);
         }
-        if (!(res == res)) res = INFINITY;
+        row_ok &= fabs(res) <= kProbeRow * own && isfinite(res);
         v[0] = fmax(v[0], fabs(res));
         v[1] = fmax(v[1], as);
         v[2] = fmax(v[2], fabs(x[r]));
-        v[3] = fmax(v[3], fabs(b));
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < 3; k++) {
         for (int o = 16; o > 0; o >>= 1) v[k] = fmax(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
         if ((threadIdx.x & 31) == 0) red[4 * (threadIdx.x >> 5) + k] = v[k];
     }
-    __syncthreads();
+    row_ok = __syncthreads_and(row_ok);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < 3; k++) {
         v[k] = 0.0;
         for (int w = 0; w < NT / 32; w++) v[k] = fmax(v[k], red[4 * w + k]);
     }
     __syncthreads();
-    return v[0] <= tol * (v[1] * v[2] + v[3]) && isfinite(v[0]);
+    return row_ok && v[0] <= kProbeError * (v[1] * v[2] + 2.0);
 }
 
 // Whether X is the inverse of A (N x N, column-major, leading dimension N) as a stable elimination leaves it: for

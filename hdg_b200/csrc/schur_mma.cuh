@@ -7,6 +7,8 @@
 //   SD = D + B Mi C,  R = [Ru - B Mi Rq | B Mi E - F],
 //   G' = GK_u + GK_q Mi C,  AE <- H - GK_q Mi E,
 // and after the solve AE += G' dlu, FE = Rh - GK_q Mi Rq - G' du (DUDG_DUH is never read back).
+// The blocks are a caller's: M and SD are eliminated without pivoting together with one fixed right-hand side
+// (probe_rhs), and again with partial pivoting when that is not solved to rounding.
 // Bound by the reads of the blocks and the elimination; 2D p = 3, 4,050 elements (190 KB each):
 // 3.41 -> 0.347 ms, of which the DRAM traffic takes 0.12 ms at 6.5 TB/s.
 #pragma once
@@ -89,10 +91,10 @@ template <int ND, int NPV, int NCU, int NDF>
 struct SchurShape {
     static constexpr int ev2(int x) { return (x + 1) / 2 * 2; }
     static constexpr int NC = NCU * (ND + 1), NU = NPV * NCU, NH = NCU * NDF, NQ = NPV * NC;
-    static constexpr int LDR = pad4(NU), SG = pad4(NH), NX = NPV * ND + NDF * ND + NCU * ND;
-    static constexpr int o_M = 0, o_Mi = o_M + NPV * NPV, o_SD = o_Mi + NPV * NX, o_R = ev2(o_SD + NU * NU),
-                         o_G = o_R + LDR * (1 + NH), o_pub = ev2(o_G + NU * SG),
-                         o_part = o_pub + BlockGJ<NU, 1, 32>::pub_doubles, o_b0 = o_part + NCU * NH, o_red = o_b0 + NU,
+    static constexpr int LDR = pad4(NU), SG = pad4(NH), NX = NPV * ND + NDF * ND + NCU * ND;   // and one probe_rhs
+    static constexpr int o_M = 0, o_Mi = o_M + NPV * NPV, o_SD = o_Mi + NPV * (NX + 1), o_R = ev2(o_SD + NU * NU),
+                         o_G = o_R + LDR * (2 + NH), o_pub = ev2(o_G + NU * SG),
+                         o_part = o_pub + BlockGJ<NU, 1, 32>::pub_doubles, o_red = o_part + NCU * NH,
                          o_int = o_red + 32, doubles = o_int;
     static constexpr int i_ord = 0, i_face = NU, i_var = i_face + NPV, i_slot = i_var + NU, i_bad = i_slot + 4, ints = i_bad + 2;
     static constexpr size_t bytes = sizeof(double) * doubles + sizeof(int) * ints;
@@ -105,14 +107,12 @@ __global__ void __launch_bounds__(SchurShape<ND, NPV, NCU, NDF>::threads, SchurS
     schur_uq_mma_kernel(const __grid_constant__ SchurParams P) {
     using S = SchurShape<ND, NPV, NCU, NDF>;
     constexpr int NT = S::threads, NU = S::NU, NH = S::NH, NQ = S::NQ, LDR = S::LDR, SG = S::SG, NX = S::NX;
-    // where a sound elimination without pivoting leaves 1.2e-16 at most
-    constexpr double kBackwardError = 2e-15;
     extern __shared__ __align__(16) double sm[];
     double *sM = sm + S::o_M, *sMi = sm + S::o_Mi, *sMiE = sMi + NPV * NPV * ND, *sMiRq = sMiE + NPV * NDF * ND;
     double *sSD = sm + S::o_SD, *sR = sm + S::o_R, *sG = sm + S::o_G, *pub = sm + S::o_pub, *part = sm + S::o_part;
     // the published blocks' place also holds B Mi Rq by component before SD's elimination, and what a pivoted one works with
     double *partu = pub, *fall = pub;
-    double *b0 = sm + S::o_b0, *red = sm + S::o_red;
+    double *red = sm + S::o_red;
     int *si = reinterpret_cast<int *>(sm + S::o_int), *ord = si + S::i_ord, *face = si + S::i_face, *var = si + S::i_var,
         *slot = si + S::i_slot, *sbad = si + S::i_bad;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, m = lane >> 2, q = lane & 3;
@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(SchurShape<ND, NPV, NCU, NDF>::threads, SchurS
             if (v != 0.0) face[i % NPV] = 1;             // a node of some face
         }
         for (int i = tid; i < NPV * NCU * ND; i += NT) sMiRq[i] = P.Rq[(size_t)e * NPV * NCU * ND + i];
+        for (int r = tid; r < NPV; r += NT) sMi[NPV * NX + r] = probe_rhs(r);
         __syncthreads();
         // the elimination order of the local system: face nodes first, the density of each kind last
         for (int r = tid; r < NPV; r += NT) {
@@ -150,8 +151,8 @@ __global__ void __launch_bounds__(SchurShape<ND, NPV, NCU, NDF>::threads, SchurS
             o[(NCU - 1) * n + before] = r;
         }
         if (pivot_m) gj_regs<NPV, NX, NT, 8, true>(sM, sMi, fall, fall + 2 * NPV, var, slot, sbad);
-        else block_gj<NPV, NX, NPV, NT>(sM, sMi, pub, sbad, NaturalOrder{});
-        if (!pivot_m && (!backward_error_ok<NPV, NT>(sM, sMi, [&](int r) { return C[r]; }, kBackwardError, red) || *sbad)) {
+        else block_gj<NPV, NX + 1, NPV, NT>(sM, sMi, pub, sbad, NaturalOrder{});
+        if (!pivot_m && (!probe_ok<NPV, NT>(sM, sMi + NPV * NX, red) || *sbad)) {
             pivot_m = true;
             __syncthreads();
             goto element;
@@ -187,14 +188,15 @@ __global__ void __launch_bounds__(SchurShape<ND, NPV, NCU, NDF>::threads, SchurS
             double v = P.Ru[(size_t)e * NU + r];
 #pragma unroll
             for (int b = 0; b < NCU; b++) v -= partu[r + NU * b];
-            sR[r] = b0[r] = v;
+            sR[r] = v;
+            sR[LDR * (1 + NH) + r] = probe_rhs(r);
         }
         __syncthreads();
         if (pivot_sd) {
             gj_regs<NU, 1 + NH, NT, 8, true, LDR>(sSD, sR, fall, fall + 2 * NU, var, slot, sbad);
         } else {
-            block_gj<NU, 1 + NH, LDR, NT>(sSD, sR, pub, sbad, TableOrder{ord});
-            if (!backward_error_ok<NU, NT>(sSD, sR, [&](int r) { return b0[r]; }, kBackwardError, red) || *sbad != bad_m) {
+            block_gj<NU, 2 + NH, LDR, NT>(sSD, sR, pub, sbad, TableOrder{ord});
+            if (!probe_ok<NU, NT>(sSD, sR + LDR * (1 + NH), red) || *sbad != bad_m) {
                 pivot_sd = true;
                 __syncthreads();
                 goto element;
