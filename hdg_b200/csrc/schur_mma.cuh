@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(SchurShape<ND, NPV, NCU, NDF>::threads, SchurS
     schur_uq_mma_kernel(const __grid_constant__ SchurParams P) {
     using S = SchurShape<ND, NPV, NCU, NDF>;
     constexpr int NT = S::threads, NU = S::NU, NH = S::NH, NQ = S::NQ, LDR = S::LDR, SG = S::SG, NX = S::NX;
+    static_assert(NQ >= NH, "DUDG_DUH has room for a trace Jacobian");
     extern __shared__ __align__(16) double sm[];
     double *sM = sm + S::o_M, *sMi = sm + S::o_Mi, *sMiE = sMi + NPV * NPV * ND, *sMiRq = sMiE + NPV * NDF * ND;
     double *sSD = sm + S::o_SD, *sR = sm + S::o_R, *sG = sm + S::o_G, *pub = sm + S::o_pub, *part = sm + S::o_part;
@@ -121,6 +122,7 @@ __global__ void __launch_bounds__(SchurShape<ND, NPV, NCU, NDF>::threads, SchurS
         const double *H = P.H + (size_t)e * NH * NH, *C = P.C + (size_t)e * NPV * NPV * ND;
         double *dd = P.DUDG_DUH + (size_t)e * NQ * NH, *ae = P.AE + (size_t)e * NH * NH;
         const bool wide = (((size_t)P.DUDG_DUH | (size_t)P.AE) & 15) == 0;
+        double *ah = ae;                                 // where H - GK_q Mi E goes
         bool pivot_m = false, pivot_sd = false;          // an elimination failed its check: again, with pivoting
     element:
         if (tid == 0) *sbad = 0;
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(SchurShape<ND, NPV, NCU, NDF>::threads, SchurS
             },
             [&](int b, int col, int r, double v) {
                 if (col < NPV) sG[SG * (col + NPV * b) + r] = v;
-                else if (col < NPV + NDF) ae[r + NH * (b + NCU * (col - NPV))] = -v;
+                else if (col < NPV + NDF) ah[r + NH * (b + NCU * (col - NPV))] = -v;
                 else part[r + NH * b] = v;
             });
         __syncthreads();
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(SchurShape<ND, NPV, NCU, NDF>::threads, SchurS
             block_gj<NU, 2 + NH, LDR, NT>(sSD, sR, pub, sbad, TableOrder{ord});
             if (!probe_ok<NU, NT>(sSD, sR + LDR * (1 + NH), red) || *sbad != bad_m) {
                 pivot_sd = true;
+                ah = dd;                                 // AE may lie over H: it keeps what it has (dd is written below)
                 __syncthreads();
                 goto element;
             }
