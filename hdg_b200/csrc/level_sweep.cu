@@ -93,10 +93,11 @@ struct SweepShape {
     static constexpr int WPC = fit > 16 ? 16 : fit;
     static constexpr size_t smem = warp_bytes * WPC;
     // Products of the neighbours that have arrived, while the last one is waited for: pays where a block's product
-    // is long.  Apply in us, all at once / as they arrive: blocks of 30, 6,528 faces in 282 levels, 702 / 597; of 20, 1,776
+    // is long.  Each has a sum of its own, and these are added in slot order, so that the result does not depend on who
+    // came first (apply 536 -> 539 us; products in slot order, each when it and those before it are there: 614).  Apply in us, all at once / as they arrive: blocks of 30, 6,528 faces in 282 levels, 702 / 597; of 20, 1,776
     // in 160, 251 / 255; of 16, 12,416 in 440, 592 / 623; of 12, 800 in 104, 129 / 133.
     static constexpr bool EARLY = BS > 20;
-    static_assert(!EARLY || PARTS == 1, "the slots of a warp are one row's");
+    static_assert(!EARLY || (PARTS == 1 && DP <= 6), "the slots of a warp are one row's");
     static_assert(BS <= 32 && RW <= 32 && WPC >= 1, "one lane per row component and per record entry");
 };
 
@@ -216,7 +217,8 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
             }
             // wait for the neighbours' values (and, backward, for the row's own y)
             unsigned long long got[DP], own = 0;
-            double acc[CH] = {};
+            [[maybe_unused]] double acc[CH] = {};
+            [[maybe_unused]] double each[6] = {};                        // EARLY: a neighbour's product
             unsigned todo = 0;                                           // slots whose product is to be added
 #pragma unroll
             for (int s = 0; s < DP; s++) todo |= k[s] >= 0 ? 1u << s : 0u;
@@ -228,7 +230,15 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
 #pragma unroll
                 for (int s = 0; s < DP; s++) {
                     const int d = part + s * PARTS;
-                    if (which >> s & 1) dot_cols<BS, BS, CH>(blk + d * BLK + r, val + d * BSP, 0, acc);
+                    if (which >> s & 1) {
+                        if constexpr (S::EARLY) {
+                            double one[CH] = {};
+                            dot_cols<BS, BS, CH>(blk + d * BLK + r, val + d * BSP, 0, one);
+                            each[s] = chain_sum(one);
+                        } else {
+                            dot_cols<BS, BS, CH>(blk + d * BLK + r, val + d * BSP, 0, acc);
+                        }
+                    }
                 }
             };
             for (int n = 0;;) {
@@ -254,7 +264,9 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
             }
             use(todo);
             if (!staged) xv = __longlong_as_double((long long)(own = kPending));
-            const double sum = add_parts(chain_sum(acc));
+            double sum;
+            if constexpr (S::EARLY) sum = (each[0] + each[1]) + (each[2] + each[3]) + (each[4] + each[5]);
+            else sum = add_parts(chain_sum(acc));
             if (!BWD) {
                 if (part == 0) store_value(out + (size_t)BS * i + r, xv - sum);
             } else {
