@@ -90,6 +90,7 @@ const char *hdgx_status_str(int code) {
         case -13: return "CUDA error while counting status";
         case -14: return "a flag-synchronised BILU(0) sweep gave up waiting (bounded spin)";
         case -15: return "the fused Gram-Schmidt step gave up waiting for another block's partial sum (bounded spin)";
+        case -16: return "a single-launch BILU(0) sweep gave up waiting for a value (bounded spin)";
         default:
             if (code <= -1000) return cudaGetErrorString((cudaError_t)(-1000 - code));
             return "unknown status";

@@ -87,13 +87,13 @@ static void sweep_color(const hdgx_bsr *A, int dir, const int *rows, int nr, con
 }
 
 int factor_level(const hdgx_bsr *A, const int *rows, int nr, double *Mg, int *status, bool first, cudaStream_t st);
-int level_sweep_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, cudaStream_t st);
-int level_sweep_apply_f32(const hdgx_bsr *A, const float *Mg, const double *x, double *y, double *v, cudaStream_t st);
+int level_sweep_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, int *err, cudaStream_t st);
+int level_sweep_apply_f32(const hdgx_bsr *A, const float *Mg, const double *x, double *y, double *v, int *err, cudaStream_t st);
 
-int trace_bilu0_apply_f32(const hdgx_bsr *A, const float *Mg32, const double *x, double *y, double *v,
+int trace_bilu0_apply_f32(const hdgx_bsr *A, const float *Mg32, const double *x, double *y, double *v, int *err,
                           cudaStream_t st) {
     if (!A->sweep_plan || A->ncolors < 1) return -2;
-    if (level_sweep_apply_f32(A, Mg32, x, y, v, st) != 0) return -2;
+    if (level_sweep_apply_f32(A, Mg32, x, y, v, err, st) != 0) return -2;
     return launched();
 }
 
@@ -109,7 +109,8 @@ static int resident_grid(const void *kern, int threads, size_t smem, int cap) {
     return g < cap ? g : cap;
 }
 
-int trace_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, cudaStream_t st) {
+int trace_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, int *err,
+                      cudaStream_t st) {
     const int threads = 256, warps = threads / 32;
     if (A->ncolors == 0) {
         if (!A->sched) return -1;
@@ -124,7 +125,7 @@ int trace_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, doub
         return launched();
     }
     (void)warps;
-    if (A->sweep_plan && level_sweep_apply(A, Mg, x, y, v, st) == 0) return launched();
+    if (A->sweep_plan && level_sweep_apply(A, Mg, x, y, v, err, st) == 0) return launched();
     for (int c = 0; c < A->ncolors; c++) {
         const int r0 = A->color_ptr[c], nr = A->color_ptr[c + 1] - r0;
         if (nr > 0) sweep_color(A, 0, A->color_rows + r0, nr, Mg, x, y, st);
@@ -239,7 +240,7 @@ int hdgx_bilu0_factor(const hdgx_bsr *A, double *Mg, int *status, hdgx_stream_t 
 
 int hdgx_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *v, double *work, hdgx_stream_t stream) {
     if (!A || !Mg || !x || !v || !work) return -1;
-    return trace_bilu0_apply(A, Mg, x, work, v, (cudaStream_t)stream);
+    return trace_bilu0_apply(A, Mg, x, work, v, nullptr, (cudaStream_t)stream);
 }
 
 int hdgx_backsub(int npv, int nc, int ncu, int ndf, int ne, const int *elcon, const double *DUDG,
@@ -283,9 +284,6 @@ constexpr size_t kGmresBatchMaxN = 262144;
 int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const float *Mg32, const double *b,
                     double *x, int restart, double tol, int maxit, int *iters, int *flag, double *relres,
                     double *history, void *mem, cudaStream_t st) {
-    auto prec = [&](const double *in, double *y, double *v) {
-        return Mg32 ? trace_bilu0_apply_f32(A, Mg32, in, y, v, st) : trace_bilu0_apply(A, Mg, in, y, v, st);
-    };
     const size_t N = (size_t)A->bs * A->nf;
     const int m = restart;
     double *V = (double *)mem;
@@ -298,13 +296,16 @@ int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const
     gs.y = gs.g + (m + 1);
     gs.scal = gs.y + (m + 1);
     double *part = gs.scal + 8;                   // [1024] partial sums
-    int *mgs_flag = reinterpret_cast<int *>(part + 1024);        // error flag of the fused step
+    int *flags = reinterpret_cast<int *>(part + 1024);           // error flags of the fused step and of the sweeps
     gs.hist = part + 1024 + 2;                    // [m] residual norm after each step of a cycle
     // [4 kMgsBlocks] packets of the fused step, on a 16-byte boundary
     unsigned long long *packets = reinterpret_cast<unsigned long long *>(((size_t)(gs.hist + m) + 15) & ~(size_t)15);
     unsigned mgs_tag = 1;                         // tags run on over the whole solve
-    cudaMemsetAsync(mgs_flag, 0, sizeof(int), st);
+    cudaMemsetAsync(flags, 0, 2 * sizeof(int), st);
     cudaMemsetAsync(packets, 0, sizeof(unsigned long long) * 4 * kMgsBlocks, st);
+    auto prec = [&](const double *in, double *y, double *v) {
+        return Mg32 ? trace_bilu0_apply_f32(A, Mg32, in, y, v, flags + 1, st) : trace_bilu0_apply(A, Mg, in, y, v, flags + 1, st);
+    };
     // host scalars on the stack (pageable copies are stream-ordered and, unlike freeing
     // pinned memory, never synchronise the other streams of the device)
     double h_scal[1 + kGmresBatch] = {};
@@ -326,7 +327,9 @@ int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const
     const double nrmb = *h_nrmb;
     int iter = 0, fl = 2;
     double res_rel = 0.0;
-    if (!(nrmb > 0.0) || rc) { fl = rc ? 3 : 0; res_rel = 0.0; }
+    if (rc) fl = 3;
+    else if (!isfinite(nrmb)) { fl = 3; res_rel = nrmb; }
+    else if (nrmb == 0.0) fl = 0;                 // x solves it as it is, to the norm of the right-hand side
     while (fl == 2) {
         // r = pb - P^{-1} A x -> V[:,0] = r / beta
         if (int r = trace_matvec(A, Hg, x, t, st)) rc = rc ? rc : r;
@@ -350,7 +353,7 @@ int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const
                 if (int r = trace_matvec(A, Hg, vj, t, st)) rc = rc ? rc : r;
                 if (int r = prec(t, w2, w)) rc = rc ? rc : r;
                 double *hc = gs.H + (size_t)(m + 1) * j;
-                const bool fused = mgs_fused(N, j + 1, V, w, packets, mgs_tag, mgs_flag, gs, m, st);
+                const bool fused = mgs_fused(N, j + 1, V, w, packets, mgs_tag, flags, gs, m, st);
                 mgs_tag += (unsigned)j + 3;
                 if (!fused) {
                     for (int i = 0; i <= j; i++) {        // modified Gram-Schmidt (gmres_bilu0.m:59-63)
@@ -387,8 +390,8 @@ int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const
     if (iters) *iters = iter;
     if (flag) *flag = fl;
     if (relres) *relres = res_rel;
-    int mgs_err = 0;
-    cudaMemcpyAsync(&mgs_err, mgs_flag, sizeof(int), cudaMemcpyDeviceToHost, st);
+    int errs[2] = {};
+    cudaMemcpyAsync(errs, flags, sizeof(errs), cudaMemcpyDeviceToHost, st);
     synced();
     int sched_err = 0;
     if (A->ncolors == 0 && A->sched) {
@@ -399,7 +402,8 @@ int gmres_bilu0_run(const hdgx_bsr *A, const double *Hg, const double *Mg, const
     if (rc) return rc;
     if (cudaGetLastError() != cudaSuccess) return -12;
     if (sched_err) return -14;
-    if (mgs_err) return -15;
+    if (errs[0]) return -15;
+    if (errs[1]) return -16;
     return 0;
 }
 

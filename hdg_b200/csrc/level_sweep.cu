@@ -17,8 +17,8 @@
 // here produces: a result with these bits is stored as the default NaN) before the launch, and a
 // reader polls the value itself at L2 until it differs.  One store and one load carry a row to its
 // readers; there is no fence, no barrier and no separate flag.  Waits are bounded (kPollLimit
-// polls, then NaN is used and passed on, so that a plan that is not a schedule ends in NaN, never
-// in a hang).
+// polls, then NaN is used and passed on and *err, where there is one, is set, so that a plan that
+// is not a schedule ends in NaN and in an error of the solve, never in a hang).
 //
 // What bounds a level is then the store-to-load time through L2 (0.47 us measured between two SMs)
 // and the arithmetic after it, so both are kept short: the row's factor blocks are staged in
@@ -119,7 +119,7 @@ __device__ __forceinline__ double chain_sum(const double (&acc)[CH]) {
 template <int BS, int MAXD, class MT>
 __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
     bilu0_sweep_kernel(int nf, const int *__restrict__ rec, const MT *__restrict__ Mg, const double *__restrict__ x,
-                       double *y, double *v, int phases) {
+                       double *y, double *v, int phases, int *err) {
     using S = SweepShape<BS, MAXD, MT>;
     constexpr int PARTS = S::PARTS, DP = S::DP, RW = S::RW, BLK = S::BLK, BSP = S::BSP, CH = S::CH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -210,7 +210,10 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
             bool staged = true;
             if (wide) {
                 staged = stage_wait(bar, parity, stage_limit);
-                if (!staged) stage_limit = 1;
+                if (!staged) {
+                    stage_limit = 1;
+                    if (err && lane == 0) atomicExch(err, 1);
+                }
                 parity ^= 1;
             } else {
                 asm volatile("cp.async.wait_all;" ::: "memory");
@@ -252,6 +255,7 @@ __global__ void __launch_bounds__(SweepShape<BS, MAXD, MT>::WPC * 32)
                 if (__all_sync(0xffffffffu, !miss)) break;
                 if (++n >= limit) {                                      // NaN (kPending is one) from here on
                     limit = 1;
+                    if (err && lane == 0) atomicExch(err, 1);
                     break;
                 }
                 if constexpr (S::EARLY) {
@@ -304,7 +308,7 @@ __global__ void fill_pending_kernel(size_t n, unsigned long long *a, unsigned lo
 // together or not at all, so that the sweeps of many concurrent solves share the GPU; larger grids
 // are a cooperative launch.
 template <int BS, int MAXD, class MT>
-static int launch_sweep(const hdgx_bsr *A, const MT *Mg, const double *x, double *y, double *v, cudaStream_t st) {
+static int launch_sweep(const hdgx_bsr *A, const MT *Mg, const double *x, double *y, double *v, int *err, cudaStream_t st) {
     using S = SweepShape<BS, MAXD, MT>;
     auto kern = bilu0_sweep_kernel<BS, MAXD, MT>;
     if (allow_dynamic_smem((const void *)kern, S::smem) != cudaSuccess) {
@@ -327,7 +331,7 @@ static int launch_sweep(const hdgx_bsr *A, const MT *Mg, const double *x, double
     auto launch = [&](int phases) -> bool {
         if (G > 8) {
             int nf_ = nf, ph = phases;
-            void *args[] = {&nf_, &rec, &Mg, &x, &y, &v, &ph};
+            void *args[] = {&nf_, &rec, &Mg, &x, &y, &v, &ph, &err};
             if (cudaLaunchCooperativeKernel((const void *)kern, dim3(G), dim3(S::WPC * 32), args, S::smem, st) == cudaSuccess)
                 return true;
             cudaGetLastError();
@@ -344,7 +348,7 @@ static int launch_sweep(const hdgx_bsr *A, const MT *Mg, const double *x, double
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kern, nf, rec, Mg, x, y, v, phases) == cudaSuccess;
+        return cudaLaunchKernelEx(&cfg, kern, nf, rec, Mg, x, y, v, phases, err) == cudaSuccess;
     };
     unsigned long long *yb = reinterpret_cast<unsigned long long *>(y), *vb = reinterpret_cast<unsigned long long *>(v);
     if (v == x) {                                       // x is read before v is marked
@@ -360,7 +364,8 @@ static int launch_sweep(const hdgx_bsr *A, const MT *Mg, const double *x, double
 // 0 when launched, 1 when there is no plan, no specialisation for it, or the vectors overlap in a
 // way the marked values do not allow (the caller falls back to one launch per level)
 template <class MT>
-static int level_sweep_apply_t(const hdgx_bsr *A, const MT *Mg, const double *x, double *y, double *v, cudaStream_t st) {
+static int level_sweep_apply_t(const hdgx_bsr *A, const MT *Mg, const double *x, double *y, double *v, int *err,
+                               cudaStream_t st) {
     if (!A->sweep_plan || A->ncolors < 1 || A->nf < 1) return 1;
     const int md = A->sweep_maxd;
     if (md != 4 && md != 6) return 1;
@@ -370,19 +375,20 @@ static int level_sweep_apply_t(const hdgx_bsr *A, const MT *Mg, const double *x,
     switch (A->bs) {
 #define HDGX_LS(B)                                                                            \
     case B:                                                                                   \
-        return md == 4 ? launch_sweep<B, 4, MT>(A, Mg, x, y, v, st) : launch_sweep<B, 6, MT>(A, Mg, x, y, v, st);
+        return md == 4 ? launch_sweep<B, 4, MT>(A, Mg, x, y, v, err, st) : launch_sweep<B, 6, MT>(A, Mg, x, y, v, err, st);
         HDGX_LS(8) HDGX_LS(12) HDGX_LS(15) HDGX_LS(16) HDGX_LS(20) HDGX_LS(30)
 #undef HDGX_LS
         default: return 1;
     }
 }
 
-int level_sweep_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, cudaStream_t st) {
-    return level_sweep_apply_t<double>(A, Mg, x, y, v, st);
+int level_sweep_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, int *err, cudaStream_t st) {
+    return level_sweep_apply_t<double>(A, Mg, x, y, v, err, st);
 }
 // The same sweeps with the factors stored in FP32 (the mixed-precision preconditioner)
-int level_sweep_apply_f32(const hdgx_bsr *A, const float *Mg, const double *x, double *y, double *v, cudaStream_t st) {
-    return level_sweep_apply_t<float>(A, Mg, x, y, v, st);
+int level_sweep_apply_f32(const hdgx_bsr *A, const float *Mg, const double *x, double *y, double *v, int *err,
+                          cudaStream_t st) {
+    return level_sweep_apply_t<float>(A, Mg, x, y, v, err, st);
 }
 
 }  // namespace hdgx

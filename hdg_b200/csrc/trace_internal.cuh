@@ -33,12 +33,14 @@ int trace_matvec(const hdgx_bsr *A, const double *Hg, const double *x, double *y
 
 // v = (L U)^{-1} x (kernel/applyBILU0.m); y [bs*nf] is the forward sweep's output.  Single-launch
 // level sweeps when A->sweep_plan is set, flag-scheduled sweeps when A->ncolors == 0, one launch
-// per colour otherwise.  Allocates nothing.
-int trace_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, cudaStream_t st);
+// per colour otherwise.  Allocates nothing.  err (device, may be NULL) is set when a wait of the
+// single-launch sweeps runs out (the result is then NaN).
+int trace_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, int *err,
+                      cudaStream_t st);
 
 // The same sweeps with the factors stored in FP32 (every sum in FP64); only the single-launch
 // level sweeps of A->sweep_plan are offered in this form (-2 otherwise).
-int trace_bilu0_apply_f32(const hdgx_bsr *A, const float *Mg32, const double *x, double *y, double *v,
+int trace_bilu0_apply_f32(const hdgx_bsr *A, const float *Mg32, const double *x, double *y, double *v, int *err,
                           cudaStream_t st);
 
 // Restarted left-preconditioned GMRES (kernel/gmres_bilu0.m) with every scratch array carved from

@@ -324,7 +324,7 @@ int hdgx_matvec(const hdgx_bsr *A, const double *Hg, const double *x, double *y,
 int hdgx_bilu0_factor(const hdgx_bsr *A, double *Mg, int *status, hdgx_stream_t stream);
 
 /* v = (L U)^{-1} x (kernel/applyBILU0.m); work[bs*nf] scratch.  With a sweep_plan the sweeps are one launch
- * whose waits for a value end in NaN after a bounded number of polls; v may be x.  Where work overlaps x or v, or
+ * whose waits for a value end in NaN after a bounded number of polls (a plan that is no schedule); v may be x.  Where work overlaps x or v, or
  * v overlaps x in part, one launch per level is used instead. */
 int hdgx_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *v, double *work,
                      hdgx_stream_t stream);
@@ -334,8 +334,9 @@ size_t hdgx_gmres_workspace_bytes(const hdgx_bsr *A, int restart);
 
 /* Left-preconditioned restarted GMRES with modified Gram-Schmidt (kernel/gmres_bilu0.m):
  * x (in: initial guess, out: solution) [bs,nf]; stops when |P^{-1}(b - A x)| <= tol |P^{-1} b|
- * or after maxit iterations.  iters, flag (0 converged, 1 maxit, 3 breakdown), relres and
- * history[maxit] (optional) are host outputs.  workspace (device, hdgx_gmres_workspace_bytes)
+ * or after maxit iterations.  iters, flag (0 converged, 1 maxit, 3 breakdown, also when a residual or
+ * |P^{-1} b| is not finite), relres and history[maxit] (optional) are host outputs.  A bounded wait that runs
+ * out is a status: -14 (flag-scheduled sweeps), -15 (Gram-Schmidt step), -16 (single-launch sweeps).  workspace (device, hdgx_gmres_workspace_bytes)
  * may be NULL, in which case it is taken from the stream-ordered allocator. */
 int hdgx_gmres_bilu0(const hdgx_bsr *A, const double *Hg, const double *Mg, const double *b, double *x,
                      int restart, double tol, int maxit, int *iters, int *flag, double *relres,
