@@ -520,9 +520,10 @@ __device__ __forceinline__ void gj_regs_t(const double *__restrict__ A, double *
             a[i][jj] = (T)v;
         }
     unsigned used = 0u;
-    // owners of column kc publish it and choose its pivot row: key = bits of (float)|v| with
-    // the low 10 bits replaced by the row (|v| within 2^-13 relative counts as a tie, won
-    // by the higher row; NaN wins so that it is reported)
+    // owners of column kc publish it and choose its pivot row: key = the upper 32 bits of |v| as a double (its
+    // whole range of exponents) with the low 7 bits replaced by the row (|v| within 2^-13 relative counts as a
+    // tie, won by the higher row; NaN wins so that it is reported)
+    static_assert(!PIVOT || N <= 128, "a row number has 7 bits");
     auto publish = [&](int kc, int jq) {
         T *pn = pcol + (kc & 1) * N;
         unsigned best = 0u;
@@ -535,8 +536,8 @@ __device__ __forceinline__ void gj_regs_t(const double *__restrict__ A, double *
             if (r < N) {
                 pn[r] = v;
                 if (PIVOT && !((used >> i) & 1u)) {
-                    const float av = (float)fabs(v);
-                    const unsigned key = (av == av ? (__float_as_uint(av) & ~0x3FFu) : 0xFFFFFC00u) | (unsigned)r;
+                    const double av = fabs((double)v);
+                    const unsigned key = (av == av ? ((unsigned)__double2hiint(av) & ~0x7Fu) : 0xFFFFFF80u) | (unsigned)r;
                     best = key > best ? key : best;
                 }
             }
@@ -547,7 +548,7 @@ __device__ __forceinline__ void gj_regs_t(const double *__restrict__ A, double *
                 const unsigned ob = __shfl_xor_sync(gmask, best, o, TR);
                 best = ob > best ? ob : best;
             }
-            if (tr == 0) slot[kc & 1] = (int)(best & 0x3FFu);
+            if (tr == 0) slot[kc & 1] = (int)(best & 0x7Fu);
         }
     };
     if (tc == 0) publish(0, 0);
