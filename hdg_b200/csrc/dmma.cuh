@@ -29,11 +29,11 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-// 1 / x from the hardware's 23-bit approximation (rcp.approx.ftz.f64) and one step of the third-order
-// Newton (Householder) iteration y (1 + e + e^2), e = 1 - x y: the relative error goes from 2^-23
-// to 2^-69 plus rounding, i.e. within one unit in the last place of the quotient, in three dependent
-// operations (the compiled division takes 230 cycles in a dependent chain, this takes about 90).
-// A subnormal, zero or non-finite x gives a value that is not finite or not 1 / x: callers check.
+// 1 / x from the hardware's approximation (rcp.approx.ftz.f64, which reads and returns the upper 32 bits of a
+// double: a relative error e of some 2^-20) and one step of the third-order Newton (Householder) iteration
+// y (1 + e + e^2), e = 1 - x y, which leaves e^3, below 2^-59, and two roundings: within 2 ulp of the quotient
+// (compared with it in tests/test_range_gpu.py), in three dependent operations (the compiled division takes 230
+// cycles in a dependent chain, this takes about 90).  For x and 1 / x that are normal numbers; see rcp_in_range.
 __device__ __forceinline__ double fast_rcp(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -41,11 +41,16 @@ __device__ __forceinline__ double fast_rcp(double x) {
     return fma(y, fma(e, e, e), y);
 }
 
+// Whether fast_rcp holds: x and 1 / x normal numbers, with a margin (exponents -1020 to 1020; not zero, not infinite, a number).
+__device__ __forceinline__ bool rcp_in_range(double x) {
+    return (unsigned)((__double2hiint(x) >> 20 & 2047) - 3) <= 2040u;
+}
+
 // Inverse of the 8 x 8 matrix held as a C fragment by a warp, in place: Gauss-Jordan over the four
 // diagonal 2 x 2 blocks in order (no pivoting).  One 2 x 2 block costs one shuffle round, one
 // reciprocal (of its determinant, the products with it formed meanwhile) and two multiply-adds in
 // sequence; between(b) is issued while block b's reciprocal is on its way.  Returns false when a
-// determinant is zero or not finite.
+// determinant is zero, not finite or outside the range of fast_rcp.
 template <class F>
 __device__ __forceinline__ bool inv8(double (&z)[2], F between) {
     const unsigned full = 0xffffffffu;
@@ -60,7 +65,7 @@ __device__ __forceinline__ bool inv8(double (&z)[2], F between) {
         const double r00 = __shfl_sync(full, z[0], 4 * p + h), r01 = __shfl_sync(full, z[1], 4 * p + h);
         const double r10 = __shfl_sync(full, z[0], 4 * p + 4 + h), r11 = __shfl_sync(full, z[1], 4 * p + 4 + h);
         const double det = fma(a00, a11, -(a01 * a10));
-        ok &= fabs(det) > 0.0 && isfinite(det);
+        ok &= rcp_in_range(det);
         const double rd = fast_rcp(det);
         between(b);
         // the block's rows become its inverse times them; row m loses (x0, x1) inverse times them
@@ -109,7 +114,10 @@ struct TableOrder {
 // CTAs of 192 threads per SM: 31,500 -> 14,200; N = 60, 61, one CTA of 256: 50,200 -> 19,700; N = 50,
 // 121, one of 256: 45,700 -> 21,100; N = 24, 37, four of 128: 14,700 -> 6,500.
 // pub: pub_doubles doubles of shared memory, 16-byte aligned, that overlap neither A nor B.
-// *bad = 8 k + 1 when block k is singular.
+// *bad = 8 k + 1 when block k is singular, or its determinants are out of the range of fast_rcp.
+// SCALED: the system is solved as (s A) x = s B with s the power of two that brings the first entry of A to 1 .. 2
+// (exact, so the bits do not change), for matrices whose entries are of one size but may be very small or large (mass
+// matrices: of the order of the volume): their 2 x 2 determinants leave the range first.
 template <int N, int NR, int NT>
 struct BlockGJ {
     static constexpr int MT = (N + 7) / 8, RT = (NR + 7) / 8, CT = MT + RT, NW = NT / 32, CPT = (CT + NW - 1) / NW;
@@ -170,12 +178,18 @@ __device__ __forceinline__ void publish_tiles(double (&z)[MT][2], const double *
             i == k ? make_double2(z[i][0], z[i][1]) : make_double2(-z[i][0], -z[i][1]);
 }
 
-template <int N, int NR, int LDB, int NT, class Order>
+__device__ __forceinline__ double power_of_two_to_one(double x) {     // 2^-exponent(x); 1 when that is no normal number
+    const int e = __double2hiint(x) >> 20 & 2047;
+    return e >= 1 && e <= 2045 ? __hiloint2double((2046 - e) << 20, 0) : 1.0;
+}
+
+template <int N, int NR, int LDB, int NT, bool SCALED = false, class Order>
 __device__ __forceinline__ void block_gj(const double *__restrict__ A, double *B, double *pub, int *bad, Order order) {
     using G = BlockGJ<N, NR, NT>;
     constexpr int MT = G::MT, CT = G::CT, NW = G::NW, CPT = G::CPT, TS = G::TS;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = lane >> 2, n0 = 2 * (lane & 3);
     double z[CPT][MT][2];
+    [[maybe_unused]] const double scale = SCALED ? power_of_two_to_one(A[0]) : 1.0;
 #pragma unroll
     for (int s = 0; s < CPT; s++) {
         const int c = w + s * NW, col = 8 * c + m;
@@ -186,7 +200,7 @@ __device__ __forceinline__ void block_gj(const double *__restrict__ A, double *B
 #pragma unroll
             for (int t = 0; t < 2; t++) {
                 const int row = 8 * i + n0 + t;
-                z[s][i][t] = (in && row < N) ? src[order(row)] : (c < MT && col == row ? 1.0 : 0.0);
+                z[s][i][t] = (in && row < N) ? (SCALED ? scale * src[order(row)] : src[order(row)]) : (c < MT && col == row ? 1.0 : 0.0);
             }
     }
     auto step = [&](auto kc) {

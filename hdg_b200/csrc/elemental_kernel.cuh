@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
         double *pub = wk;                                 // column blocks of the eliminations
         if constexpr (L::WS) pub = smd + L::ws_pub;
         else pub = wk + ev(L::x_wrl);
-        block_gj<NPV, NPV * ND + NDF * ND + NCU * ND, NPV, NT>(s_M, s_MiC, pub, s_bad, NaturalOrder{});
+        block_gj<NPV, NPV * ND + NDF * ND + NCU * ND, NPV, NT, true>(s_M, s_MiC, pub, s_bad, NaturalOrder{});
         if (tid == 0 && *s_bad) *s_bad = 1;
         __syncthreads();
 

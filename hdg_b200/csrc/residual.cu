@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(NT, residual_blocks<D>(NT, WARPS)) residual_ke
         }
 
         // ---- q = inv(M) (M SH_q / fc_q + C u - E uh): M is SPD, eliminated without pivoting
-        block_gj<NPV, NQD, NPV, NT>(s_M, s_R, sm + L::pub, s_bad, NaturalOrder{});
+        block_gj<NPV, NQD, NPV, NT, true>(s_M, s_R, sm + L::pub, s_bad, NaturalOrder{});
         __syncthreads();
         if (P.QDG) {
             for (int i = tid; i < NPV * NQD; i += NT) P.QDG[(size_t)e * NPV * NQD + i] = s_R[i];
