@@ -324,8 +324,8 @@ int hdgx_matvec(const hdgx_bsr *A, const double *Hg, const double *x, double *y,
 int hdgx_bilu0_factor(const hdgx_bsr *A, double *Mg, int *status, hdgx_stream_t stream);
 
 /* v = (L U)^{-1} x (kernel/applyBILU0.m); work[bs*nf] scratch.  With a sweep_plan the sweeps are one launch
- * whose waits for a value end in NaN after a bounded number of polls (a plan that is no schedule); v may be x.  Where work overlaps x or v, or
- * v overlaps x in part, one launch per level is used instead. */
+ * (two where v overlaps x) whose waits for a value end in NaN after a bounded number of polls (a plan that is no
+ * schedule).  The three may overlap; where work lies over x or v, the library's memory pool gives another one. */
 int hdgx_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *v, double *work,
                      hdgx_stream_t stream);
 
