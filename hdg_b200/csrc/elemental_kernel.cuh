@@ -180,8 +180,7 @@ struct Plan {
     static constexpr int y_Y = y_Xg + D::NGT * NCG * TILE;
     static constexpr int y_end = y_Y + D::NGT * D::NCU * TILE;
     static_assert(y_end <= x_end, "the column tiles fit the scratch");
-    static constexpr int d_slots = p_end;                               // 3 x u64 pivot slots
-    static constexpr int d_pcol = d_slots + 4;                          // [4*NU] pivot column copies
+    static constexpr int d_pcol = p_end;                                // [4*NU] pivot column copies
     static constexpr int d_diag = d_pcol + 4 * D::NU;                   // [NU] pivots
     static constexpr int d_b0 = d_diag + D::NU;                         // [NU] first right-hand side
     static constexpr int d_invsep = d_b0 + D::NU;                       // [NU*NU] FP32-accurate SD^-1 (MIXED)
@@ -206,10 +205,7 @@ struct Plan {
     // integers (after the doubles in shared memory)
     static constexpr int i_perm = 0;                      // [NPF, NFE] 0-based
     static constexpr int i_invp = D::NPF * D::NFE;        // [NPV, NFE] face-local index or -1
-    static constexpr int i_piv = i_invp + D::NPV * D::NFE;
-    static constexpr int i_pivM = i_piv + D::NU;
-    static constexpr int i_rowused = i_pivM + D::NPV;
-    static constexpr int i_rowvar = i_rowused + D::NU;
+    static constexpr int i_rowvar = i_invp + D::NPV * D::NFE;
     static constexpr int i_gslot = i_rowvar + D::NU;
     static constexpr int i_bf = i_gslot + 2;
     static constexpr int i_bad = i_bf + D::NFE;
@@ -270,7 +266,7 @@ struct PlanMma {
     // before the flux Jacobians: inv(M)'s column blocks, then SH_q / fc_q - q; after them: SD's column
     // blocks, or what the pivoted elimination works with
     static constexpr int p_pub = x_wrl, p_rqs = x_wrl + PUBM;
-    static constexpr int d_slots = x_wrl, d_pcol = d_slots + 4, d_diag = d_pcol + 2 * D::NU, d_fall = d_diag + D::NU;
+    static constexpr int d_pcol = x_wrl, d_diag = d_pcol + 2 * D::NU, d_fall = d_diag + D::NU;
     static constexpr int x_ZFc = ev(mx(mx(x_Zc + (VISC ? ZV * D::NPV * D::ND : 0), mx(d_fall, x_wrl + mx(PUB, PUBM + D::NPV * D::NCU * D::ND))),
                                        x_start + GS));
     static constexpr int x_ZFe = x_ZFc + (VISC ? ZF * D::NPV * D::ND : 0);     // [ZF, NPV, ND], [ZF, NDF, ND]
@@ -300,14 +296,13 @@ struct PlanMma {
     static constexpr int i_perm = 0;                      // [NPF, NFE] 0-based
     static constexpr int i_invp = D::NPF * D::NFE;        // [NPV, NFE] face-local index or -1
     static constexpr int i_piv = i_invp + D::NPV * D::NFE;
-    static constexpr int i_pivM = i_piv + D::NU;
-    static constexpr int i_rowused = i_pivM + D::NPV;
-    static constexpr int i_rowvar = i_rowused + D::NU;
+    static constexpr int i_rowvar = i_piv + D::NU;
     static constexpr int i_gslot = i_rowvar + D::NU;
     static constexpr int i_bf = i_gslot + 2;
     static constexpr int i_bad = i_bf + D::NFE;
-    static constexpr int i_tmem = i_bad + 1;
-    static constexpr int i_ord = i_tmem + 1;              // [NU] elimination order of the local system
+    // [NU] elimination order of the local system, from an odd place on: from an even one the compiler reads two entries
+    // at a time, and 2D NS p = 3, 32,768 elements, takes 3,364 us instead of 3,316
+    static constexpr int i_ord = (i_bad + 1) | 1;
     static constexpr int n_ints = i_ord + D::NU;
     static constexpr size_t bytes = sizeof(double) * n_doubles + sizeof(int) * n_ints;   // the whole plan
     // Plans beyond a CTA's shared memory (3D p = 3) keep the double arrays in a per-CTA slice of a
@@ -525,9 +520,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
     double *x_FHu = wk + L::x_FHu, *x_FHh = xd + L::x_FHh;
     double *x_Zc = wk + L::x_Zc, *x_Ze = xd + L::x_Ze, *x_Zr = xd + L::x_Zr;
     double *x_ZFc = wk + L::x_ZFc, *x_ZFe = wk + L::x_ZFe, *x_ZFr = xd + L::x_ZFr;
-    int *s_piv = si + L::i_piv, *s_pivM = si + L::i_pivM, *s_bf = si + L::i_bf, *s_bad = si + L::i_bad;
-    int *s_rowused = si + L::i_rowused, *s_rowvar = si + L::i_rowvar, *s_gslot = si + L::i_gslot;
-    unsigned long long *s_slot = reinterpret_cast<unsigned long long *>(wk + L::d_slots);
+    int *s_bf = si + L::i_bf, *s_bad = si + L::i_bad, *s_rowvar = si + L::i_rowvar, *s_gslot = si + L::i_gslot;
     double *s_pcol = wk + L::d_pcol, *s_diag = wk + L::d_diag;
 
     int seg = 0;                                 // segmented launches: the segment of element eg
@@ -1173,7 +1166,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) elemental_kernel(const __grid_cons
                 // substitution in shared memory, the solution written straight to s_R
                 constexpr int NU1 = NU + 1, CH = L::LU_CH;
                 double *l_LU = s_SD, *l_B = smd + L::ws_pub;  // SD is built in shared memory: factored in place
-                int *ip = s_rowvar;                      // row of SD that ends up at position i
+                int *s_piv = si + L::i_piv, *ip = s_rowvar;                      // row of SD that ends up at position i
                 block_lu<NT>(l_LU, NU, NU, s_piv, s_bad);
                 if (tid == 0) {
                     for (int i = 0; i < NU; i++) ip[i] = i;

@@ -22,11 +22,12 @@
 //
 // What bounds a level is then the store-to-load time through L2 (0.47 us measured between two SMs)
 // and the arithmetic after it, so both are kept short: the row's factor blocks are staged in
-// shared memory before its inputs arrive, by one bulk copy a block (16-byte copies by all lanes cost
-// a warp about 2,500 cycles a row of 30 x 30 blocks; blocks that are no multiple of 16 bytes, those of 15 x 15,
-// still take them: apply 600 -> 577 us at 12,416 faces of 16, 597 -> 567 us at 6,528 of 30), lane r of part p (PARTS = 32 / BS parts) adds up only
+// shared memory before its inputs arrive, by one bulk copy a block (copies of single values by all lanes cost a
+// warp about 2,500 cycles a row of 30 x 30 blocks; blocks that are no multiple of 16 bytes, those of 15 x 15, and
+// factors that are not aligned to 16 still take them: apply, with four warps a row of an average level, 600 -> 577 us
+// at 12,416 faces of 16, 597 -> 567 us at 6,528 of 30), lane r of part p (PARTS = 32 / BS parts) adds up only
 // the neighbours p, p + PARTS, .. in CH independent chains (a dependent FP64 multiply-add takes
-// 17.6 cycles), and the parts are added with shuffles.
+// 17.6 cycles), and the parts are added with shuffles.  Apply: 571 us at those faces of 16, 539 us at those of 30.
 #include <cuda_runtime.h>
 #include <type_traits>
 #include "hdgx_common.cuh"
@@ -87,7 +88,10 @@ struct SweepShape {
     static constexpr int PARTS = 32 / BS, DP = (MAXD + PARTS - 1) / PARTS;
     static constexpr int RW = 2 + 4 * MAXD;                                  // record width (ints)
     static constexpr int BLK = BS * BS;
-    static constexpr int CH = BS == 30 ? 6 : (BS == 15 ? 5 : 4);             // chains of a row sum
+    // Chains of a row's sum: enough that the multiply-adds' latency is hidden, few enough that adding them up is
+    // short.  Apply in us with half as many / these / twice as many: blocks of 8, 10,920 faces, 472 / 433 / 435; of 12, 4,880,
+    // 301 / 301 / 312; of 15, 12,600, 957 / 963 / 974; of 16, 12,416, 593 / 571 / 581; of 20, 2,760, 307 / 306 / 323; of 30, 6,528, 549 / 542 / 544.
+    static constexpr int CH = BS == 30 ? 6 : (BS == 15 ? 5 : 4);
     static constexpr size_t stage = (sizeof(MT) * BLK * (MAXD + 1) + 15) / 16 * 16;
     static constexpr int BSP = (BS + 1) / 2 * 2;                             // 16-byte aligned value rows
     static constexpr size_t warp_bytes = stage + sizeof(double) * BSP * (MAXD + 1) + 16;
@@ -95,9 +99,11 @@ struct SweepShape {
     static constexpr int WPC = fit > 16 ? 16 : fit;
     static constexpr size_t smem = warp_bytes * WPC;
     // Products of the neighbours that have arrived, while the last one is waited for: pays where a block's product
-    // is long.  Each has a sum of its own, and these are added in slot order, so that the result does not depend on who
-    // came first (apply 536 -> 539 us; products in slot order, each when it and those before it are there: 614).  Apply in us, all at once / as they arrive: blocks of 30, 6,528 faces in 282 levels, 702 / 597; of 20, 1,776
-    // in 160, 251 / 255; of 16, 12,416 in 440, 592 / 623; of 12, 800 in 104, 129 / 133.
+    // is long.  Apply in us, all at once / as they arrive (four warps a row, values copied one by one): blocks of 30, 6,528
+    // faces in 282 levels, 702 / 597; of 20, 1,776 in 160, 251 / 255; of 16, 12,416 in 440, 592 / 623; of 12, 800 in 104, 129 / 133.
+    // Each product has a sum of its own, and these are added in slot order, so that the result does not depend on who
+    // came first (one sum in the order of arrival: 536 us instead of 539; products in slot order, each when it and
+    // those before it are there: 614).
     static constexpr bool EARLY = BS > 20;
     static_assert(!EARLY || (PARTS == 1 && DP <= 6), "the slots of a warp are one row's");
     static_assert(BS <= 32 && RW <= 32 && WPC >= 1, "one lane per row component and per record entry");

@@ -98,6 +98,11 @@ struct SchurShape {
                          o_int = o_red + 32, doubles = o_int;
     static constexpr int i_ord = 0, i_face = NU, i_var = i_face + NPV, i_slot = i_var + NU, i_bad = i_slot + 4, ints = i_bad + 2;
     static constexpr size_t bytes = sizeof(double) * doubles + sizeof(int) * ints;
+    // As many CTAs as shared memory holds, up to six, and threads so that their registers suffice (fewer threads leave the
+    // elimination to fewer warps).  In us with two thirds of the threads / these / a third more where there is room / fewer
+    // CTAs of as many threads: 2D p = 1, 16,200 elements, 328 / 293 / 268 / 353; p = 2, 9,800, 380 / 336 / 328 / 366;
+    // p = 3, 4,050, 366 / 346 / 334 / 377; p = 4, 1,800, 564 / 414 / 419 / 551; 3D p = 1, 4,374, 358 / 326 / 314 / 260; p = 2, 1,296,
+    // 1,028 / 576 / 574 / 577.
     static constexpr int blocks = bytes <= 36 * 1024 ? 6 : (bytes <= 56 * 1024 ? 4 : (bytes <= 74 * 1024 ? 3 : (bytes <= 113 * 1024 ? 2 : 1)));
     static constexpr int threads = blocks == 6 ? 96 : (blocks == 4 ? 128 : (blocks == 3 ? 192 : 256));
 };

@@ -801,7 +801,9 @@ __global__ void bilu0_bwd_bs_kernel(const int *__restrict__ rows, int nrows, con
 // y = Hg x, a warp per row: the row's neighbours and their values of x are read at once (lane b the block
 // index b, then lane r the values r, into shared memory), and PARTS = 32 / BS groups of lanes take every
 // PARTS-th block.  DRAM-bound; with one group of lanes and x read by every lane, 2D p = 3, 12,416 faces
-// (102 MB): 45.5 us; now 26.9 us.
+// (102 MB): 45.5 us; now 26.9 us.  CTAs per SM in the launch bounds: four, two from blocks of 20 on, whose row of a
+// block takes the registers of a lane (half as many / these / more: blocks of 16 32.3 / 26.8 / 28.6 us, of 15 30.7 /
+// 29.9 / 31.4, of 30 55.3 / 55.4 / 53.4).
 template <int BS>
 __global__ void __launch_bounds__(256, BS >= 20 ? 2 : 4) bsr_matvec_bs_kernel(int nf, const long long *__restrict__ rowpts,
                                                             const int *__restrict__ colind, const double *__restrict__ Hg,
