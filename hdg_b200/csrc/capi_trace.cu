@@ -147,8 +147,8 @@ __global__ void mgs_coop_kernel(size_t, int, const double *, double *, unsigned 
 // nv - 1 of H as one cooperative launch (mgs_coop_kernel); false when the device cannot hold the grid at
 // once, or the vectors are long: the caller then issues the separate products.  One block an SM streams them more
 // slowly than full grids do, and the exchanges saved no longer make up for it: a GMRES step, fused / separate, of
-// 1,013,840 unknowns 1,843 / 1,878 us, 1,560,960: 2,391 / 2,397, 2,330,240: 3,012 / 2,981, 2,540,160 (3D): 4,162 / 4,116.  packets: 4 * kMgsBlocks words, zero before the first
-// call; tag: above every tag of earlier calls on them by more than nv.
+// 1,013,840 unknowns 1,843 / 1,878 us, 1,560,960: 2,391 / 2,397, 2,330,240: 3,012 / 2,981, 2,540,160 (3D): 4,162 /
+// 4,116.  packets: 4 * kMgsBlocks words, zero before the first call; tag: above every tag of earlier calls on them by more than nv.
 static bool mgs_fused(size_t n, int nv, const double *V, double *w, unsigned long long *packets, unsigned tag, int *err,
                       GmresState gs, int m, cudaStream_t st) {
     if (n > kMgsMaxN) return false;

@@ -41,7 +41,8 @@ __device__ __forceinline__ double fast_rcp(double x) {
     return fma(y, fma(e, e, e), y);
 }
 
-// Whether fast_rcp holds: x and 1 / x normal numbers, with a margin (exponents -1020 to 1020; not zero, not infinite, a number).
+// Whether fast_rcp holds: x and 1 / x normal numbers, with a margin (exponents -1020 to 1020; so x is a number,
+// not zero and not infinite).
 __device__ __forceinline__ bool rcp_in_range(double x) {
     return (unsigned)((__double2hiint(x) >> 20 & 2047) - 3) <= 2040u;
 }

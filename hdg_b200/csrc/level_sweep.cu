@@ -89,8 +89,9 @@ struct SweepShape {
     static constexpr int RW = 2 + 4 * MAXD;                                  // record width (ints)
     static constexpr int BLK = BS * BS;
     // Chains of a row's sum: enough that the multiply-adds' latency is hidden, few enough that adding them up is
-    // short.  Apply in us with half as many / these / twice as many: blocks of 8, 10,920 faces, 472 / 433 / 435; of 12, 4,880,
-    // 301 / 301 / 312; of 15, 12,600, 957 / 963 / 974; of 16, 12,416, 593 / 571 / 581; of 20, 2,760, 307 / 306 / 323; of 30, 6,528, 549 / 542 / 544.
+    // short.  Apply in us with half as many / these / twice as many: blocks of 8, 10,920 faces, 472 / 433 / 435; of 12,
+    // 4,880, 301 / 301 / 312; of 15, 12,600, 957 / 963 / 974; of 16, 12,416, 593 / 571 / 581; of 20, 2,760, 307 / 306 / 323;
+    // of 30, 6,528, 549 / 542 / 544.
     static constexpr int CH = BS == 30 ? 6 : (BS == 15 ? 5 : 4);
     static constexpr size_t stage = (sizeof(MT) * BLK * (MAXD + 1) + 15) / 16 * 16;
     static constexpr int BSP = (BS + 1) / 2 * 2;                             // 16-byte aligned value rows

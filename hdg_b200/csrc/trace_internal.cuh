@@ -33,8 +33,8 @@ int trace_matvec(const hdgx_bsr *A, const double *Hg, const double *x, double *y
 
 // v = (L U)^{-1} x (kernel/applyBILU0.m); y [bs*nf] is the forward sweep's output.  Single-launch
 // level sweeps when A->sweep_plan is set, flag-scheduled sweeps when A->ncolors == 0, one launch
-// per colour otherwise.  Allocates nothing.  err (device, may be NULL) is set when a wait of the
-// single-launch sweeps runs out (the result is then NaN).
+// per colour otherwise.  Allocates nothing, except for the level sweeps where y overlaps x or v.  err
+// (device, may be NULL) is set when a wait of the level sweeps runs out (the result is then NaN).
 int trace_bilu0_apply(const hdgx_bsr *A, const double *Mg, const double *x, double *y, double *v, int *err,
                       cudaStream_t st);
 
